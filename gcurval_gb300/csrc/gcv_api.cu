@@ -1265,6 +1265,7 @@ gcv_status run_sampling(gcv_ctx* c, const int64_t* d_sample_off, double* d_pos, 
     P.collect = c->opt.collect_stats;
     P.rtol = c->opt.rtol;
     P.eps_frac = (float)(SAMPLE_EPS_FRAC * c->opt.rtol);
+    P.min_runs = sm_count() * SAMPLE_RUNS_PER_SM;
     P.curve_list = nullptr;
     P.list_off = nullptr;
     P.cb = P.ce = 0;
@@ -1480,6 +1481,7 @@ gcv_status enqueue_sampling_graph(gcv_ctx* c, const int* d_counts, const double*
     P.collect = c->opt.collect_stats;
     P.rtol = c->opt.rtol;
     P.eps_frac = (float)(SAMPLE_EPS_FRAC * c->opt.rtol);
+    P.min_runs = sm_count() * SAMPLE_RUNS_PER_SM;
     // grids for any sample count: the kernels loop over their ranges
     const int64_t nominal = (int64_t)sm_count() * c->knobs.sample_blocks_per_sm * c->knobs.sample_threads;
     if (c->code >= 0) {

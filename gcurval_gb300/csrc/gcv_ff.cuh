@@ -48,6 +48,38 @@ __device__ __forceinline__ ff ff_from_double(double x)
     return fast_two_sum(hi, sign ? -lo : lo);
 }
 
+// x 2^-s -> float-float from the bit pattern, for data of any double range:
+// the caller's s brings the values it works with near 1, and what falls below
+// 2^-70 there is 0 (far under any float-float rounding of them), what rises
+// above 2^126 is infinite.  NaN and infinities pass through.  Selects, no
+// branches: the samplers convert up to 15 coefficients per Newton step.
+__device__ __forceinline__ ff ff_from_double_scaled(double x, int s)
+{
+    const unsigned top = (unsigned)__double2hiint(x), low = (unsigned)__double2loint(x);
+    const unsigned sign = top & 0x80000000u, raw = (top >> 20) & 0x7FFu;
+    const int e = (int)raw - 1023 - s;
+    const bool tiny = raw == 0u || e < -70, huge = raw == 0x7FFu || e > 126;
+    const unsigned m = ((top & 0xFFFFFu) << 3) | (low >> 29);
+    const unsigned special = raw == 0x7FFu && ((top & 0xFFFFFu) | low) != 0u ? 0x7FC00000u : 0x7F800000u;
+    const float hi = __uint_as_float(sign | (huge ? special : tiny ? 0u : ((unsigned)(e + 127) << 23) | m));
+    const float lo = __uint2float_rn(low & 0x1FFFFFFFu) * __uint_as_float(((unsigned)(e - 52 + 127) << 23) | sign);
+    return tiny || huge ? ff{hi, 0.0f} : fast_two_sum(hi, lo);
+}
+
+// binary exponent of a double's magnitude (0 for 0, infinities and NaN)
+__device__ __forceinline__ int exponent_of(double x)
+{
+    const int raw = (int)((unsigned)(__double2hiint(x)) >> 20) & 0x7FF;
+    return raw == 0 || raw == 0x7FF ? 0 : raw - 1023;
+}
+
+// x 2^-s, s of any size (flushes to 0 / overflows to infinity)
+__device__ __forceinline__ float scale_down(float x, int s)
+{
+    const int c = s < -252 ? -252 : (s > 252 ? 252 : s), h = c / 2;
+    return x * __int_as_float((127 - h) << 23) * __int_as_float((127 - (c - h)) << 23);
+}
+
 __device__ __forceinline__ double ff_to_double(ff a) { return (double)a.hi + (double)a.lo; }
 
 // double -> float by truncation of the significand, from the bit pattern

@@ -99,6 +99,25 @@ struct EvalFF {
             }
         }
     }
+    // the same from the FP64 table's position polynomial, all lengths times
+    // 2^-s: b[k] = (k + 1) a[k + 1], or A, B (squared lengths) and w0
+    __device__ __forceinline__ static void load(const double* __restrict__ seg, ff* r, int s)
+    {
+        if constexpr (CODE == 0) {
+            r[0] = ff_from_double_scaled(seg[0], 2 * s);
+            r[1] = ff_from_double_scaled(seg[1], 2 * s);
+            r[2] = ff{__double2float_rn(seg[2]), 0.0f};
+        } else {
+#pragma unroll
+            for (int k = 0; k < P; ++k)
+#pragma unroll
+                for (int d = 0; d < D; ++d) {
+                    const ff a = ff_from_double_scaled(seg[(k + 1) * D + d], s);
+                    // exact for the powers of two
+                    r[k * D + d] = (k & (k + 1)) == 0 ? ff_scale(a, float(k + 1)) : ff_mul_f(a, float(k + 1));
+                }
+        }
+    }
     __device__ __forceinline__ static ff speed(const ff* r, ff v)
     {
         if constexpr (CODE == 0) {

@@ -103,6 +103,7 @@ struct SampleParams {
     int64_t cb, ce;
     int64_t s_begin, s_end;  // sample range of the launch when curve_list is NULL
     const int64_t* s_end_dev;  // when set: the end of that range, read on the device
+    int min_runs;  // k_sample_ff: runs the launch should at least consist of (shorter runs then)
 };
 
 // Sample range of a launch and, for launch-local sample i, its curve and its
@@ -153,8 +154,11 @@ __device__ __forceinline__ int sample_curve_hint(const SampleParams& P, int64_t 
     gi = i + h.shift;
     return h.c;
 }
-// samples per warp and turn in the mixed sampler (8 per lane, 32 apart)
+// samples per warp and turn in k_sample_ff: up to 256 (8 per lane, 32 apart),
+// fewer in launches too small to give every warp slot of the GPU
+// (SAMPLE_RUNS_PER_SM) a run that long
 constexpr int SAMPLE_RUN = 256;
+constexpr int SAMPLE_RUNS_PER_SM = 96;
 
 // Newton stops once the estimated residual of its last step is below
 // SAMPLE_EPS_FRAC * rtol * L.  The table itself is good to rtol * L (the

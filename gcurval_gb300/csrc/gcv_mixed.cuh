@@ -1,4 +1,4 @@
-// Mixed-precision path (GCV_MIXED): the integrand and the panel sums run on
+// Mixed-precision path (GCV_MIXED), and the sampling of FP64 tables: the integrand and the panel sums run on
 // the FP32 pipes in float-float arithmetic (gcv_ff.cuh, ~48-bit significand);
 // FP64 is kept for the three steps whose stability needs it:
 //   * the compensated prefix sum of interval lengths (k_scan, shared with the
@@ -13,6 +13,8 @@
 // Ellipse integrands (sin^2(pi v)) are evaluated with an own float-float
 // series for sin^2(pi u), |u| <= 1/4, after folding (gcv_ff_eval.cuh).
 #pragma once
+
+#include <type_traits>
 
 #include "gcv_ff_eval.cuh"
 #include "gcv_kernels.cuh"
@@ -81,10 +83,13 @@ __device__ __forceinline__ ff gl8_pairs(ff* b, ff m, ff h)
 // UNROLL: small integrands unroll the Gauss loop; large ones (panel_rolled)
 // and the runtime-dispatch kernel keep it rolled, so that the body fits the
 // instruction cache.
-template <int C, bool UNROLL>
-__device__ __forceinline__ double ff_leaf_newton(const float2* __restrict__ seg, ff vaf, float dv, ff rl, ff dS,
+// TAB: the coefficient table's element: float2 (float-float, mixed tables) or
+// double (FP64 tables; lengths then come scaled by 2^-sexp, see k_sample_ff).
+template <int C, bool UNROLL, typename TAB>
+__device__ __forceinline__ double ff_leaf_newton(const TAB* __restrict__ seg, int sexp, ff vaf, float dv, ff rl, ff dS,
                                                  float dvg, float eps_s, unsigned long long& newton)
 {
+    constexpr bool FROM64 = std::is_same<TAB, double>::value;
     constexpr bool PAIRS = sample_node_pairs(C);
     float blo = 0.0f, bhi = dv;
     ff w{dvg, 0.0f};
@@ -92,7 +97,11 @@ __device__ __forceinline__ double ff_leaf_newton(const float2* __restrict__ seg,
     for (int it = 0; it < NEWTON_MAXIT; ++it) {
         ++newton;
         ff r[MAX_COEF];
-        EvalFF<C>::load(seg, r);  // every iteration: the node-pair Gauss sum shifts r
+        // every iteration: the node-pair Gauss sum shifts r
+        if constexpr (FROM64)
+            EvalFF<C>::load(seg, r, sexp);
+        else
+            EvalFF<C>::load(seg, r);
         const bool from_left = w.hi <= 0.5f * dv;
         // [a0, a1] in local offsets: [0, w] or [w, dv]
         const ff a0 = from_left ? ff{0.0f, 0.0f} : w;
@@ -145,7 +154,10 @@ __device__ __forceinline__ double ff_leaf_newton(const float2* __restrict__ seg,
                 f1 = EvalFF<C>::speed_slope_f(r, ff_add(vaf, ff_add_f(w, -dn)), q1);
             const float d = 2.0f * Fh / (f0 + f1);
             const float s0 = q0 / f0, s1 = q1 / f1;  // f'(w), f'(w - dn)
-            const float res = dn * dn * (fabsf(s1 - s0) * (1.0f / 3.0f) + s1 * s1 * fabsf(dn) / (4.0f * f1));
+            float res = dn * dn * (fabsf(s1 - s0) * (1.0f / 3.0f) + s1 * s1 * fabsf(dn) / (4.0f * f1));
+            // at FP64 tolerances the FP32 rounding of the step itself counts:
+            // f0, f1 and the quotient are good to a few 2^-24 of F
+            if constexpr (FROM64) res = fmaf(5e-7f, fabsf(Fh), res);
             const float wd = w.hi - d;
             if (res <= eps_s && wd >= 0.0f && wd <= dv) {
                 last = d;  // converged: the step is applied in FP64
@@ -175,22 +187,45 @@ __device__ __forceinline__ double ff_leaf_newton(const float2* __restrict__ seg,
 // batch took 139.9 ms, against 143.7 ms with a spill-free 96 (5 blocks).
 __host__ __device__ constexpr int sample_ff_regs(int code) { return code == bs_code(5, 3) ? 88 : 80; }
 static_assert(88 * SAMPLE_THREADS_MAX <= 65536, "a block of SAMPLE_THREADS_MAX must fit one SM");
-template <int CODE>
-__global__ void __maxnreg__(sample_ff_regs(CODE)) k_sample_ff(SampleParams P, const float2* __restrict__ coef_ff)
+//
+// TAB = double runs the same kernel on an FP64 table (GCV_PLAIN_FP64 at
+// tolerances down to PLAIN_SPLIT_RTOL).  What it computes in float-float is
+// the offset inside one leaf: the sums over a curve, the target and the
+// parameter stay FP64, so a float-float rounding (2^-45) enters a sample's
+// position only times the leaf's share of the curve, below FP64's own
+// rounding of the target on curves of some tens of leaves and at most 2.8e-14
+// of the curve's length otherwise, far under the stopping threshold
+// SAMPLE_EPS_FRAC * rtol * L >= 1e-13 L.  Lengths inside the leaf are scaled by
+// 2^-sexp, the binary exponent of its mean speed, so that curves of any
+// double magnitude fit FP32's exponent range.  The FP64 kernel was bound by
+// the FP64 pipe (91 % busy, one warp instruction per 64 issue slots); this one
+// by issue.  4,096 ellipses x 1,000 samples: 4.15 -> 0.64 ms; 10,000 planar
+// cubics x 1,024: 8.51 -> 0.96 ms.  Position errors at rtol 1e-10 .. 1e-12 on
+// ellipses, cubics and an uneven batch, rms and worst, are at or below the FP64
+// kernel's: the extra term of its stopping test makes it iterate further.
+template <int CODE, typename TAB>
+__global__ void __maxnreg__(sample_ff_regs(CODE)) k_sample_ff(SampleParams P, const TAB* __restrict__ coef)
 {
+    constexpr bool FROM64 = std::is_same<TAB, double>::value;
     const Batch& b = P.b;
     const Table& t = P.t;
     unsigned long long newton = 0;
     int64_t i0, i1;
     sample_range(P, i0, i1);
-    // each warp takes runs of SAMPLE_RUN consecutive samples, 32 at a time:
-    // a lane's samples then mostly share their curve (see CurveHint)
+    // each warp takes runs of up to SAMPLE_RUN consecutive samples, 32 at a
+    // time: a lane's samples then mostly share their curve (see CurveHint).
+    // Small launches shorten the runs to 32 so that no lane places 8 samples
+    // one after another while most of the GPU idles (6,400 ellipse samples:
+    // 120 us with runs of 256, 34 us with 32; the uneven batch of 301 curves,
+    // nine launches: 750 us and 185 us)
+    const int64_t per = (i1 - i0) / P.min_runs & ~(int64_t)31;
+    const int run_len = per >= SAMPLE_RUN ? SAMPLE_RUN : (per < 32 ? 32 : (int)per);
     CurveHint hint;
     const int lane = threadIdx.x & 31;
     const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t run = i0 + wid * SAMPLE_RUN; run < i1; run += n_warps * SAMPLE_RUN)
-    for (int64_t ii = run + lane; ii < run + SAMPLE_RUN && ii < i1; ii += 32) {
+    for (int64_t run = i0 + wid * run_len; run < i1; run += n_warps * run_len)
+    for (int64_t ii = run + lane; ii < run + run_len && ii < i1; ii += 32) {
         int64_t i;
         const int c = sample_curve_hint(P, ii, i, hint);
         const int code = CODE >= 0 ? CODE : curve_code(b, c);
@@ -207,7 +242,8 @@ __global__ void __maxnreg__(sample_ff_regs(CODE)) k_sample_ff(SampleParams P, co
             // target <= 0 / target >= L on the bit patterns (L >= 0; a negative
             // target has a negative pattern): integer compares, off the FP64 pipe
             const long long tb = __double_as_longlong(target), lb = __double_as_longlong(L);
-            if (tb <= 0) {
+            // (FP64 tables: a NaN target is the curve's start, as !(target > 0) in k_sample)
+            if (tb <= 0 || (FROM64 && tb > 0x7FF0000000000000ll)) {
                 s = s0;
                 v = -1.0;
             } else if (tb >= lb) {
@@ -235,11 +271,24 @@ __global__ void __maxnreg__(sample_ff_regs(CODE)) k_sample_ff(SampleParams P, co
                 }
                 const double vb = t.leaf_v[lo + j];
                 const double cb = t.leaf_cum[lo + j];
-                const float fb = (float)t.leaf_f[lo + j];
-                const float qb = (float)t.leaf_q[lo + j];
-                const ff rl = ff_from_double(rr - base);   // target inside the leaf
-                const ff dS = ff_from_double(cb - base);   // leaf length
-                const double dvd = vb - va;                 // leaf width (exact dyadic)
+                float fb = t.leaf_f[lo + j];
+                float qb = t.leaf_q[lo + j];
+                const double rd = rr - base, dSd = cb - base;  // target inside the leaf, leaf length
+                const double dvd = vb - va;                     // leaf width (exact dyadic)
+                int sexp = 0;
+                ff rl, dS;
+                if constexpr (FROM64) {
+                    sexp = exponent_of(dSd) - exponent_of(dvd);
+                    rl = ff_from_double_scaled(rd, sexp);
+                    dS = ff_from_double_scaled(dSd, sexp);
+                    fa = scale_down(fa, sexp);
+                    fb = scale_down(fb, sexp);
+                    qa = scale_down(qa, 2 * sexp);
+                    qb = scale_down(qb, 2 * sexp);
+                } else {
+                    rl = ff_from_double(rd);
+                    dS = ff_from_double(dSd);
+                }
                 const float dv = (float)dvd;
                 const ff vaf = ff_from_double(va);
                 // quintic Hermite guess of v(S) on the leaf (FP32)
@@ -259,16 +308,16 @@ __global__ void __maxnreg__(sample_ff_regs(CODE)) k_sample_ff(SampleParams P, co
                     dvg = h5 * dv + dS.hi * (h1 * ia + h4 * ib) + dS.hi * dS.hi * (h2 * ka + h3 * kb);
                     dvg = fminf(fmaxf(dvg, 0.0f), dv);
                 }
-                const float2* seg = coef_ff + b.coef_off[c] + (s - s0) * code_stride(code);
-                const float eps_s = P.eps_frac * f32_of_f64_trunc(L);
+                const TAB* seg = coef + b.coef_off[c] + (s - s0) * code_stride(code);
+                const float eps_s = P.eps_frac * (FROM64 ? ff_from_double_scaled(L, sexp).hi : f32_of_f64_trunc(L));
                 double wfinal;
                 if constexpr (CODE >= 0) {
                     wfinal = ff_leaf_newton<(CODE >= 0 ? CODE : 0), !panel_rolled<(CODE >= 0 ? CODE : 0)>()>(
-                        seg, vaf, dv, rl, dS, dvg, eps_s, newton);
+                        seg, sexp, vaf, dv, rl, dS, dvg, eps_s, newton);
                 } else {
                     switch (code) {
 #define GCV_CASE(C)                                                                                \
-    case C: wfinal = ff_leaf_newton<C, false>(seg, vaf, dv, rl, dS, dvg, eps_s, newton); break;
+    case C: wfinal = ff_leaf_newton<C, false>(seg, sexp, vaf, dv, rl, dS, dvg, eps_s, newton); break;
                         GCV_FOR_EACH_CODE(GCV_CASE)
 #undef GCV_CASE
                     default: wfinal = dvg; break;
@@ -297,19 +346,24 @@ __global__ void __maxnreg__(sample_ff_regs(CODE)) k_sample_ff(SampleParams P, co
         } else {
             double p3[3] = {0.0, 0.0, 0.0};
             if (s >= 0) {
-                // points from the float-float coefficients, evaluated in FP64
-                // (a B-spline stores a[0] and then b[k - 1] = k a[k])
-                const float2* seg = coef_ff + b.coef_off[c] + (s - s0) * code_stride(code);
+                const TAB* seg = coef + b.coef_off[c] + (s - s0) * code_stride(code);
                 double cd[MAX_COEF];
-                const int n = code_stride(code), dim = code_dim(code);
-                for (int k = 0; k < n; ++k) {
-                    cd[k] = (double)seg[k].x + (double)seg[k].y;
-                    if (code != 0 && k >= 2 * dim) cd[k] *= 1.0 / (double)(k / dim);
+                const double* pc = cd;
+                if constexpr (FROM64) {
+                    pc = seg;
+                } else {
+                    // points from the float-float coefficients, evaluated in FP64
+                    // (a B-spline stores a[0] and then b[k - 1] = k a[k])
+                    const int n = code_stride(code), dim = code_dim(code);
+                    for (int k = 0; k < n; ++k) {
+                        cd[k] = (double)seg[k].x + (double)seg[k].y;
+                        if (code != 0 && k >= 2 * dim) cd[k] *= 1.0 / (double)(k / dim);
+                    }
                 }
                 if constexpr (CODE >= 0)
-                    Eval<(CODE >= 0 ? CODE : 0)>::point(cd, v, p3);
+                    Eval<(CODE >= 0 ? CODE : 0)>::point(pc, v, p3);
                 else
-                    point_dyn(code, cd, v, p3);
+                    point_dyn(code, pc, v, p3);
             }
             for (int k = 0; k < P.pdim; ++k) P.out[i * P.pdim + k] = p3[k];
         }

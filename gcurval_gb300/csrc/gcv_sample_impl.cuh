@@ -11,7 +11,9 @@ template <int CODE, int PREC>
 cudaError_t sample_launch(const SampleParams& P, const float2* coef_ff, cudaStream_t stream, int grid, int threads)
 {
     if constexpr (PREC == 1)
-        k_sample_ff<CODE><<<grid, threads, 0, stream>>>(P, coef_ff);
+        k_sample_ff<CODE, float2><<<grid, threads, 0, stream>>>(P, coef_ff);
+    else if (P.rtol >= PLAIN_SPLIT_RTOL)
+        k_sample_ff<CODE, double><<<grid, threads, 0, stream>>>(P, P.t.coef);
     else
         k_sample<CODE><<<grid, threads, 0, stream>>>(P);
     return cudaGetLastError();

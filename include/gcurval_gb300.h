@@ -59,7 +59,9 @@ typedef enum gcv_enum {
 } gcv_enum;
 
 typedef enum gcv_precision {
-    GCV_PLAIN_FP64 = 0,    /* every step in FP64 */
+    GCV_PLAIN_FP64 = 0,    /* FP64 lengths, sums, targets and parameters; at rtol >= 1e-12
+                              the Newton steps inside one table entry run in float-float
+                              (48 bits), below it in FP64 */
     GCV_MIXED = 1          /* FP32 integrand and panels; FP64 prefix sum,
                               error test near tolerance and final Newton step */
 } gcv_precision;
