@@ -809,11 +809,17 @@ gcv_status launch_length_code(gcv_ctx* c, int code, const LengthParams& P)
     cudaError_t e = cudaErrorInvalidValue;
     if constexpr (MODE == 0) {
         const int cap = c->knobs.length_cap[code_slot(code)];
-        const bool half_warp = PREC == 1 && c->opt.mapping == GCV_MAP_HALF_WARP;
+        // FP64 tables: k_walk wherever its float-float partition resolves the
+        // tolerance and the depth, the FP64 walk beyond
+        const bool half_warp = c->opt.mapping == GCV_MAP_HALF_WARP;
+        const bool walk64 = c->opt.rtol >= PLAIN_SPLIT_RTOL && P.max_depth <= FF_MAX_DEPTH;
         switch (code) {
 #define GCV_CASE(C)                                                                                \
     case C:                                                                                        \
-        e = half_warp ? length_launch_hw<C>(P, c->stream, sms, cap) : length_launch<0, C, PREC>(P, c->stream, sms, cap); \
+        if constexpr (PREC == 1)                                                                   \
+            e = half_warp ? length_launch_hw<C>(P, c->stream, sms, cap) : walk_launch<C, 1>(P, c->stream, sms, cap); \
+        else                                                                                       \
+            e = walk64 ? walk_launch<C, 2>(P, c->stream, sms, cap) : length_launch<0, C, 0>(P, c->stream, sms, cap); \
         break;
             GCV_FOR_EACH_CODE(GCV_CASE)
 #undef GCV_CASE
@@ -1039,7 +1045,7 @@ gcv_status build_table(gcv_ctx* c)
         // start depths of every B-spline interval from the network (ellipse pieces keep 0)
         CHECK(c->starts.reserve((size_t)c->n_seg));
         CU(cudaMemsetAsync(c->starts.p, 0, (size_t)c->n_seg * sizeof(uint32_t), c->stream));
-        const int md = mixed ? std::min(c->opt.max_depth, 44) : c->opt.max_depth;
+        const int md = mixed ? std::min(c->opt.max_depth, FF_MAX_DEPTH) : c->opt.max_depth;
         // start depths in the order of the work items (the grouped list)
         auto run = [&](const uint4* f16, uint32_t* starts, int64_t n) -> gcv_status {
             cudaError_t e = mlp_starts_launch_bf16(f16, nullptr, n, c->mlp_w, md, starts, c->stream);
@@ -1065,8 +1071,7 @@ gcv_status build_table(gcv_ctx* c)
         P.b = b;
         P.t = table_view(c);
         P.rtol = c->opt.rtol;
-        // float-float panel bounds are exact to depth 44
-        P.max_depth = mixed ? std::min(c->opt.max_depth, 44) : c->opt.max_depth;
+        P.max_depth = mixed ? std::min(c->opt.max_depth, FF_MAX_DEPTH) : c->opt.max_depth;
         P.collect = c->opt.collect_stats;
         P.list = nullptr;
         P.n_items = 0;
@@ -1077,6 +1082,13 @@ gcv_status build_table(gcv_ctx* c)
         CHECK(read_counters(c));
         const unsigned long long err = c->h_ctr[C_ERR];
         if (err & ERR_BAD_KNOTS) return fail(GCV_ERR_INVALID, "knot vector decreases or holds NaN");
+        if (err & ERR_POOL) {
+            // k_walk's leaves did not fit the pool: once more with a larger one
+            const int64_t need = (int64_t)c->h_ctr[C_LEAF_TOP];
+            CHECK(grow_pool(c, need + need / 16 + 4096, 0));
+            CU(cudaMemsetAsync(c->ctr.p + C_ERR, 0, sizeof(unsigned long long), c->stream));
+            continue;
+        }
         if (err & ERR_DEEP_LIST) {
             DBuf<int>& dl = c->deep_list;
             const size_t need = (size_t)(c->h_ctr[C_DEEP] * 1.25) + 1024;
@@ -1392,7 +1404,7 @@ gcv_status enqueue_table_graph(gcv_ctx* c)
     CU(cudaEventRecordWithFlags(c->ev[1], c->stream, cudaEventRecordExternal));
     if (learned) {
         CU(cudaMemsetAsync(c->starts.p, 0, (size_t)c->n_seg * sizeof(uint32_t), c->stream));
-        const int md = mixed ? std::min(c->opt.max_depth, 44) : c->opt.max_depth;
+        const int md = mixed ? std::min(c->opt.max_depth, FF_MAX_DEPTH) : c->opt.max_depth;
         // start depths in the order of the work items (the grouped list)
         auto run = [&](const uint4* f16, uint32_t* starts, int64_t n) -> gcv_status {
             cudaError_t e = mlp_starts_launch_bf16(f16, nullptr, n, c->mlp_w, md, starts, c->stream);
@@ -1413,7 +1425,7 @@ gcv_status enqueue_table_graph(gcv_ctx* c)
         P.b = b;
         P.t = table_view(c);
         P.rtol = c->opt.rtol;
-        P.max_depth = mixed ? std::min(c->opt.max_depth, 44) : c->opt.max_depth;
+        P.max_depth = mixed ? std::min(c->opt.max_depth, FF_MAX_DEPTH) : c->opt.max_depth;
         P.collect = c->opt.collect_stats;
         P.coef_ff = c->coef_ff.p;
         P.starts = learned ? c->starts.p : nullptr;

@@ -77,6 +77,86 @@ __device__ __forceinline__ ff ff_sinpi_sq(ff x)
     return up ? ff_add_f(ff_neg(S), 1.0f) : S;
 }
 
+// sin(pi x) and cos(pi x) for small x by their Taylor series, at compile time
+__host__ __device__ constexpr double series_sinpi(double x)
+{
+    double t = PI * x, s = 0.0;
+    for (int k = 1; t > 1e-40 || t < -1e-40; k += 2) {
+        s += t;
+        t *= -(PI * x) * (PI * x) / ((k + 1) * (k + 2));
+    }
+    return s;
+}
+__host__ __device__ constexpr double series_cospi(double x)
+{
+    double t = 1.0, s = 0.0;
+    for (int k = 0; t > 1e-20 || t < -1e-20; k += 2) {
+        s += t;
+        t *= -(PI * x) * (PI * x) / ((k + 1) * (k + 2));
+    }
+    return s;
+}
+
+// Ellipse panels by angle addition: with w_m the panel's midpoint and d_i =
+// 2^-depth x_i / ELLIPSE_PIECES the offset of the Kronrod pair i from it,
+// sin(pi (w_m -+ d_i)) = sin(pi w_m) cos(pi d_i) -+ cos(pi w_m) sin(pi d_i).
+// The offsets depend on the depth alone, so their sines and cosines are a
+// table, and a panel evaluates one sine and cosine instead of fifteen.
+constexpr int ANGLE_DEPTHS = 49;  // 0 .. MAX_DEPTH_LIMIT
+struct alignas(16) AngleTable {
+    double sc[ANGLE_DEPTHS][8][2];  // pair i: sin(pi d_i), 1 - cos(pi d_i); entry 7 is the centre
+    float ff[ANGLE_DEPTHS][8][4];   // float-float sine and cosine: sin hi, lo, cos hi, lo
+    __host__ __device__ constexpr AngleTable() : sc(), ff()
+    {
+        double h = ELLIPSE_PIECE_SCALE;
+        for (int d = 0; d < ANGLE_DEPTHS; ++d, h *= 0.5)
+            for (int i = 0; i < 8; ++i) {
+                const double x = i < 7 ? h * gk_x(i) : 0.0;
+                const double s = series_sinpi(x), c = series_cospi(x), h2 = series_sinpi(0.5 * x);
+                sc[d][i][0] = s;
+                sc[d][i][1] = 2.0 * h2 * h2;
+                ff[d][i][0] = split_const(s).hi;
+                ff[d][i][1] = split_const(s).lo;
+                ff[d][i][2] = split_const(c).hi;
+                ff[d][i][3] = split_const(c).lo;
+            }
+    }
+};
+static __device__ const AngleTable c_angle{};
+
+// sin(pi u) and cos(pi u) for |u| <= 1/4 in the two lanes of one packed series
+// in u^2 (nine terms: the next are below 1e-17 relative); the sine's lane
+// is then multiplied by u
+constexpr int SINCOS_TERMS = 9;
+__host__ __device__ constexpr double sinpi_coef(int k)
+{
+    double c = PI;
+    for (int i = 1; i <= k; ++i) c *= -PI * PI / ((2 * i) * (2 * i + 1));
+    return c;
+}
+__host__ __device__ constexpr double cospi_coef(int k)
+{
+    double c = 1.0;
+    for (int i = 1; i <= k; ++i) c *= -PI * PI / ((2 * i - 1) * (2 * i));
+    return c;
+}
+// |sin(pi x)| and |cos(pi x)| for x in [-1, 1]
+__device__ __forceinline__ void ff_abs_sincospi(ff x, ff& s, ff& c)
+{
+    ff y = x.hi < 0.0f ? ff_neg(x) : x;
+    if (y.hi > 0.5f) y = ff_add_f(ff_neg(y), 1.0f);
+    const bool swap = y.hi > 0.25f;
+    const ff u = swap ? ff_add_f(ff_neg(y), 0.5f) : y;
+    const ff2 U = splat(ff_mul(u, u));
+    ff2 p = pack(to_ff(split_const(sinpi_coef(SINCOS_TERMS - 1))), to_ff(split_const(cospi_coef(SINCOS_TERMS - 1))));
+#pragma unroll
+    for (int k = SINCOS_TERMS - 2; k >= 0; --k)
+        p = ff2_fma(p, U, pack(to_ff(split_const(sinpi_coef(k))), to_ff(split_const(cospi_coef(k)))));
+    const ff a = ff_mul(lane0(p), u), b = lane1(p);
+    s = swap ? b : a;
+    c = swap ? a : b;
+}
+
 // ------------------------------------------------------------- evaluators
 template <int CODE>
 struct EvalFF {
@@ -316,52 +396,6 @@ __device__ void bspline_setup_ff(const double* __restrict__ kv, const double* __
     }
 }
 
-// float-float panel: K15, G7, right-end speed and slope of [vlo, vlo + 2 hw]
-// with vlo = -1 + k 2^(1-depth) built exactly from the integer k.
-// Kronrod nodes x0..x6, weights wk0..wk7 and Gauss weights wg0..wg7 (0 for
-// the Kronrod-only nodes) as float-float pairs, for the rolled panel loop
-#define GCV_FFC2(x) {split_const(x).hi, split_const(x).lo}
-static __constant__ float2 c_gk_ff[23] = {
-    GCV_FFC2(gk_x(0)),  GCV_FFC2(gk_x(1)),  GCV_FFC2(gk_x(2)),  GCV_FFC2(gk_x(3)),  GCV_FFC2(gk_x(4)),
-    GCV_FFC2(gk_x(5)),  GCV_FFC2(gk_x(6)),  GCV_FFC2(gk_wk(0)), GCV_FFC2(gk_wk(1)), GCV_FFC2(gk_wk(2)),
-    GCV_FFC2(gk_wk(3)), GCV_FFC2(gk_wk(4)), GCV_FFC2(gk_wk(5)), GCV_FFC2(gk_wk(6)), GCV_FFC2(gk_wk(7)),
-    GCV_FFC2(gk_wg(0)), GCV_FFC2(gk_wg(1)), GCV_FFC2(gk_wg(2)), GCV_FFC2(gk_wg(3)), GCV_FFC2(gk_wg(4)),
-    GCV_FFC2(gk_wg(5)), GCV_FFC2(gk_wg(6)), GCV_FFC2(gk_wg(7))};
-#undef GCV_FFC2
-
-// Large integrands (high degree x dimension, and the float-float ellipse with
-// its two Taylor series) keep the node loop rolled: fourteen inlined copies
-// overflow the instruction cache.
-template <int CODE>
-constexpr bool panel_rolled()
-{
-    return CODE == 0 || code_degree(CODE) * code_dim(CODE) >= 8;
-}
-
-template <int CODE>
-__device__ __forceinline__ void panel_k15_ff(const ff* r, unsigned long long k, int depth, ff& K, ff& G)
-{
-    const float hw = __int_as_float((127 - depth) << 23);  // 2^-depth, exact
-    const float kh = (float)(unsigned)(k >> 24), kl = (float)(unsigned)(k & 0xFFFFFFull);
-    const float sh = __int_as_float((127 + 25 - depth) << 23), sl = 2.0f * hw;  // 2^(25-depth), 2^(1-depth)
-    const ff vlo = ff_add_f(two_sum(-1.0f, kh * sh), kl * sl);
-    const ff mid = ff_add_f(vlo, hw);
-    const ff fc = EvalFF<CODE>::speed(r, mid);
-    ff kk = ff_mul(to_ff(split_const(gk_wk(7))), fc);
-    ff gg = ff_mul(to_ff(split_const(gk_wg(7))), fc);
-    // the two nodes of a pair in packed lanes
-#pragma unroll 1
-    for (int i = 0; i < 7; ++i) {
-        const ff dx = ff_scale(ff{c_gk_ff[i].x, c_gk_ff[i].y}, hw);
-        const ff2 f = EvalFF<CODE>::speed2(r, pack(ff_add(mid, ff_neg(dx)), ff_add(mid, dx)));
-        const ff s = ff_add(lane0(f), lane1(f));
-        kk = ff_fma(ff{c_gk_ff[7 + i].x, c_gk_ff[7 + i].y}, s, kk);
-        if (i & 1) gg = ff_fma(ff{c_gk_ff[15 + i].x, c_gk_ff[15 + i].y}, s, gg);  // the Gauss nodes
-    }
-    K = ff_scale(kk, hw);
-    G = ff_scale(gg, hw);
-}
-
 // B-spline panels by node pairs.  The speed polynomials p_d (degree P - 1 in
 // v) are shifted to the panel's midpoint m and scaled to its half width h:
 // b_j = h^j p_d^(j)(m) / j!, so p_d(m + h x) = sum_j b_j x^j on x in [-1, 1]
@@ -372,8 +406,7 @@ __device__ __forceinline__ void panel_k15_ff(const ff* r, unsigned long long k, 
 // E = b_0 + b_2 x^2 + ... and the odd part O = x (b_1 + b_3 x^2 + ...):
 // p(m -+ h x) = E -+ O.  Per pair of nodes this replaces two Horner passes
 // in v (2 (P - 1) float-float FMAs per dimension) and the two node
-// positions by about half the work; K15 and G7 are formed as in
-// panel_k15_ff.
+// positions by about half the work.
 
 template <int P, int D>
 __device__ __forceinline__ void ff_node_pair(const ff* b, ff x, ff x2, ff& fm, ff& fp)
@@ -460,6 +493,36 @@ __host__ __device__ constexpr double gk_pair_wg(int i) { return i < 7 ? gk_wg(i)
 static __constant__ GkStep2 c_gk_step2[4] = {GCV_GK_STEP2(0), GCV_GK_STEP2(1), GCV_GK_STEP2(2), GCV_GK_STEP2(3)};
 #undef GCV_GK_STEP2
 
+// An ellipse piece's panel by angle addition (AngleTable), two node pairs per
+// packed step as in panel_k15_ff_pairs.  Signs of the midpoint's sine and
+// cosine only swap a pair's two nodes, so magnitudes do.  r: A, B, w0.
+__device__ __forceinline__ void panel_k15_ff_ellipse(const ff* r, unsigned long long k, int depth, ff& K, ff& G)
+{
+    const float hw = __int_as_float((127 - depth) << 23);  // 2^-depth, exact
+    const float kh = (float)(unsigned)(k >> 24), kl = (float)(unsigned)(k & 0xFFFFFFull);
+    const float sh = __int_as_float((127 + 25 - depth) << 23), sl = 2.0f * hw;
+    const ff mid = ff_add_f(ff_add_f(two_sum(-1.0f, kh * sh), kl * sl), hw);
+    ff sm, cm;
+    ff_abs_sincospi(ff_add_f(ff_scale(mid, (float)ELLIPSE_PIECE_SCALE), r[2].hi), sm, cm);
+    const ff2 s2 = splat(sm), c2 = splat(cm), A = splat(r[0]), B = splat(r[1]);
+    const float4* tab = reinterpret_cast<const float4*>(c_angle.ff[depth]);
+    ff2 kk2{}, gg2{};
+#pragma unroll 1
+    for (int j = 0; j < 4; ++j) {
+        const float4 a = __ldg(tab + 2 * j), b = __ldg(tab + 2 * j + 1);
+        const ff2 sd{make_float2(a.x, b.x), make_float2(a.y, b.y)}, cd{make_float2(a.z, b.z), make_float2(a.w, b.w)};
+        const ff2 p = ff2_mul(s2, cd);
+        const ff2 up = ff2_fma(c2, sd, p), dn = ff2_fma(c2, ff2_neg(sd), p);
+        const ff2 fm = ff2_sqrt(ff2_fma(A, ff2_mul(dn, dn), B)), fp = ff2_sqrt(ff2_fma(A, ff2_mul(up, up), B));
+        const ff2 sum = ff2_add(fm, fp);
+        const GkStep2 c = c_gk_step2[j];
+        kk2 = ff2_fma(ff2{c.wkh, c.wkl}, sum, kk2);
+        gg2 = ff2_fma(ff2{c.wgh, c.wgl}, sum, gg2);
+    }
+    K = ff_scale(ff_add(lane0(kk2), lane1(kk2)), hw);
+    G = ff_scale(ff_add(lane0(gg2), lane1(gg2)), hw);
+}
+
 // b: the interval's speed coefficients on entry, shifted in place
 template <int CODE>
 __device__ __forceinline__ void panel_k15_ff_pairs(ff* b, unsigned long long k, int depth, ff& K, ff& G)
@@ -487,30 +550,18 @@ __device__ __forceinline__ void panel_k15_ff_pairs(ff* b, unsigned long long k, 
     // the node pairs two at a time in packed lanes (the centre in the last
     // step's second lane); the two lanes' sums are added at the end
     ff2 kk2{}, gg2{};
-    if constexpr (panel_rolled<CODE>()) {
+    // Rolled: four inlined copies of even a planar quadratic's step missed the
+    // instruction cache (k_walk of planar degree 2-3: no_instruction first
+    // among the stalls after the fixed latencies; the uneven batch's walk 14.4 ms
+    // unrolled, 13.0 rolled).
 #pragma unroll 1
-        for (int j = 0; j < 4; ++j) {
-            const GkStep2 c = c_gk_step2[j];
-            ff2 fm, fp;
-            ff_node_pair2<P, D>(b, ff2{c.xh, c.xl}, ff2{c.x2h, c.x2l}, fm, fp);
-            const ff2 sum = ff2_add(fm, fp);
-            kk2 = ff2_fma(ff2{c.wkh, c.wkl}, sum, kk2);
-            gg2 = ff2_fma(ff2{c.wgh, c.wgl}, sum, gg2);  // zero weights on the Kronrod-only pairs
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const ff2 x = pack(to_ff(split_const(gk_pair_x(2 * j))), to_ff(split_const(gk_pair_x(2 * j + 1))));
-            const ff2 x2 = pack(to_ff(split_const(gk_pair_x(2 * j) * gk_pair_x(2 * j))),
-                                to_ff(split_const(gk_pair_x(2 * j + 1) * gk_pair_x(2 * j + 1))));
-            ff2 fm, fp;
-            ff_node_pair2<P, D>(b, x, x2, fm, fp);
-            const ff2 sum = ff2_add(fm, fp);
-            kk2 = ff2_fma(pack(to_ff(split_const(gk_pair_wk(2 * j))), to_ff(split_const(gk_pair_wk(2 * j + 1)))), sum, kk2);
-            // the Gauss nodes: pairs 1, 3, 5 and the centre (lane 1)
-            gg2 = ff2_fma(pack(to_ff(split_const(gk_pair_wg(2 * j))), to_ff(split_const(gk_pair_wg(2 * j + 1)))), sum,
-                          gg2);
-        }
+    for (int j = 0; j < 4; ++j) {
+        const GkStep2 c = c_gk_step2[j];
+        ff2 fm, fp;
+        ff_node_pair2<P, D>(b, ff2{c.xh, c.xl}, ff2{c.x2h, c.x2l}, fm, fp);
+        const ff2 sum = ff2_add(fm, fp);
+        kk2 = ff2_fma(ff2{c.wkh, c.wkl}, sum, kk2);
+        gg2 = ff2_fma(ff2{c.wgh, c.wgl}, sum, gg2);  // zero weights on the Kronrod-only pairs
     }
     const ff kk = ff_add(lane0(kk2), lane1(kk2));
     const ff gg = ff_add(lane0(gg2), lane1(gg2));
@@ -525,7 +576,7 @@ template <int CODE>
 __device__ __forceinline__ void panel_ff(ff* r, unsigned long long k, int depth, ff& K, ff& G)
 {
     if constexpr (CODE == 0)
-        panel_k15_ff<CODE>(r, k, depth, K, G);
+        panel_k15_ff_ellipse(r, k, depth, K, G);
     else
         panel_k15_ff_pairs<CODE>(r, k, depth, K, G);
 }

@@ -1,5 +1,7 @@
-// Adaptive length of every knot interval (FP64): persistent workers, one
-// lane per knot interval.
+// Adaptive length of every knot interval, one lane per knot interval: the main
+// pass of FP64 tables below PLAIN_SPLIT_RTOL, and the two passes over the deep
+// list (intervals with more leaves than the main pass stages).  The main pass of
+// all other tables is the warp-wide walk of gcv_walk.cuh, over the same panels.
 //
 // Each lane owns one segment at a time and refines it depth-first over the
 // dyadic panels of v in [-1, 1].  A panel is named by (k, depth): it spans
@@ -32,6 +34,7 @@ constexpr int LK_THREADS = 64;
 constexpr int LCAP = 16;
 constexpr long long PANEL_BUDGET = 1ll << 22;
 constexpr int MAX_DEPTH_LIMIT = 48;
+constexpr int FF_MAX_DEPTH = 44;  // float-float panel bounds are exact to this depth
 
 struct LengthParams {
     Batch b;
@@ -58,11 +61,17 @@ struct LengthParams {
 // Launches k_length<MODE, CODE, PREC> over P (persistent grid sized from the
 // occupancy, capped at blocks_per_sm_cap per SM, and sm_count); defined with the kernel in gcv_length_impl.cuh and
 // instantiated per curve code in the gcv_len_*.cu units.
-//   MODE 0: main pass; MODE 1: count pass of the deep list; MODE 2: write pass.
+//   MODE 0: main pass (FP64 panels only); MODE 1: count pass of the deep list;
+//   MODE 2: write pass.
 //   CODE: curve code, or -1 for runtime dispatch per segment.
 //   PREC 0: FP64 panels; 1: float-float panels.
 template <int MODE, int CODE, int PREC>
 cudaError_t length_launch(const LengthParams& P, cudaStream_t stream, int sm_count, int blocks_per_sm_cap);
+
+// The main pass with one list of pending panels per warp (gcv_walk.cuh).
+//   PREC 1: float-float table; 2: FP64 table, float-float partition, FP64 leaves.
+template <int CODE, int PREC>
+cudaError_t walk_launch(const LengthParams& P, cudaStream_t stream, int sm_count, int blocks_per_sm_cap);
 
 // The main pass (MODE 0) with float-float panels and one half-warp per knot
 // interval instead of one lane (gcv_length_hw.cuh); same table.

@@ -1,5 +1,5 @@
 // The length pass with one half-warp per knot interval (float-float panels):
-// the alternative mapping to k_length's one lane per interval, chosen by the
+// the alternative mapping to k_walk's one lane per panel, chosen by the
 // caller through gcv_options.mapping (GCV_MAP_HALF_WARP).  It is not an
 // autotuner choice: the two mappings sum K15 and G7 in different orders, and
 // a tuner's choice must leave every result bit-identical.
@@ -11,7 +11,8 @@
 // lanes.  Lane 0 of the half stages accepted leaves in shared memory; the
 // lanes write them out together when the interval is done.  The acceptance
 // test, the learned start, the leaf table and the deep-list hand-over are
-// those of k_length<0, CODE, 1>, so both mappings build the same table (up
+// those of k_walk<CODE, 1> (intervals of more than LCAP leaves go to the deep
+// passes here), so both mappings build the same table (up
 // to the summation order of K15 and G7).
 //
 // Per panel this mapping spends 16 lanes on one node each plus the

@@ -19,8 +19,8 @@ __device__ __forceinline__ void panel_k15(const double* r, double vlo, double hw
     const double fc = Eval<CODE>::speed(r, mid);
     double k = gk_wk(7) * fc;
     double g = gk_wg(7) * fc;
-    // unrolled: the FP64 integrands are compact (the float-float panels of
-    // large integrands keep their node loop rolled, see panel_k15_ff)
+    // unrolled: the FP64 integrands are compact (the float-float panels keep
+    // their node loop rolled)
     {
 #pragma unroll
         for (int i = 0; i < 7; ++i) {
@@ -81,31 +81,17 @@ __device__ __forceinline__ float chord_of(const T* r)
     return sqrtf(c2);
 }
 
-// Resident blocks per SM the float-float main pass asks for, per curve code:
-// 10 (at most 96 registers) for degree 3-5 in 3D, 12 (80) for the others.
-// Single-code batches of the uneven 100k batch, main pass alone, at 12 / 10 /
-// 8 blocks: degree 2-3 in 2D and degree 2 in 3D are fastest at 12 (3-14 %
-// ahead of 8), degree 4-5 in 2D tie at 12 and 10, degree 3-5 in 3D gain 2-4 %
-// at 10 (they spill 112-216 bytes at 80 registers, less at 96).
-__host__ __device__ constexpr int length_ff_blocks(int code)
-{
-    return code > 0 && code_dim(code) == 3 && code_degree(code) >= 3 ? 10 : 12;
-}
-
 // PREC 0: FP64 panels; PREC 1: float-float panels (GCV_MIXED), whose K15 /
 // G7 / end values enter the same FP64 bookkeeping (error test, leaf table).
 template <int MODE, int CODE, int PREC = 0>
-__global__ void __launch_bounds__(LK_THREADS, (MODE == 0 && PREC == 1) ? length_ff_blocks(CODE) : 1)
-    k_length(LengthParams P)
+__global__ void __launch_bounds__(LK_THREADS) k_length(LengthParams P)
 {
-    __shared__ double lf_v[MODE == 0 ? LCAP : 1][LK_THREADS];
-    __shared__ double lf_c[MODE == 0 ? LCAP : 1][LK_THREADS];
-    // the float-float path does not stage the leaves' end speed and slope:
-    // it re-evaluates them in FP32 when it flushes the leaves (same values),
-    // which leaves 16 of the 24 bytes per staged leaf and more blocks per SM
-    constexpr int FQ_ROWS = MODE == 0 && PREC == 0 ? LCAP : 1;
-    __shared__ float lf_f[FQ_ROWS][LK_THREADS];
-    __shared__ float lf_q[FQ_ROWS][LK_THREADS];
+    static_assert(MODE != 0 || PREC == 0, "the main pass of float-float tables is k_walk");
+    constexpr int ROWS = MODE == 0 ? LCAP : 1;
+    __shared__ double lf_v[ROWS][LK_THREADS];
+    __shared__ double lf_c[ROWS][LK_THREADS];
+    __shared__ float lf_f[ROWS][LK_THREADS];
+    __shared__ float lf_q[ROWS][LK_THREADS];
 
     const Batch& b = P.b;
     const Table& t = P.t;
@@ -181,14 +167,7 @@ __global__ void __launch_bounds__(LK_THREADS, (MODE == 0 && PREC == 1) ? length_
                         // learned start: the predicted depths, tolerance from the chord
                         if (P.starts) {
                             const uint32_t q = P.starts[by_item ? item : s];
-                            float ch;
-                            if constexpr (PREC == 1) {
-                                ff rc[MAX_COEF];
-                                EvalFF<(CODE > 0 ? CODE : 16 + 4 + 2)>::load(cff, rc);
-                                ch = chord_of<CODE>(rc);
-                            } else {
-                                ch = chord_of<CODE>(r);
-                            }
+                            const float ch = chord_of<CODE>(r);
                             if (q != 0u && ch > 0.0f) {
                                 dq = q;
                                 tol_unit = P.rtol * (double)ch;
@@ -211,10 +190,8 @@ __global__ void __launch_bounds__(LK_THREADS, (MODE == 0 && PREC == 1) ? length_
                         if (MODE == 0) {
                             lf_v[0][tid] = 1.0;
                             lf_c[0][tid] = 0.0;
-                            if constexpr (PREC == 0) {
-                                lf_f[0][tid] = 0.0f;
-                                lf_q[0][tid] = 0.0f;
-                            }
+                            lf_f[0][tid] = 0.0f;
+                            lf_q[0][tid] = 0.0f;
                         } else if (MODE == 2 && pool >= 0) {
                             t.leaf_v[pool] = 1.0;
                             t.leaf_cum[pool] = 0.0;
@@ -308,10 +285,8 @@ __global__ void __launch_bounds__(LK_THREADS, (MODE == 0 && PREC == 1) ? length_
                     if (nleaf < LCAP) {
                         lf_v[nleaf][tid] = vr;
                         lf_c[nleaf][tid] = cum;
-                        if constexpr (PREC == 0) {
-                            lf_f[nleaf][tid] = (float)fend;
-                            lf_q[nleaf][tid] = (float)qend;
-                        }
+                        lf_f[nleaf][tid] = (float)fend;
+                        lf_q[nleaf][tid] = (float)qend;
                     } else {
                         ovf = true;
                     }
@@ -368,31 +343,11 @@ __global__ void __launch_bounds__(LK_THREADS, (MODE == 0 && PREC == 1) ? length_
                     const int64_t o_off = (int64_t)__shfl_sync(FULL, (unsigned long long)off, owner);
                     const int i = gi - o_first;          // the leaf's index in its interval
                     const int otid = (tid & ~31) + owner;  // the owner's staging column
-                    if constexpr (PREC == 1) {
-                        const float2* o_cff = reinterpret_cast<const float2*>(
-                            __shfl_sync(FULL, reinterpret_cast<unsigned long long>(cff), owner));
-                        const int o_code = CODE >= 0 ? CODE : __shfl_sync(FULL, code, owner);
-                        if (gi < total && o_fits) {
-                            ff rl[MAX_COEF];
-                            if constexpr (CODE >= 0)
-                                EvalFF<(CODE >= 0 ? CODE : 0)>::load(o_cff, rl);
-                            else
-                                load_ff_dyn(o_code, o_cff, rl);
-                            const double vi = lf_v[i][otid];
-                            float q32;
-                            const float f32 = speed_slope32_of<CODE>(o_code, rl, (float)vi, q32);
-                            t.leaf_v[o_off + i] = vi;
-                            t.leaf_cum[o_off + i] = lf_c[i][otid];
-                            t.leaf_f[o_off + i] = f32;
-                            t.leaf_q[o_off + i] = q32;
-                        }
-                    } else {
-                        if (gi < total && o_fits) {
-                            t.leaf_v[o_off + i] = lf_v[i][otid];
-                            t.leaf_cum[o_off + i] = lf_c[i][otid];
-                            t.leaf_f[o_off + i] = lf_f[i][otid];
-                            t.leaf_q[o_off + i] = lf_q[i][otid];
-                        }
+                    if (gi < total && o_fits) {
+                        t.leaf_v[o_off + i] = lf_v[i][otid];
+                        t.leaf_cum[o_off + i] = lf_c[i][otid];
+                        t.leaf_f[o_off + i] = lf_f[i][otid];
+                        t.leaf_q[o_off + i] = lf_q[i][otid];
                     }
                 }
                 if (fin) {
@@ -457,7 +412,7 @@ cudaError_t length_launch(const LengthParams& P, cudaStream_t stream, int sm_cou
 
 #define GCV_LENGTH_INST(MODE, CODE, PREC)                                                          \
     template cudaError_t length_launch<MODE, CODE, PREC>(const LengthParams&, cudaStream_t, int, int);
-// both precisions of one (MODE, CODE)
+// both precisions of one deep pass
 #define GCV_LENGTH_INST2(MODE, CODE) GCV_LENGTH_INST(MODE, CODE, 0) GCV_LENGTH_INST(MODE, CODE, 1)
 
 }  // namespace gcv

@@ -57,7 +57,7 @@ __host__ __device__ constexpr bool sample_node_pairs(int code)
 // w_k (f(m - X) + f(m + X)) into the sum (the caller scales it by h).  For
 // degree 5 in 3D that is 30 float-float multiply-adds of shift plus 4 pairs
 // instead of 8 Horner evaluations of 12.
-template <int C, bool UNROLL>
+template <int C>
 __device__ __forceinline__ ff gl8_pairs(ff* b, ff m, ff h)
 {
     constexpr int P = code_degree(C), D = code_dim(C);
@@ -80,12 +80,9 @@ __device__ __forceinline__ ff gl8_pairs(ff* b, ff m, ff h)
     return ff_add(lane0(I2), lane1(I2));
 }
 
-// UNROLL: small integrands unroll the Gauss loop; large ones (panel_rolled)
-// and the runtime-dispatch kernel keep it rolled, so that the body fits the
-// instruction cache.
 // TAB: the coefficient table's element: float2 (float-float, mixed tables) or
 // double (FP64 tables; lengths then come scaled by 2^-sexp, see k_sample_ff).
-template <int C, bool UNROLL, typename TAB>
+template <int C, typename TAB>
 __device__ __forceinline__ double ff_leaf_newton(const TAB* __restrict__ seg, int sexp, ff vaf, float dv, ff rl, ff dS,
                                                  float dvg, float eps_s, unsigned long long& newton)
 {
@@ -110,7 +107,7 @@ __device__ __forceinline__ double ff_leaf_newton(const TAB* __restrict__ seg, in
         const ff m2 = ff_add(ff_add(vaf, a0), h2);
         ff I{0.0f, 0.0f};
         if constexpr (PAIRS) {
-            I = gl8_pairs<C, UNROLL>(r, m2, h2);  // r now holds the coefficients about m2
+            I = gl8_pairs<C>(r, m2, h2);  // r now holds the coefficients about m2
         } else {
             // nodes -x_k and +x_k in packed lanes
 #pragma unroll 1
@@ -312,12 +309,12 @@ __global__ void __maxnreg__(sample_ff_regs(CODE)) k_sample_ff(SampleParams P, co
                 const float eps_s = P.eps_frac * (FROM64 ? ff_from_double_scaled(L, sexp).hi : f32_of_f64_trunc(L));
                 double wfinal;
                 if constexpr (CODE >= 0) {
-                    wfinal = ff_leaf_newton<(CODE >= 0 ? CODE : 0), !panel_rolled<(CODE >= 0 ? CODE : 0)>()>(
+                    wfinal = ff_leaf_newton<(CODE >= 0 ? CODE : 0)>(
                         seg, sexp, vaf, dv, rl, dS, dvg, eps_s, newton);
                 } else {
                     switch (code) {
 #define GCV_CASE(C)                                                                                \
-    case C: wfinal = ff_leaf_newton<C, false>(seg, sexp, vaf, dv, rl, dS, dvg, eps_s, newton); break;
+    case C: wfinal = ff_leaf_newton<C>(seg, sexp, vaf, dv, rl, dS, dvg, eps_s, newton); break;
                         GCV_FOR_EACH_CODE(GCV_CASE)
 #undef GCV_CASE
                     default: wfinal = dvg; break;

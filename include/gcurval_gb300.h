@@ -81,7 +81,8 @@ typedef struct gcv_options {
                              network installed with gcv_set_learned_model
                              (gcurval_gb300_learned.h); no effect without one */
     int mapping;          /* the length walk's main pass with float-float panels (GCV_MIXED):
-                             GCV_MAP_LANE (default) one thread per knot interval, or
+                             GCV_MAP_LANE (default) one thread per panel, a warp
+                             sharing its intervals' panels, or
                              GCV_MAP_HALF_WARP 16 threads per knot interval, one panel node
                              each; the same table up to the summation order of each
                              panel's nodes (float-float rounding); no effect on GCV_PLAIN_FP64 */
