@@ -12,10 +12,10 @@
 //     every curve has at least 2 degree + 1 knots) and records the first bad
 //     curve; the kernels after it return at once when it found one, so
 //     malformed offsets never steer a read outside the caller's arrays;
-//   * kernel 1, a lengths-only variant of the interval-length kernel: one
-//     thread per knot interval builds the interval's polynomial in registers
-//     and runs the same adaptive G7-K15 depth-first refinement, writing the
-//     interval's length to the scratch array (no leaf table);
+//   * kernel 1, the lengths-only form of the warp-wide walk (gcv_walk.cuh): a
+//     lane builds an interval's polynomial in shared memory when its warp
+//     takes the interval, the warp runs the same adaptive G7-K15 refinement,
+//     and the interval's length goes to the scratch array (no leaf table);
 //   * kernel 2: one thread per curve sums its intervals' lengths with
 //     double-double compensation into the caller's output.
 //
@@ -40,7 +40,8 @@
 #include <string>
 
 #include "gcv_kernels.cuh"
-#include "gcv_length_impl.cuh"
+#include "gcv_sample.cuh"
+#include "gcv_walk.cuh"
 
 extern "C" gcv_status gcv_internal_fail(gcv_status s, const char* msg);
 
@@ -50,7 +51,8 @@ using namespace gcv;
 
 constexpr int64_t NOALLOC_MAX_INTERVALS = GCV_NOALLOC_MAX_INTERVALS;
 // header words (64-bit): [0] error bits, [1] capped panels, [2] n_curve minus
-// the first curve whose offsets are bad (0: none); the rest is unused
+// the first curve whose offsets are bad (0: none), [3] the walk's work-queue
+// head; the rest is unused
 constexpr int HEADER_DOUBLES = 32;
 // beside the table's ERR_* bits: knots_offset[0] != 0, a curve with fewer
 // than 2 degree + 1 knots (decreasing offsets included)
@@ -157,45 +159,79 @@ __global__ void k_noalloc_check(int n_curve, int P, const int* __restrict__ ko, 
     }
 }
 
-template <int P, int D>
-__global__ void __launch_bounds__(128) k_noalloc_intervals(int n_curve, const int* __restrict__ ko,
-                                                           const double* __restrict__ knots,
-                                                           const double* __restrict__ ctrl, double rtol,
-                                                           int max_depth, int64_t n_seg, double* scratch)
+// the curve of interval s: the last c with first_interval(c) <= s (-1: none,
+// only with first_interval(0) > 0, which kernel 0 rules out)
+__device__ __forceinline__ int curve_of(const int* __restrict__ ko, int n_curve, int64_t s, int P)
 {
-    if (offsets_bad(scratch)) return;
-    unsigned long long capped = 0;
-    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n_seg;
-         s += (int64_t)gridDim.x * blockDim.x) {
-        // curve of interval s: the last c with first_interval(c) <= s
-        int lo = 0, cnt = n_curve;
-        while (cnt > 0) {
-            const int h = cnt >> 1;
-            if (first_interval(ko, lo + h, P) <= s) {
-                lo += h + 1;
-                cnt -= h + 1;
-            } else {
-                cnt = h;
-            }
+    int lo = 0, cnt = n_curve;
+    while (cnt > 0) {
+        const int h = cnt >> 1;
+        if (first_interval(ko, lo + h, P) <= s) {
+            lo += h + 1;
+            cnt -= h + 1;
+        } else {
+            cnt = h;
         }
-        const int c = lo - 1;
-        if (c < 0) continue;  // only with first_interval(0) > 0, which kernel 0 rules out
+    }
+    return lo - 1;
+}
+
+// The batch as k_walk takes intervals from it (PREC 3): the position
+// polynomial of interval s, built in FP64 when the walk takes it, and its
+// length into the scratch array.
+template <int P, int D>
+struct NoallocSource {
+    int n_curve;
+    const int* ko;
+    const double* knots;
+    const double* ctrl;
+    double rtol;
+    int max_depth;
+    double* scratch;
+
+    __device__ __forceinline__ bool stop() const { return offsets_bad(scratch); }
+    __device__ __forceinline__ void setup(int64_t s, double* cf) const
+    {
+#pragma unroll
+        for (int i = 0; i < (P + 1) * D; ++i) cf[i] = 0.0;
+        const int c = curve_of(ko, n_curve, s, P);
+        if (c < 0) return;
         const int span = int(s - first_interval(ko, c, P)) + P;
         const double* kv = knots + ko[c];
-        const double* cp = ctrl + ((int64_t)ko[c] - (int64_t)(P + 1) * c) * D;
         const double ka = kv[span], kb = kv[span + 1];
-        double len = 0.0;
-        if (!(kb >= ka)) {
+        if (!(kb >= ka))
             atomicOr(reinterpret_cast<unsigned long long*>(scratch), (unsigned long long)ERR_BAD_KNOTS);
-        } else if (kb > ka) {
-            double cf[(P + 1) * D], der[P * D];
-            bspline_setup<P, D>(kv, cp, span, cf);
-            Eval<bs_code(P, D)>::load_speed(cf, der);
-            len = interval_length<bs_code(P, D)>(der, rtol, max_depth, &capped);
-        }
-        scratch[HEADER_DOUBLES + s] = len;
+        else if (kb > ka)
+            bspline_setup<P, D>(kv, ctrl + ((int64_t)ko[c] - (int64_t)(P + 1) * c) * D, span, cf);
     }
-    if (capped) atomicAdd(reinterpret_cast<unsigned long long*>(scratch + 1), capped);
+    __device__ __forceinline__ void finish(int64_t s, double len) const { scratch[HEADER_DOUBLES + s] = len; }
+    // an interval with more leaves than a warp keeps: by its lane alone
+    __device__ __noinline__ void deep(int64_t s, const double* cf) const
+    {
+        double der[P * D];
+        Eval<bs_code(P, D)>::load_speed(cf, der);
+        unsigned long long capped = 0;
+        finish(s, interval_length<bs_code(P, D)>(der, rtol, max_depth, &capped));
+        if (capped) count_capped(capped);
+    }
+    __device__ __forceinline__ void count_capped(unsigned long long n) const
+    {
+        atomicAdd(reinterpret_cast<unsigned long long*>(scratch + 1), n);
+    }
+};
+
+// one thread per interval, all FP64: below PLAIN_SPLIT_RTOL or above
+// FF_MAX_DEPTH, where the float-float partition of k_walk does not reach
+template <int P, int D>
+__global__ void __launch_bounds__(128) k_noalloc_intervals(NoallocSource<P, D> src, int64_t n_seg)
+{
+    if (offsets_bad(src.scratch)) return;
+    for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n_seg;
+         s += (int64_t)gridDim.x * blockDim.x) {
+        double cf[(P + 1) * D];
+        src.setup(s, cf);
+        src.deep(s, cf);
+    }
 }
 
 __global__ void k_noalloc_curves(int n_curve, int P, const int* __restrict__ ko, int64_t n_seg,
@@ -221,10 +257,22 @@ cudaError_t launch(int n_curve, const int* ko, const double* knots, const double
     int dev = 0, sms = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int64_t want = (n_seg + 127) / 128;
-    const int grid = (int)(want < (int64_t)sms * 16 ? (want > 0 ? want : 1) : (int64_t)sms * 16);
-    k_noalloc_intervals<P, D><<<grid, 128, 0, st>>>(n_curve, ko, knots, ctrl, rtol, max_depth, n_seg, scratch);
-    return cudaGetLastError();
+    const NoallocSource<P, D> src{n_curve, ko, knots, ctrl, rtol, max_depth, scratch};
+    if (rtol < PLAIN_SPLIT_RTOL || max_depth > FF_MAX_DEPTH) {
+        const int64_t want = (n_seg + 127) / 128;
+        const int grid = (int)(want < (int64_t)sms * 16 ? (want > 0 ? want : 1) : (int64_t)sms * 16);
+        k_noalloc_intervals<P, D><<<grid, 128, 0, st>>>(src, n_seg);
+        return cudaGetLastError();
+    }
+    // the warp-wide walk: one thread per interval lasted as long as the
+    // deepest interval of each warp (999,424 cubic intervals at 1e-10: 12.17 ms,
+    // here 1.45 ms)
+    LengthParams L{};
+    L.rtol = rtol;
+    L.max_depth = max_depth;
+    L.n_items = n_seg;
+    L.work = reinterpret_cast<unsigned long long*>(scratch + 3);
+    return walk_launch<bs_code(P, D), 3>(L, st, sms, 32, src);
 }
 
 }  // namespace

@@ -47,15 +47,15 @@ enum WalkDead {
     WK_PLAIN = 3   // more than LCAP leaves from its learned start: once more from the whole interval
 };
 
-// node key: dyadic panel (k, depth), and whether the learned start depths
-// still have to be looked at
+// node key: dyadic panel (k, depth), whether the learned start depths still have
+// to be looked at, and whether a leaf was accepted short of the tolerance
 constexpr unsigned long long WK_K_MASK = (1ull << 56) - 1;
-constexpr unsigned long long WK_FLAG = 1ull << 63;
+constexpr unsigned long long WK_FLAG = 1ull << 63, WK_CAPPED = 1ull << 62;
 __device__ __forceinline__ unsigned long long wk_key(unsigned long long k, int depth, bool flag)
 {
     return k | ((unsigned long long)depth << 56) | (flag ? WK_FLAG : 0ull);
 }
-__device__ __forceinline__ int wk_depth(unsigned long long key) { return (int)(key >> 56) & 0x7F; }
+__device__ __forceinline__ int wk_depth(unsigned long long key) { return (int)(key >> 56) & 0x3F; }
 
 struct WalkWarp {
     unsigned long long key[WK_NODES];
@@ -119,17 +119,27 @@ __host__ __device__ constexpr int walk_blocks(int code)
 
 // PREC 1: float-float table, K15 in float-float; PREC 2: FP64 table, the
 // partition from float-float panels with the FP64 test near the tolerance, and
-// K15 of every leaf in FP64 (leaf_k15).
-template <int CODE, int PREC>
-__global__ void __launch_bounds__(WK_THREADS, walk_blocks(CODE)) k_walk(LengthParams P)
+// K15 of every leaf in FP64 (leaf_k15); PREC 3: the same without a table, for
+// callers that only want the intervals' lengths: `src` gives an interval's
+// FP64 coefficients when the walk takes it (kept in shared memory) and receives
+// its length.
+struct NoSource {};
+template <int CODE, int PREC, typename SRC = NoSource>
+__global__ void __launch_bounds__(WK_THREADS, PREC == 3 ? 6 : walk_blocks(CODE)) k_walk(LengthParams P, SRC src = SRC{})
 {
     __shared__ WalkWarp s_walk[WK_THREADS / 32];
+    // PREC 3: the slots' coefficients (an odd stride keeps the lanes' banks apart)
+    constexpr int SLOT_COEF = code_stride(CODE) | 1;
+    __shared__ double s_coef[WK_THREADS / 32][PREC == 3 ? WK_SLOTS * SLOT_COEF : 1];
     const Table& t = P.t;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
     WalkWarp& W = s_walk[threadIdx.x >> 5];
     constexpr int STRIDE = code_stride(CODE);
+    if constexpr (PREC == 3) {
+        if (src.stop()) return;
+    }
     const double eps50 = 50.0 * 1.4210854715202004e-14;  // 50 float-float units
     const float rtolf = (float)P.rtol;
 
@@ -145,12 +155,19 @@ __global__ void __launch_bounds__(WK_THREADS, walk_blocks(CODE)) k_walk(LengthPa
     unsigned long long my_panels = 0;
     unsigned my_capped = 0, my_nonfinite = 0;
 
-    auto load = [&](int item, int sexp, ff* r) {
-        const int64_t ci = P.coef_base + (int64_t)item * STRIDE;
-        if constexpr (PREC == 1)
-            EvalFF<CODE>::load(P.coef_ff + ci, r);
+    double* slot_coef = s_coef[threadIdx.x >> 5];
+    // FP64 coefficients of the interval in a slot
+    auto coef64 = [&](int sl) -> const double* {
+        if constexpr (PREC == 3)
+            return slot_coef + sl * SLOT_COEF;
         else
-            EvalFF<CODE>::load(t.coef + ci, r, sexp);
+            return t.coef + P.coef_base + (int64_t)W.item[sl] * STRIDE;
+    };
+    auto load = [&](int sl, ff* r) {
+        if constexpr (PREC == 1)
+            EvalFF<CODE>::load(P.coef_ff + P.coef_base + (int64_t)W.item[sl] * STRIDE, r);
+        else
+            EvalFF<CODE>::load(coef64(sl), r, W.sexp[sl]);
     };
     auto to_deep = [&](int s) {
         const unsigned long long o = atomicAdd(t.ctr + C_DEEP, 1ull);
@@ -186,17 +203,14 @@ __global__ void __launch_bounds__(WK_THREADS, walk_blocks(CODE)) k_walk(LengthPa
                     const int item = (int)base + lane;
                     const int sl = W.fslot[nslot - 1 - lane], nd = W.freel[nfree - 1 - lane];
                     W.item[sl] = item;
-                    int sexp = 0;
-                    if constexpr (PREC == 2) {
-                        sexp = interval_exponent<CODE>(t.coef + P.coef_base + (int64_t)item * STRIDE);
-                        W.sexp[sl] = sexp;
-                    }
+                    if constexpr (PREC == 3) src.setup(item, slot_coef + sl * SLOT_COEF);
+                    if constexpr (PREC >= 2) W.sexp[sl] = interval_exponent<CODE>(coef64(sl));
                     uint32_t dq = 0;
-                    if constexpr (CODE > 0) {
+                    if constexpr (CODE > 0 && PREC != 3) {
                         // learned start: the predicted depths, tolerance from the chord
                         if (P.starts && (dq = P.starts[item]) != 0u) {
                             ff r[MAX_COEF];
-                            load(item, sexp, r);
+                            load(sl, r);
                             const float ch = chord_of<CODE>(r);
                             W.tolf[sl] = rtolf * ch;
                             W.whole[sl] = pack_ff(ff{ch, 0.0f});
@@ -269,7 +283,7 @@ __global__ void __launch_bounds__(WK_THREADS, walk_blocks(CODE)) k_walk(LengthPa
             __syncwarp(FULL);
             return none_left;
         };
-        if constexpr (CODE > 0) {
+        if constexpr (CODE > 0 && PREC != 3) {
             if (P.starts) {
                 // down to the learned start depths without evaluating
                 for (int guard = 0; guard < 16; ++guard) {
@@ -288,7 +302,7 @@ __global__ void __launch_bounds__(WK_THREADS, walk_blocks(CODE)) k_walk(LengthPa
         bool reject = false;
         if (active && !dead) {
             ff r[MAX_COEF], Kf, Gf;
-            load(W.item[sl], PREC == 2 ? W.sexp[sl] : 0, r);
+            load(sl, r);
             panel_ff<CODE>(r, k, depth, Kf, Gf);
             const float hwf = __int_as_float((127 - depth) << 23);  // 2^-depth
             if (depth == 0) {
@@ -320,15 +334,14 @@ __global__ void __launch_bounds__(WK_THREADS, walk_blocks(CODE)) k_walk(LengthPa
                 else if (errf - noise > 1.01f * thr)
                     ok = false;
                 else
-                    ok = !finite || accept_fp64<CODE>(t.coef + P.coef_base + (int64_t)W.item[sl] * STRIDE, k, depth,
+                    ok = !finite || accept_fp64<CODE>(coef64(sl), k, depth,
                                                       depth == 0 ? P.rtol : scalbn(tolerance(), W.sexp[sl]));
             }
             ++my_panels;
             if (ok || depth >= P.max_depth || !finite) {
-                my_capped += !ok && finite;
                 my_nonfinite += !finite;
                 W.val[nd] = pack_ff(Kf);
-                W.key[nd] = key;
+                W.key[nd] = !ok && finite ? key | WK_CAPPED : key;
             } else {
                 reject = true;
             }
@@ -375,11 +388,13 @@ __global__ void __launch_bounds__(WK_THREADS, walk_blocks(CODE)) k_walk(LengthPa
             const int cnt = gone ? 0 : nodes;
             const int incl = warp_incl_scan(cnt, lane), total = __shfl_sync(FULL, incl, 31);
             unsigned long long base = 0;
-            if (lane == 0) base = atomicAdd(t.ctr + C_LEAF_TOP, (unsigned long long)total);
-            base = __shfl_sync(FULL, base, 0);
+            if constexpr (PREC != 3) {
+                if (lane == 0) base = atomicAdd(t.ctr + C_LEAF_TOP, (unsigned long long)total);
+                base = __shfl_sync(FULL, base, 0);
+            }
             const int first = incl - cnt;
             const int64_t off = (int64_t)base + first;
-            const bool fits = !gone && off + cnt <= t.leaf_cap;
+            const bool fits = !gone && (PREC == 3 || off + cnt <= t.leaf_cap);
             if (mine) {
                 W.fits[fs] = fits;
                 int q = W.head[fs];
@@ -389,14 +404,13 @@ __global__ void __launch_bounds__(WK_THREADS, walk_blocks(CODE)) k_walk(LengthPa
                 }
             }
             __syncwarp(FULL);
-            if constexpr (PREC == 2) {
+            if constexpr (PREC >= 2) {
                 for (int g = lane; g < total; g += 32) {
                     const int q = W.order[g], qs = W.slot[q];
                     const ff kf = unpack_ff(W.val[q]);
                     double K = ff_to_double(kf);
                     if (W.fits[qs] && isfinite(kf.hi))
-                        K = leaf_k15<CODE>(t.coef + P.coef_base + (int64_t)W.item[qs] * STRIDE, W.sexp[qs],
-                                           W.key[q] & WK_K_MASK, wk_depth(W.key[q]));
+                        K = leaf_k15<CODE>(coef64(qs), W.sexp[qs], W.key[q] & WK_K_MASK, wk_depth(W.key[q]));
                     W.val[q] = K;
                 }
                 __syncwarp(FULL);
@@ -414,8 +428,13 @@ __global__ void __launch_bounds__(WK_THREADS, walk_blocks(CODE)) k_walk(LengthPa
                     }
                     W.val[q] = cum;
                 }
-                const int s = P.list ? P.list[W.item[fs]] : W.item[fs];
-                if (why == WK_DEEP) {
+                const int s = PREC != 3 && P.list ? P.list[W.item[fs]] : W.item[fs];
+                if constexpr (PREC == 3) {
+                    if (why == WK_DEEP)
+                        src.deep(s, coef64(fs));
+                    else if (!gone)
+                        src.finish(s, cum);
+                } else if (why == WK_DEEP) {
                     to_deep(s);
                 } else if (!gone) {
                     // a full pool: the pass is run again with a larger one
@@ -428,19 +447,19 @@ __global__ void __launch_bounds__(WK_THREADS, walk_blocks(CODE)) k_walk(LengthPa
             __syncwarp(FULL);
             for (int g = lane; g < total; g += 32) {
                 const int q = W.order[g], qs = W.slot[q];
-                if (W.fits[qs]) {
-                    const unsigned long long qk = W.key[q];
+                const unsigned long long qk = W.key[q];
+                my_capped += (qk & WK_CAPPED) != 0ull;
+                if (PREC != 3 && W.fits[qs]) {
                     const int qd = wk_depth(qk);
                     // right end -1 + (k + 1) 2^(1 - depth): exact
                     const double vr = fma(__ull2double_rn((qk & WK_K_MASK) + 1), 2.0 * pow2_neg(qd), -1.0);
                     ff r[MAX_COEF];
-                    const int se = PREC == 2 ? W.sexp[qs] : 0;
-                    load(W.item[qs], se, r);
+                    load(qs, r);
                     float q32;
                     float f32 = EvalFF<CODE>::speed_slope32(r, f32_of_f64_trunc(vr), q32);
                     if constexpr (PREC == 2) {
-                        f32 = scale_down(f32, -se);
-                        q32 = scale_down(q32, -2 * se);
+                        f32 = scale_down(f32, -W.sexp[qs]);
+                        q32 = scale_down(q32, -2 * W.sexp[qs]);
                     }
                     t.leaf_v[base + g] = vr;
                     t.leaf_cum[base + g] = W.val[q];
@@ -485,18 +504,20 @@ __global__ void __launch_bounds__(WK_THREADS, walk_blocks(CODE)) k_walk(LengthPa
         capped += __shfl_xor_sync(FULL, capped, o);
         nonfinite += __shfl_xor_sync(FULL, nonfinite, o);
     }
-    if (lane == 0) {
+    if constexpr (PREC == 3) {
+        if (lane == 0 && capped) src.count_capped(capped);
+    } else if (lane == 0) {
         if (P.collect && my_panels) atomicAdd(t.ctr + C_PANELS, my_panels);
         if (capped) atomicAdd(t.ctr + C_CAPPED, capped);
         if (nonfinite) atomicAdd(t.ctr + C_NONFINITE, nonfinite);
     }
 }
 
-template <int CODE, int PREC>
-cudaError_t walk_launch(const LengthParams& P, cudaStream_t stream, int sm_count, int blocks_per_sm_cap)
+template <int CODE, int PREC, typename SRC>
+cudaError_t walk_launch(const LengthParams& P, cudaStream_t stream, int sm_count, int blocks_per_sm_cap, SRC src)
 {
     int occ = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_walk<CODE, PREC>, WK_THREADS, 0);
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_walk<CODE, PREC, SRC>, WK_THREADS, 0);
     if (e != cudaSuccess) return e;
     const int cap = blocks_per_sm_cap < 1 ? 1 : blocks_per_sm_cap;
     occ = occ < 1 ? 1 : (occ > cap ? cap : occ);
@@ -505,8 +526,13 @@ cudaError_t walk_launch(const LengthParams& P, cudaStream_t stream, int sm_count
     int64_t grid = (int64_t)sm_count * occ;
     if (want < grid) grid = want;
     if (grid < 1) grid = 1;
-    k_walk<CODE, PREC><<<(unsigned)grid, WK_THREADS, 0, stream>>>(P);
+    k_walk<CODE, PREC, SRC><<<(unsigned)grid, WK_THREADS, 0, stream>>>(P, src);
     return cudaGetLastError();
+}
+template <int CODE, int PREC>
+cudaError_t walk_launch(const LengthParams& P, cudaStream_t stream, int sm_count, int blocks_per_sm_cap)
+{
+    return walk_launch<CODE, PREC, NoSource>(P, stream, sm_count, blocks_per_sm_cap, NoSource{});
 }
 
 // the mixed and the FP64 walk of one curve code

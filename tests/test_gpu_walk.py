@@ -147,3 +147,24 @@ def test_work_sharing_does_not_change_the_table(network, gpu_lib):
     for L, u in out[1:]:
         np.testing.assert_array_equal(L, out[0][0])
         np.testing.assert_array_equal(u, out[0][1])
+
+
+@pytest.mark.parametrize("rtol,max_depth", [(1e-9, 30), (1e-12, 44), (1e-12, 45), (0.9e-12, 44), (1e-9, 3)])
+@pytest.mark.parametrize("n", [1, 5, 300])
+def test_lengths_without_a_table(n, rtol, max_depth, gpu_lib):
+    """gcv_bspline_lengths_noalloc on both sides of its rule, against the walk in NumPy."""
+    import ctypes
+
+    torch = pytest.importorskip("torch")
+    ref = Cusps(n, 3, seed=n + 1)
+    b = ref.batch
+    ko = torch.from_numpy(b.knot_off.astype(np.int32)).cuda()
+    kv, cp = torch.from_numpy(b.knots).cuda(), torch.from_numpy(b.ctrl).cuda()
+    out = torch.empty(n, dtype=torch.float64, device="cuda")
+    capped = ctypes.c_int64()
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    assert gpu_lib.gcv_bspline_lengths_noalloc(n, 5, 2, p(ko), p(kv), p(cp), rtol, max_depth, p(out), None,
+                                               ctypes.byref(capped)) == 0
+    want = np.array([ref.walk(i, rtol, max_depth, 2.0 ** -52) for i in range(n)])
+    assert np.max(np.abs(out.cpu().numpy() - want[:, 0]) / want[:, 0]) <= rtol + 1e-13
+    assert abs(capped.value - want[:, 2].sum()) <= 0.002 * want[:, 2].sum()
