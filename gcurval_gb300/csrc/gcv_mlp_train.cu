@@ -7,6 +7,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <random>
@@ -22,52 +23,6 @@ namespace {
 thread_local std::string g_err_train;
 
 // ---------------------------------------------------------------- kernels
-constexpr int GB = 64, GK = 16;  // SGEMM tile: 64 x 64 outputs, K step 16, 256 threads
-
-// C[M x N] = op(A)[M x K] op(B)[K x N], row-major storage:
-// op(A)[m][k] = TA ? A[k * lda + m] : A[m * lda + k]; likewise B with TB.
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(256) k_sgemm(int M, int N, int K, const float* __restrict__ A, int lda,
-                                               const float* __restrict__ B, int ldb, float* __restrict__ C, int ldc)
-{
-    __shared__ float As[GK][GB + 4];
-    __shared__ float Bs[GK][GB + 4];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int m0 = blockIdx.y * GB, n0 = blockIdx.x * GB;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += GK) {
-        for (int i = threadIdx.x; i < GK * GB; i += 256) {
-            const int kk = i / GB, mm = i % GB;
-            const int m = m0 + mm, k = k0 + kk;
-            As[kk][mm] = (m < M && k < K) ? (TA ? A[(size_t)k * lda + m] : A[(size_t)m * lda + k]) : 0.0f;
-            const int n = n0 + mm;
-            Bs[kk][mm] = (n < N && k < K) ? (TB ? B[(size_t)n * ldb + k] : B[(size_t)k * ldb + n]) : 0.0f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < GK; ++kk) {
-            float a[4], bb[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                a[i] = As[kk][ty * 4 + i];
-                bb[i] = Bs[kk][tx * 4 + i];
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], bb[j], acc[i][j]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
-            if (m < M && n < N) C[(size_t)m * ldc + n] = acc[i][j];
-        }
-}
-
 __device__ __forceinline__ float gelu(float x, float& t)
 {
     t = tanhf(GELU_C * (x + GELU_A * x * x * x));
@@ -80,24 +35,146 @@ __device__ __forceinline__ float gelu_grad(float x)
     return 0.5f * (1.0f + t) + 0.5f * x * (1.0f - t * t) * GELU_C * (1.0f + 3.0f * GELU_A * x * x);
 }
 
-// Z += bias (per column); H = GELU(Z) when act
-__global__ void k_bias_act(float* Z, float* H, const float* bias, int n, int cols, int act)
+// SGEMM tile: 64 x 64 outputs, K step 16, 256 threads of 4 x 4 outputs; the next
+// step's operands are loaded into registers while the current one is summed.
+constexpr int GB = 64, GK = 16;
+
+// what happens to an output tile
+enum Epilogue {
+    EP_BIAS,       // C = AB + bias
+    EP_BIAS_GELU,  // C = AB + bias, H = GELU(C)
+    EP_ACT_GRAD,   // C = AB * GELU'(Z)
+    EP_PARTIAL     // split K: chunk z's sums to C + z * stride, and below the last row the column sums of B
+};
+
+struct GemmArgs {
+    int M, N, K;
+    const float *A, *B;
+    int lda, ldb;
+    float* C;  // row-major, N columns
+    const float* aux;  // EP_BIAS*: bias [N]; EP_ACT_GRAD: Z [M x N]
+    float* H;
+    int chunk;      // EP_PARTIAL: rows of K per chunk (a multiple of GK)
+    size_t stride;  // EP_PARTIAL: floats between the chunks' results
+};
+
+// 4 consecutive floats; vec: p is 16-byte aligned
+__device__ __forceinline__ float4 load4(const float* __restrict__ p, bool vec)
 {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < (size_t)n * cols; i += (size_t)gridDim.x * blockDim.x) {
-        const float z = Z[i] + bias[i % cols];
-        Z[i] = z;
-        if (act) {
-            float t;
-            H[i] = gelu(z, t);
+    return vec ? *reinterpret_cast<const float4*>(p) : make_float4(p[0], p[1], p[2], p[3]);
+}
+
+// C[M x N] = op(A)[M x K] op(B)[K x N], row-major storage:
+// op(A)[m][k] = TA ? A[k * lda + m] : A[m * lda + k]; likewise B with TB.
+// The contiguous extents (K of a plain A or transposed B, M and N otherwise)
+// are multiples of 4.
+//
+// What bounds it: latency and the number of blocks, not FP32 throughput.  The
+// weight gradients sum over the batch's rows into 16 x 128 .. 128 x 128 outputs,
+// one to four tiles: split over K they fill the GPU, and a plain operand is read
+// 16 bytes a lane along its rows (it was read column by column).  A batch
+// of 8,192 rows: weight gradients 4 x 1,350 us -> 4 x 9-13 us, bias gradients (one block,
+// one thread per column) 4 x 460 us -> part of the same pass; bias, GELU and its
+// derivative in the epilogues instead of passes of their own (all under ncu; a call
+// of gcv_mlp_trainer_gradients 4.21 -> 0.20 ms).
+template <bool TA, bool TB, Epilogue EP>
+__global__ void __launch_bounds__(256) k_sgemm(GemmArgs g)
+{
+    __shared__ __align__(16) float As[GK][GB + 4];
+    __shared__ __align__(16) float Bs[GK][GB + 4];
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int m0 = blockIdx.y * GB, n0 = blockIdx.x * GB;
+    const int k_begin = EP == EP_PARTIAL ? blockIdx.z * g.chunk : 0;
+    const int k_end = EP == EP_PARTIAL ? min(g.K, k_begin + g.chunk) : g.K;
+    const bool vec_a = ((reinterpret_cast<size_t>(g.A) | (size_t)g.lda * 4) & 15) == 0;
+    const bool vec_b = ((reinterpret_cast<size_t>(g.B) | (size_t)g.ldb * 4) & 15) == 0;
+    // an operand stored along k: thread -> row tid % 64, k quad tid / 64;
+    // stored across k: k row tid / 16, quad tid % 16
+    auto fetch = [&](const float* X, int ld, bool along_k, int row0, int rows, int k0, bool vec) {
+        const int r = row0 + (along_k ? tid & 63 : 4 * (tid & 15)), k = k0 + (along_k ? 4 * (tid >> 6) : tid >> 4);
+        if (r >= rows || k >= k_end) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        return load4(along_k ? X + (size_t)r * ld + k : X + (size_t)k * ld + r, vec);
+    };
+    auto stage = [&](float (*S)[GB + 4], bool along_k, float4 v) {
+        if (along_k) {
+            const int r = tid & 63, k = 4 * (tid >> 6);
+            S[k][r] = v.x;
+            S[k + 1][r] = v.y;
+            S[k + 2][r] = v.z;
+            S[k + 3][r] = v.w;
+        } else {
+            *reinterpret_cast<float4*>(&S[tid >> 4][4 * (tid & 15)]) = v;
+        }
+    };
+    float acc[4][4] = {};
+    float col[4] = {};  // EP_PARTIAL: column sums of B over this thread's share of k (k % 16 == ty)
+    float4 a4 = fetch(g.A, g.lda, !TA, m0, g.M, k_begin, vec_a);
+    float4 b4 = fetch(g.B, g.ldb, TB, n0, g.N, k_begin, vec_b);
+    for (int k0 = k_begin; k0 < k_end; k0 += GK) {
+        stage(As, !TA, a4);
+        stage(Bs, TB, b4);
+        __syncthreads();
+        if (k0 + GK < k_end) {
+            a4 = fetch(g.A, g.lda, !TA, m0, g.M, k0 + GK, vec_a);
+            b4 = fetch(g.B, g.ldb, TB, n0, g.N, k0 + GK, vec_b);
+        }
+#pragma unroll
+        for (int kk = 0; kk < GK; ++kk) {
+            const float4 av = *reinterpret_cast<const float4*>(&As[kk][ty * 4]);
+            const float4 bv = *reinterpret_cast<const float4*>(&Bs[kk][tx * 4]);
+            const float a[4] = {av.x, av.y, av.z, av.w}, bb[4] = {bv.x, bv.y, bv.z, bv.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], bb[j], acc[i][j]);
+        }
+        if constexpr (EP == EP_PARTIAL) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) col[j] += Bs[ty][tx * 4 + j];
+        }
+        __syncthreads();
+    }
+    float* C = EP == EP_PARTIAL ? g.C + blockIdx.z * g.stride : g.C;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
+            if (m >= g.M || n >= g.N) continue;
+            const size_t at = (size_t)m * g.N + n;
+            float v = acc[i][j];
+            if constexpr (EP == EP_BIAS || EP == EP_BIAS_GELU) v += g.aux[n];
+            if constexpr (EP == EP_ACT_GRAD) v *= gelu_grad(g.aux[at]);
+            C[at] = v;
+            if constexpr (EP == EP_BIAS_GELU) {
+                float t;
+                g.H[at] = gelu(v, t);
+            }
+        }
+    if constexpr (EP == EP_PARTIAL) {
+        if (blockIdx.y == 0) {  // the 16 threads of a column, added in a fixed order
+#pragma unroll
+            for (int j = 0; j < 4; ++j) As[ty][tx * 4 + j] = col[j];
+            __syncthreads();
+            if (tid < GB && n0 + tid < g.N) {
+                float s = 0.0f;
+#pragma unroll
+                for (int k = 0; k < GK; ++k) s += As[k][tid];
+                C[(size_t)g.M * g.N + n0 + tid] = s;
+            }
         }
     }
 }
 
-// dZ = dH * GELU'(Z)
-__global__ void k_act_grad(const float* dH, const float* Z, float* dZ, size_t count)
+// g[i] = the sum of the chunks' partial gradients, in chunk order
+__global__ void k_sum_partials(const float* __restrict__ part, int chunks, int count, float* __restrict__ g)
 {
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < count; i += (size_t)gridDim.x * blockDim.x)
-        dZ[i] = dH[i] * gelu_grad(Z[i]);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    float s = 0.0f;
+#pragma unroll 8
+    for (int c = 0; c < chunks; ++c) s += part[(size_t)c * count + i];
+    g[i] = s;
 }
 
 // loss parts (sums over the batch) and dOut = d(mean loss) / d out
@@ -148,16 +225,6 @@ __global__ void k_loss(const float* out, const int* depth, const float* share, c
     }
 }
 
-// db[c] = sum over rows of dZ[r][c] (one thread per column, rows strided)
-__global__ void k_colsum(const float* dZ, int n, int cols, float* db)
-{
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    float s = 0.0f;
-    for (int r = 0; r < n; ++r) s += dZ[(size_t)r * cols + c];
-    db[c] = s;
-}
-
 __global__ void k_adam(float* w, const float* g, float* m, float* v, int count, float lr, float b1, float b2, float eps,
                        float c1, float c2)
 {
@@ -171,11 +238,20 @@ __global__ void k_adam(float* w, const float* g, float* m, float* v, int count, 
     }
 }
 
-template <bool TA, bool TB>
-void sgemm(int M, int N, int K, const float* A, int lda, const float* B, int ldb, float* C, int ldc, cudaStream_t st)
+template <bool TA, bool TB, Epilogue EP>
+void sgemm(const GemmArgs& g, int chunks, cudaStream_t st)
 {
-    dim3 grid((N + GB - 1) / GB, (M + GB - 1) / GB);
-    k_sgemm<TA, TB><<<grid, 256, 0, st>>>(M, N, K, A, lda, B, ldb, C, ldc);
+    dim3 grid((g.N + GB - 1) / GB, (g.M + GB - 1) / GB, chunks);
+    k_sgemm<TA, TB, EP><<<grid, 256, 0, st>>>(g);
+}
+
+// chunks of rows the weight gradients are summed in: up to GRAD_CHUNKS, of at
+// least 64 rows (with two to four tiles each, 64 chunks fill 152 SMs)
+constexpr int GRAD_CHUNKS = 64;
+int grad_chunk_rows(int n)
+{
+    const int rows = std::max(64, (n + GRAD_CHUNKS - 1) / GRAD_CHUNKS);
+    return (rows + GK - 1) / GK * GK;
 }
 
 unsigned blocks_for(size_t n) { return (unsigned)std::min<size_t>((n + 255) / 256, 152 * 32); }
@@ -187,6 +263,7 @@ struct gcv_mlp_trainer {
     cudaStream_t st = nullptr;
     float *w = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
     float *Z[3] = {}, *H[3] = {}, *out = nullptr, *dOut = nullptr, *dA = nullptr, *dB = nullptr, *loss3 = nullptr;
+    float* part = nullptr;  // GRAD_CHUNKS partial gradients, each packed like w
     long long step = 0;
 };
 
@@ -204,41 +281,48 @@ gcv_status tfail(gcv_status s, const std::string& m)
         if (e_ != cudaSuccess) return tfail(GCV_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
+constexpr int OFF_W[4] = {MLP_OFF_W1, MLP_OFF_W2, MLP_OFF_W3, MLP_OFF_W4};
+constexpr int OFF_B[4] = {MLP_OFF_B1, MLP_OFF_B2, MLP_OFF_B3, MLP_OFF_B4};
+static_assert(MLP_OFF_B1 == MLP_OFF_W1 + MLP_IN * MLP_H && MLP_OFF_B4 == MLP_OFF_W4 + MLP_H * MLP_OUT,
+              "a layer's bias gradient follows its weights' like a last row");
+
 // forward pass of n rows of X into tr->Z / H / out
 void forward(gcv_mlp_trainer* tr, const float* X, int n)
 {
     const float* in = X;
     int fan = MLP_IN;
-    const int offW[3] = {MLP_OFF_W1, MLP_OFF_W2, MLP_OFF_W3}, offB[3] = {MLP_OFF_B1, MLP_OFF_B2, MLP_OFF_B3};
     for (int l = 0; l < 3; ++l) {
-        sgemm<false, false>(n, MLP_H, fan, in, fan, tr->w + offW[l], MLP_H, tr->Z[l], MLP_H, tr->st);
-        k_bias_act<<<blocks_for((size_t)n * MLP_H), 256, 0, tr->st>>>(tr->Z[l], tr->H[l], tr->w + offB[l], n, MLP_H, 1);
+        sgemm<false, false, EP_BIAS_GELU>(GemmArgs{n, MLP_H, fan, in, tr->w + OFF_W[l], fan, MLP_H, tr->Z[l],
+                                                   tr->w + OFF_B[l], tr->H[l]}, 1, tr->st);
         in = tr->H[l];
         fan = MLP_H;
     }
-    sgemm<false, false>(n, MLP_OUT, MLP_H, in, MLP_H, tr->w + MLP_OFF_W4, MLP_OUT, tr->out, MLP_OUT, tr->st);
-    k_bias_act<<<blocks_for((size_t)n * MLP_OUT), 256, 0, tr->st>>>(tr->out, nullptr, tr->w + MLP_OFF_B4, n, MLP_OUT, 0);
+    sgemm<false, false, EP_BIAS>(GemmArgs{n, MLP_OUT, MLP_H, in, tr->w + OFF_W[3], MLP_H, MLP_OUT, tr->out,
+                                          tr->w + OFF_B[3]}, 1, tr->st);
 }
 
 // loss and gradients of the mean loss into tr->g
 void backward(gcv_mlp_trainer* tr, const float* X, const int* depth, const float* share, const float* tg, int n)
 {
     cudaMemsetAsync(tr->loss3, 0, 3 * sizeof(float), tr->st);
-    k_loss<<<blocks_for((size_t)n), 256, 0, tr->st>>>(tr->out, depth, share, tg, n, tr->dOut, tr->loss3);
-    // output layer
-    sgemm<true, false>(MLP_H, MLP_OUT, n, tr->H[2], MLP_H, tr->dOut, MLP_OUT, tr->g + MLP_OFF_W4, MLP_OUT, tr->st);
-    k_colsum<<<1, 64, 0, tr->st>>>(tr->dOut, n, MLP_OUT, tr->g + MLP_OFF_B4);
-    sgemm<false, true>(n, MLP_H, MLP_OUT, tr->dOut, MLP_OUT, tr->w + MLP_OFF_W4, MLP_OUT, tr->dA, MLP_H, tr->st);
-    const int offW[3] = {MLP_OFF_W1, MLP_OFF_W2, MLP_OFF_W3}, offB[3] = {MLP_OFF_B1, MLP_OFF_B2, MLP_OFF_B3};
-    for (int l = 2; l >= 0; --l) {
-        // dA = dH of layer l -> dB = dZ
-        k_act_grad<<<blocks_for((size_t)n * MLP_H), 256, 0, tr->st>>>(tr->dA, tr->Z[l], tr->dB, (size_t)n * MLP_H);
+    k_loss<<<(unsigned)std::min<size_t>(((size_t)n + 63) / 64, 152 * 32), 64, 0, tr->st>>>(tr->out, depth, share, tg, n,
+                                                                                          tr->dOut, tr->loss3);
+    const int rows = grad_chunk_rows(n), chunks = (n + rows - 1) / rows;
+    const float* dz = tr->dOut;  // d loss / d (layer l's output before its activation)
+    float* bufs[2] = {tr->dA, tr->dB};
+    for (int l = 3; l >= 0; --l) {
         const float* in = l ? tr->H[l - 1] : X;
-        const int fan = l ? MLP_H : MLP_IN;
-        sgemm<true, false>(fan, MLP_H, n, in, fan, tr->dB, MLP_H, tr->g + offW[l], MLP_H, tr->st);
-        k_colsum<<<1, MLP_H, 0, tr->st>>>(tr->dB, n, MLP_H, tr->g + offB[l]);
-        if (l) sgemm<false, true>(n, MLP_H, MLP_H, tr->dB, MLP_H, tr->w + offW[l], MLP_H, tr->dA, MLP_H, tr->st);
+        const int fan = l ? MLP_H : MLP_IN, cols = l == 3 ? MLP_OUT : MLP_H;
+        sgemm<true, false, EP_PARTIAL>(GemmArgs{fan, cols, n, in, dz, fan, cols, tr->part + OFF_W[l], nullptr, nullptr,
+                                                rows, MLP_NPARAM}, chunks, tr->st);
+        if (l) {
+            float* next = bufs[l & 1];
+            sgemm<false, true, EP_ACT_GRAD>(GemmArgs{n, MLP_H, cols, dz, tr->w + OFF_W[l], cols, cols, next, tr->Z[l - 1]},
+                                            1, tr->st);
+            dz = next;
+        }
     }
+    k_sum_partials<<<(MLP_NPARAM + 127) / 128, 128, 0, tr->st>>>(tr->part, chunks, MLP_NPARAM, tr->g);
 }
 
 }  // namespace
@@ -270,6 +354,7 @@ gcv_status gcv_mlp_trainer_create(gcv_mlp_trainer** out, int max_batch, unsigned
     if (e == cudaSuccess) e = cudaMalloc(&tr->dA, A);
     if (e == cudaSuccess) e = cudaMalloc(&tr->dB, A);
     if (e == cudaSuccess) e = cudaMalloc(&tr->loss3, 3 * sizeof(float));
+    if (e == cudaSuccess) e = cudaMalloc(&tr->part, GRAD_CHUNKS * P);
     if (e != cudaSuccess) {
         gcv_mlp_trainer_destroy(tr);
         return tfail(GCV_ERR_OUT_OF_MEMORY, std::string("trainer buffers: ") + cudaGetErrorString(e));
@@ -298,7 +383,7 @@ gcv_status gcv_mlp_trainer_destroy(gcv_mlp_trainer* tr)
 {
     if (!tr) return GCV_OK;
     float* bufs[] = {tr->w, tr->g, tr->m, tr->v, tr->Z[0], tr->Z[1], tr->Z[2], tr->H[0], tr->H[1], tr->H[2],
-                     tr->out, tr->dOut, tr->dA, tr->dB, tr->loss3};
+                     tr->out, tr->dOut, tr->dA, tr->dB, tr->loss3, tr->part};
     for (float* b : bufs)
         if (b) cudaFree(b);
     delete tr;
