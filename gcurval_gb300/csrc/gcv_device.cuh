@@ -401,6 +401,19 @@ __device__ __forceinline__ int64_t lower_bound_key(const double* __restrict__ a,
     return lo;
 }
 
+// the same over n entries from a, as an offset in 32 bits
+__device__ __forceinline__ int lower_bound_key32(const double* __restrict__ a, int n, long long key)
+{
+    int lo = 0;
+    while (n > 0) {
+        const int h = n >> 1;
+        const bool less = dkey(__ldg(a + lo + h)) < key;
+        lo = less ? lo + h + 1 : lo;
+        n = less ? n - h - 1 : h;
+    }
+    return lo;
+}
+
 // last index i in [0, n) with off[i] <= x (off non-decreasing, off[0] <= x)
 __device__ __forceinline__ int upper_bound_i64(const int64_t* __restrict__ off, int n, int64_t x)
 {

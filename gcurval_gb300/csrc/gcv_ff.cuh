@@ -82,6 +82,24 @@ __device__ __forceinline__ float scale_down(float x, int s)
 
 __device__ __forceinline__ double ff_to_double(ff a) { return (double)a.hi + (double)a.lo; }
 
+// Local parameters v in [-1, 1] and offsets in them as 64-bit integers in units
+// of 2^-60: panel ends are exact, sums and differences are integer adds, and
+// nothing of it occupies the FP64 pipe.
+constexpr long long FIX_ONE = 1ll << 60;
+// |x| < 2, from the bit pattern (truncated below 2^-60; panel ends are exact)
+__device__ __forceinline__ long long fix_of_double(double x)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+    const int raw = (int)(b >> 52) & 0x7FF, sh = raw - 1023 + 8;
+    const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | (1ull << 52);
+    const long long v = sh >= 0 ? (long long)(m << (sh & 15)) : (sh > -53 ? (long long)(m >> -sh) : 0ll);
+    return (long long)b < 0 ? -v : v;
+}
+__device__ __forceinline__ long long fix_of_float(float x) { return __float2ll_rn(x * 1152921504606846976.0f); }
+
+// reciprocal to an ulp, for factors that carry FP32 rounding anyway
+__device__ __forceinline__ float rcp_approx(float x) { return __fdividef(1.0f, x); }
+
 // double -> float by truncation of the significand, from the bit pattern
 // (integer operations only), for scale factors that need a few digits;
 // outside the normal float range (and for 0, NaN, Inf) the FP64 conversion

@@ -90,11 +90,4 @@ __device__ __forceinline__ ff2 ff2_sqrt(ff2 a)
     return q;
 }
 
-// exact scaling of both lanes by the same power of two
-__device__ __forceinline__ ff2 ff2_scale(ff2 a, float pow2)
-{
-    const float2 s = make_float2(pow2, pow2);
-    return ff2{mul2(a.hi, s), mul2(a.lo, s)};
-}
-
 }  // namespace gcv

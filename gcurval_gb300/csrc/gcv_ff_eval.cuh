@@ -24,9 +24,7 @@ __device__ __forceinline__ ff to_ff(ffc c) { return ff{c.hi, c.lo}; }
 // sin^2(pi y) = S(y) for y <= 1/4 and 1 - S(1/2 - y) above, with S the
 // even series S(u) = sin^2(pi u) = sum_{k >= 1} c_k u^(2k),
 // c_k = (-1)^(k+1) 2^(2k-1) pi^(2k) / (2k)!, for |u| <= 1/4.  Eleven terms:
-// the twelfth is below 1e-19 there, far under float-float rounding.  One
-// series without a branch per node, so that two nodes share one packed
-// evaluation (ff2_sinpi_sq).
+// the twelfth is below 1e-19 there, far under float-float rounding.
 constexpr int SIN2_TERMS = 11;
 __host__ __device__ constexpr double sin2pi_coef(int k)
 {
@@ -42,26 +40,6 @@ __device__ __forceinline__ ff sinpi_sq_fold(ff x, bool& upper)
     if (y.hi > 0.5f) y = ff_add_f(ff_neg(y), 1.0f);  // 1 - |x|
     upper = y.hi > 0.25f;
     return upper ? ff_add_f(ff_neg(y), 0.5f) : y;
-}
-
-// S(u) = sin^2(pi u), two lanes
-__device__ __forceinline__ ff2 ff2_sin2pi_series(ff2 u)
-{
-    const ff2 U = ff2_mul(u, u);
-    ff2 p = splat(to_ff(split_const(sin2pi_coef(SIN2_TERMS))));
-#pragma unroll
-    for (int k = SIN2_TERMS - 1; k >= 1; --k) p = ff2_fma(p, U, splat(to_ff(split_const(sin2pi_coef(k)))));
-    return ff2_mul(p, U);
-}
-
-// sin^2(pi x) for x in [-1, 1], two lanes
-__device__ __forceinline__ ff2 ff2_sinpi_sq(ff2 x)
-{
-    bool up0, up1;
-    const ff u0 = sinpi_sq_fold(lane0(x), up0), u1 = sinpi_sq_fold(lane1(x), up1);
-    const ff2 S = ff2_sin2pi_series(pack(u0, u1));
-    const ff2 C = ff2_add(splat(ff{1.0f, 0.0f}), ff2_neg(S));
-    return pack(up0 ? lane0(C) : lane0(S), up1 ? lane1(C) : lane1(S));
 }
 
 // sin^2(pi x) for x in [-1, 1]
@@ -140,11 +118,12 @@ __host__ __device__ constexpr double cospi_coef(int k)
     for (int i = 1; i <= k; ++i) c *= -PI * PI / ((2 * i - 1) * (2 * i));
     return c;
 }
-// |sin(pi x)| and |cos(pi x)| for x in [-1, 1]
-__device__ __forceinline__ void ff_abs_sincospi(ff x, ff& s, ff& c)
+// sin(pi x) and cos(pi x) for x in [-1, 1]
+__device__ __forceinline__ void ff_sincospi(ff x, ff& s, ff& c)
 {
     ff y = x.hi < 0.0f ? ff_neg(x) : x;
-    if (y.hi > 0.5f) y = ff_add_f(ff_neg(y), 1.0f);
+    const bool left = y.hi > 0.5f;
+    if (left) y = ff_add_f(ff_neg(y), 1.0f);
     const bool swap = y.hi > 0.25f;
     const ff u = swap ? ff_add_f(ff_neg(y), 0.5f) : y;
     const ff2 U = splat(ff_mul(u, u));
@@ -155,6 +134,22 @@ __device__ __forceinline__ void ff_abs_sincospi(ff x, ff& s, ff& c)
     const ff a = ff_mul(lane0(p), u), b = lane1(p);
     s = swap ? b : a;
     c = swap ? a : b;
+    if (x.hi < 0.0f) s = ff_neg(s);
+    if (left) c = ff_neg(c);
+}
+
+// sin(pi d) and cos(pi d) for |d| <= 1/16 (half an ellipse leaf's angle): six
+// terms, the next are below 2^-50 of the leading one
+constexpr int SMALL_TERMS = 6;
+__device__ __forceinline__ void ff_sincospi_small(ff d, ff& s, ff& c)
+{
+    const ff2 U = splat(ff_mul(d, d));
+    ff2 p = pack(to_ff(split_const(sinpi_coef(SMALL_TERMS - 1))), to_ff(split_const(cospi_coef(SMALL_TERMS - 1))));
+#pragma unroll
+    for (int k = SMALL_TERMS - 2; k >= 0; --k)
+        p = ff2_fma(p, U, pack(to_ff(split_const(sinpi_coef(k))), to_ff(split_const(cospi_coef(k)))));
+    s = ff_mul(lane0(p), d);
+    c = lane1(p);
 }
 
 // ------------------------------------------------------------- evaluators
@@ -221,10 +216,7 @@ struct EvalFF {
     // speed() lane by lane, each coefficient splat into both lanes
     __device__ __forceinline__ static ff2 speed2(const ff* r, ff2 v)
     {
-        if constexpr (CODE == 0) {
-            const ff2 w = ff2_add(ff2_scale(v, (float)ELLIPSE_PIECE_SCALE), splat(ff{r[2].hi, 0.0f}));
-            return ff2_sqrt(ff2_fma(splat(r[0]), ff2_sinpi_sq(w), splat(r[1])));
-        }
+        static_assert(CODE != 0, "ellipse sums go by angle addition");
         ff2 s{};
 #pragma unroll
         for (int d = 0; d < D; ++d) {
@@ -235,59 +227,53 @@ struct EvalFF {
         }
         return ff2_sqrt(s);
     }
-    // speed and q = f * df/dv (q only to FP32 accuracy: it shapes the initial guess
-    // and the stopping test, never the result)
-    __device__ __forceinline__ static ff speed_slope(const ff* r, ff v, float& q)
+    // Speed rounded to FP32 and q at a float-float point (B-splines): the
+    // components in float-float (Horner at the full point), their norm in FP32
+    // (the sampler's Newton steps use f to FP32 accuracy only); t[j][d]: the
+    // component's Taylor coefficients there in FP32, for speed_slope_near.
+    __device__ __forceinline__ static float speed_slope_f(const ff* r, ff v, float& q, float* t)
     {
-        if constexpr (CODE == 0) {
-            float sn, cs;
-            sincospif(fmaf(v.hi, (float)ELLIPSE_PIECE_SCALE, r[2].hi), &sn, &cs);
-            q = (float)(PI * ELLIPSE_PIECE_SCALE) * r[0].hi * sn * cs;
-            return speed(r, v);
-        } else {
-            ff s{0.0f, 0.0f};
-            float t = 0.0f;
+        float s = 0.0f, u = 0.0f;
 #pragma unroll
-            for (int d = 0; d < D; ++d) {
-                ff acc = r[(P - 1) * D + d];
-                float dacc = 0.0f;
+        for (int d = 0; d < D; ++d) {
+            ff acc = r[(P - 1) * D + d];
+            float c[P];  // c[j], j >= 1: p^(j)(v) / j! by the nested Horner sums
 #pragma unroll
-                for (int k = P - 2; k >= 0; --k) {
-                    dacc = fmaf(dacc, v.hi, acc.hi);
-                    acc = ff_fma(acc, v, r[k * D + d]);
-                }
-                s = d == 0 ? ff_mul(acc, acc) : ff_fma(acc, acc, s);
-                t = fmaf(acc.hi, dacc, t);
+            for (int j = 1; j < P; ++j) c[j] = 0.0f;
+#pragma unroll
+            for (int k = P - 2; k >= 0; --k) {
+#pragma unroll
+                for (int j = P - 1; j >= 2; --j)
+                    if (j <= P - 1 - k) c[j] = fmaf(c[j], v.hi, c[j - 1]);
+                c[1] = fmaf(c[1], v.hi, acc.hi);
+                acc = ff_fma(acc, v, r[k * D + d]);
             }
-            q = t;
-            return ff_sqrt(s);
+            c[0] = acc.hi + acc.lo;
+            s = fmaf(c[0], c[0], s);
+            if constexpr (P > 1) u = fmaf(c[0], c[1], u);
+#pragma unroll
+            for (int j = 0; j < P; ++j) t[j * D + d] = c[j];
         }
+        q = u;
+        return sqrtf(s);
     }
-    // speed rounded to FP32 and q at a float-float point: the components in
-    // float-float (Horner at the full point), their norm in FP32 (the
-    // sampler's Newton steps use f to FP32 accuracy only)
-    __device__ __forceinline__ static float speed_slope_f(const ff* r, ff v, float& q)
+    // speed and q at the distance x from the point of t
+    __device__ __forceinline__ static float speed_slope_near(const float* t, float x, float& q)
     {
-        if constexpr (CODE == 0) {
-            return speed_slope(r, v, q).hi;
-        } else {
-            float s = 0.0f, t = 0.0f;
+        float s = 0.0f, u = 0.0f;
 #pragma unroll
-            for (int d = 0; d < D; ++d) {
-                ff acc = r[(P - 1) * D + d];
-                float dacc = 0.0f;
+        for (int d = 0; d < D; ++d) {
+            float acc = t[(P - 1) * D + d], dacc = 0.0f;
 #pragma unroll
-                for (int k = P - 2; k >= 0; --k) {
-                    dacc = fmaf(dacc, v.hi, acc.hi);
-                    acc = ff_fma(acc, v, r[k * D + d]);
-                }
-                const float a = acc.hi + acc.lo;
-                s = fmaf(a, a, s);
-                t = fmaf(a, dacc, t);
+            for (int k = P - 2; k >= 0; --k) {
+                dacc = fmaf(dacc, x, acc);
+                acc = fmaf(acc, x, t[k * D + d]);
             }
-            q = t;
-            return sqrtf(s);
+            s = fmaf(acc, acc, s);
+            u = fmaf(acc, dacc, u);
         }
+        q = u;
+        return sqrtf(s);
     }
     // speed and q in plain FP32 from the coefficients' leading parts: for the
     // leaf table's f and q, which only shape the sampler's initial guess
@@ -408,39 +394,10 @@ __device__ void bspline_setup_ff(const double* __restrict__ kv, const double* __
 // in v (2 (P - 1) float-float FMAs per dimension) and the two node
 // positions by about half the work.
 
-template <int P, int D>
-__device__ __forceinline__ void ff_node_pair(const ff* b, ff x, ff x2, ff& fm, ff& fp)
-{
-    constexpr int N = P - 1;                       // polynomial degree
-    constexpr int JE = (N % 2 == 0) ? N : N - 1;   // highest even power
-    constexpr int JO = (N % 2 == 1) ? N : N - 1;   // highest odd power (-1: none)
-    ff sm{0.0f, 0.0f}, sp{0.0f, 0.0f};
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-        ff e = b[JE * D + d];
-#pragma unroll
-        for (int j = JE - 2; j >= 0; j -= 2) e = ff_fma(e, x2, b[j * D + d]);
-        ff lo_ = e, hi_ = e;
-        if constexpr (JO >= 1) {
-            ff o = b[JO * D + d];
-#pragma unroll
-            for (int j = JO - 2; j >= 1; j -= 2) o = ff_fma(o, x2, b[j * D + d]);
-            o = ff_mul(o, x);
-            lo_ = ff_add(e, ff_neg(o));
-            hi_ = ff_add(e, o);
-        }
-        sm = d == 0 ? ff_mul(lo_, lo_) : ff_fma(lo_, lo_, sm);
-        sp = d == 0 ? ff_mul(hi_, hi_) : ff_fma(hi_, hi_, sp);
-    }
-    fm = ff_sqrt(sm);
-    fp = ff_sqrt(sp);
-}
-
-// ff_node_pair for two node pairs at once, in the lanes of packed FP32 pairs
-// (FFMA2 / FADD2 / FMUL2): x and x2 hold the two pairs' offsets, the
-// coefficients b are shared (each is splat into both lanes where it is
-// used).  Half the float-float instructions of two ff_node_pair calls, the
-// same roundings lane by lane.
+// The speeds of two node pairs at once, in the lanes of packed FP32 pairs
+// (FFMA2 / FADD2 / FMUL2): x and x2 hold the two pairs' offsets and their
+// squares, the coefficients b are shared (each is splat into both lanes where
+// it is used).
 template <int P, int D>
 __device__ __forceinline__ void ff_node_pair2(const ff* b, ff2 x, ff2 x2, ff2& fm, ff2& fp)
 {
@@ -494,8 +451,7 @@ static __constant__ GkStep2 c_gk_step2[4] = {GCV_GK_STEP2(0), GCV_GK_STEP2(1), G
 #undef GCV_GK_STEP2
 
 // An ellipse piece's panel by angle addition (AngleTable), two node pairs per
-// packed step as in panel_k15_ff_pairs.  Signs of the midpoint's sine and
-// cosine only swap a pair's two nodes, so magnitudes do.  r: A, B, w0.
+// packed step as in panel_k15_ff_pairs.  r: A, B, w0.
 __device__ __forceinline__ void panel_k15_ff_ellipse(const ff* r, unsigned long long k, int depth, ff& K, ff& G)
 {
     const float hw = __int_as_float((127 - depth) << 23);  // 2^-depth, exact
@@ -503,7 +459,7 @@ __device__ __forceinline__ void panel_k15_ff_ellipse(const ff* r, unsigned long 
     const float sh = __int_as_float((127 + 25 - depth) << 23), sl = 2.0f * hw;
     const ff mid = ff_add_f(ff_add_f(two_sum(-1.0f, kh * sh), kl * sl), hw);
     ff sm, cm;
-    ff_abs_sincospi(ff_add_f(ff_scale(mid, (float)ELLIPSE_PIECE_SCALE), r[2].hi), sm, cm);
+    ff_sincospi(ff_add_f(ff_scale(mid, (float)ELLIPSE_PIECE_SCALE), r[2].hi), sm, cm);
     const ff2 s2 = splat(sm), c2 = splat(cm), A = splat(r[0]), B = splat(r[1]);
     const float4* tab = reinterpret_cast<const float4*>(c_angle.ff[depth]);
     ff2 kk2{}, gg2{};
@@ -615,38 +571,6 @@ __device__ __forceinline__ float speed_slope32_of(int code, const ff* r, float v
             GCV_FOR_EACH_CODE(GCV_CASE)
 #undef GCV_CASE
         default: q = 0.0f; return 0.0f;
-        }
-    }
-}
-
-template <int CODE>
-__device__ __forceinline__ ff speed_ff_of(int code, const ff* r, ff v)
-{
-    if constexpr (CODE >= 0) {
-        return EvalFF<CODE>::speed(r, v);
-    } else {
-        switch (code) {
-#define GCV_CASE(C)                                                                                \
-    case C: return EvalFF<C>::speed(r, v);
-            GCV_FOR_EACH_CODE(GCV_CASE)
-#undef GCV_CASE
-        default: return ff{0.0f, 0.0f};
-        }
-    }
-}
-
-template <int CODE>
-__device__ __forceinline__ ff speed_slope_ff_of(int code, const ff* r, ff v, float& q)
-{
-    if constexpr (CODE >= 0) {
-        return EvalFF<CODE>::speed_slope(r, v, q);
-    } else {
-        switch (code) {
-#define GCV_CASE(C)                                                                                \
-    case C: return EvalFF<C>::speed_slope(r, v, q);
-            GCV_FOR_EACH_CODE(GCV_CASE)
-#undef GCV_CASE
-        default: q = 0.0f; return ff{0.0f, 0.0f};
         }
     }
 }

@@ -1,17 +1,20 @@
-// Mixed-precision path (GCV_MIXED), and the sampling of FP64 tables: the integrand and the panel sums run on
-// the FP32 pipes in float-float arithmetic (gcv_ff.cuh, ~48-bit significand);
-// FP64 is kept for the three steps whose stability needs it:
+// Mixed-precision path (GCV_MIXED), and the sampling of FP64 tables: the
+// integrand and the panel sums run on the FP32 pipes in float-float arithmetic
+// (gcv_ff.cuh, ~48-bit significand);
+// FP64 is kept for the steps whose stability needs it:
 //   * the compensated prefix sum of interval lengths (k_scan, shared with the
 //     FP64 path),
 //   * the panel error test when the FP32 test lands near the tolerance,
-//   * the final Newton update of every sample's parameter.
+//   * a sample's target, its place among the intervals and leaves, and its
+//     parameter (the local one, final Newton update included, in 64-bit fixed
+//     point).
 // Plain FP32 integrands (rounding ~3e-8 per evaluation, plus the systematic
 // rounding of each interval's polynomial coefficients) cannot hold a 1e-8
 // relative length on curves of one or a few knot intervals; float-float can,
 // at a fraction of the FP64 cost on GB300 (FP32:FP64 throughput ~75:1).
 //
-// Ellipse integrands (sin^2(pi v)) are evaluated with an own float-float
-// series for sin^2(pi u), |u| <= 1/4, after folding (gcv_ff_eval.cuh).
+// Ellipse integrands are evaluated by angle addition from one float-float sine
+// and cosine per panel or leaf side (gcv_ff_eval.cuh).
 #pragma once
 
 #include <type_traits>
@@ -28,7 +31,7 @@ namespace gcv {
 // Second-order steps and the stopping test of leaf_newton (gcv_kernels.cuh):
 // d = 2 F / (f0 + f1) with f1 the speed at the Newton point, stop when
 // dn^2 (|f'(w - dn) - f'(w)| / 3 + |f'|^2 |dn| / (4 f)) <= eps_s.
-// Returns the final offset, whose last update is done in FP64.
+// Returns the final offset in units of 2^-60.
 // 8-point Gauss nodes (-x0..-x3, x0..x3) then weights w0..w3, float-float
 #define GCV_FFC(x) {split_const(x).hi, split_const(x).lo}
 static __constant__ float2 c_gl8_ff[12] = {
@@ -39,15 +42,13 @@ static __constant__ float2 c_gl8_ff[12] = {
 
 // Whether the sampler of curve code C takes its Gauss sums by node pairs
 // (gl8_pairs) rather than by evaluating each node: the B-spline codes of
-// degree x dimension below 8.  The larger codes hold more coefficients than
-// their register cap leaves room for beside the pairs' temporaries (100-236
-// bytes of spills at 80-88 registers, and fewer resident warps at 96-104);
-// sampling of the uneven 1M batch took 153.4 ms node by node, 149.2 with
-// pairs for the small codes, 153.1 and 154.6 with pairs for every code at
-// the two register budgets.
+// degree x dimension below 10.  The larger codes hold more coefficients than
+// their register cap leaves room for beside the pairs' temporaries: sampling of
+// 50,000 spatial cubics and quintics took 11.0 ms with pairs below 8, 10.8
+// below 10, 10.9 for every code (with the pairs' loop rolled).
 __host__ __device__ constexpr bool sample_node_pairs(int code)
 {
-    return code > 0 && code_degree(code) * code_dim(code) < 8;
+    return code > 0 && code_degree(code) * code_dim(code) < 10;
 }
 
 // The 8-point Gauss sum over [m - h, m + h] of a B-spline code by symmetric
@@ -80,17 +81,52 @@ __device__ __forceinline__ ff gl8_pairs(ff* b, ff m, ff h)
     return ff_add(lane0(I2), lane1(I2));
 }
 
+// The 8-point Gauss sum over [m - h, m + h] of an ellipse piece by symmetric
+// node pairs: with sm, cm the sine and cosine at m, a pair's are sm cos(d) -+
+// cm sin(d) for its small angle d, whose series needs six terms instead of the
+// eleven of each node's own.
+struct EllipseMid {
+    ff sm, cm;
+};
+__device__ __forceinline__ ff gl8_ellipse(const ff* r, const EllipseMid& e, ff h)
+{
+    const ff2 A = splat(r[0]), B = splat(r[1]);
+    const ff h8 = ff_scale(h, (float)ELLIPSE_PIECE_SCALE);
+    ff I{0.0f, 0.0f};
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+        ff sd, cd;
+        ff_sincospi_small(ff_mul(h8, ff{c_gl8_ff[4 + k].x, c_gl8_ff[4 + k].y}), sd, cd);
+        const ff q = ff_mul(e.cm, sd);
+        const ff2 s = ff2_add(splat(ff_mul(e.sm, cd)), pack(ff_neg(q), q));
+        const ff2 f = ff2_sqrt(ff2_fma(A, ff2_mul(s, s), B));
+        I = ff_fma(ff{c_gl8_ff[8 + k].x, c_gl8_ff[8 + k].y}, ff_add(lane0(f), lane1(f)), I);
+    }
+    return I;
+}
+// speed to FP32 accuracy and q = f f' at the offset x from the midpoint (the
+// square of the speed in float-float: on a thin ellipse's tips it cancels)
+__device__ __forceinline__ float speed_slope_ellipse(const ff* r, const EllipseMid& e, ff x, float& q)
+{
+    ff sd, cd;
+    ff_sincospi_small(ff_scale(x, (float)ELLIPSE_PIECE_SCALE), sd, cd);
+    const ff s = ff_fma(e.cm, sd, ff_mul(e.sm, cd));
+    const float c = fmaf(e.cm.hi, cd.hi, -e.sm.hi * sd.hi);
+    q = (float)(PI * ELLIPSE_PIECE_SCALE) * r[0].hi * s.hi * c;
+    return sqrtf(ff_fma(r[0], ff_mul(s, s), r[1]).hi);
+}
+
 // TAB: the coefficient table's element: float2 (float-float, mixed tables) or
 // double (FP64 tables; lengths then come scaled by 2^-sexp, see k_sample_ff).
 template <int C, typename TAB>
-__device__ __forceinline__ double ff_leaf_newton(const TAB* __restrict__ seg, int sexp, ff vaf, float dv, ff rl, ff dS,
+__device__ __forceinline__ long long ff_leaf_newton(const TAB* __restrict__ seg, int sexp, ff vaf, float dv, ff rl, ff dS,
                                                  float dvg, float eps_s, unsigned long long& newton)
 {
     constexpr bool FROM64 = std::is_same<TAB, double>::value;
     constexpr bool PAIRS = sample_node_pairs(C);
     float blo = 0.0f, bhi = dv;
     ff w{dvg, 0.0f};
-    float last = 0.0f;  // the converged Newton step, applied in FP64 at the end
+    float last = 0.0f;  // the converged Newton step
     for (int it = 0; it < NEWTON_MAXIT; ++it) {
         ++newton;
         ff r[MAX_COEF];
@@ -106,7 +142,11 @@ __device__ __forceinline__ double ff_leaf_newton(const TAB* __restrict__ seg, in
         const ff h2 = ff_scale(ff_add(a1, ff_neg(a0)), 0.5f);
         const ff m2 = ff_add(ff_add(vaf, a0), h2);
         ff I{0.0f, 0.0f};
-        if constexpr (PAIRS) {
+        EllipseMid em;
+        if constexpr (C == 0) {
+            ff_sincospi(ff_add_f(ff_scale(m2, (float)ELLIPSE_PIECE_SCALE), r[2].hi), em.sm, em.cm);
+            I = gl8_ellipse(r, em, h2);
+        } else if constexpr (PAIRS) {
             I = gl8_pairs<C>(r, m2, h2);  // r now holds the coefficients about m2
         } else {
             // nodes -x_k and +x_k in packed lanes
@@ -126,14 +166,16 @@ __device__ __forceinline__ double ff_leaf_newton(const TAB* __restrict__ seg, in
             blo = w.hi;
         else
             bhi = w.hi;
-        // speed at w: after the node-pair sum from the coefficients about m2,
-        // at the end +-h2 of the summed side that is w
-        float q0, f0;
-        if constexpr (PAIRS)
-            f0 = EvalFF<C>::speed_slope_f(r, from_left ? h2 : ff_neg(h2), q0);
+        // speed at w: after the node-pair sums from the midpoint m2, at the end
+        // +-h2 of the summed side that is w
+        float q0, f0, near_w[MAX_COEF];
+        if constexpr (C == 0)
+            f0 = speed_slope_ellipse(r, em, from_left ? h2 : ff_neg(h2), q0);
+        else if constexpr (PAIRS)
+            f0 = EvalFF<C>::speed_slope_f(r, from_left ? h2 : ff_neg(h2), q0, near_w);
         else
-            f0 = EvalFF<C>::speed_slope_f(r, ff_add(vaf, w), q0);
-        const float dn = Fh / f0;
+            f0 = EvalFF<C>::speed_slope_f(r, ff_add(vaf, w), q0, near_w);
+        const float r0 = rcp_approx(f0), dn = Fh * r0;
         float step = dn;
         // the second-order step only from a Newton point inside the closed
         // bracket (a step below one FP32 ulp of w leaves w.hi - dn == w.hi,
@@ -141,23 +183,23 @@ __device__ __forceinline__ double ff_leaf_newton(const TAB* __restrict__ seg, in
         // f1 from the polynomial extrapolated past the leaf
         const float wn = w.hi - dn;
         if (wn >= blo && wn <= bhi) {
-            float q1;
-            // after the node-pair sum from the coefficients about m2, at the
-            // offset (w - dn) - (a0 + h2) from it; else at va + w - dn
-            float f1;
-            if constexpr (PAIRS)
-                f1 = EvalFF<C>::speed_slope_f(r, ff_add(ff_add_f(w, -dn), ff_neg(ff_add(a0, h2))), q1);
+            // for the ellipse at the offset (w - dn) - (a0 + h2) from m2; for
+            // B-splines by the FP32 Taylor expansion at w (full evaluations
+            // of f1 were 7-9 % of the sampler's instructions)
+            float q1, f1;
+            if constexpr (C == 0)
+                f1 = speed_slope_ellipse(r, em, ff_add(ff_add_f(w, -dn), ff_neg(ff_add(a0, h2))), q1);
             else
-                f1 = EvalFF<C>::speed_slope_f(r, ff_add(vaf, ff_add_f(w, -dn)), q1);
-            const float d = 2.0f * Fh / (f0 + f1);
-            const float s0 = q0 / f0, s1 = q1 / f1;  // f'(w), f'(w - dn)
-            float res = dn * dn * (fabsf(s1 - s0) * (1.0f / 3.0f) + s1 * s1 * fabsf(dn) / (4.0f * f1));
+                f1 = EvalFF<C>::speed_slope_near(near_w, -dn, q1);
+            const float d = 2.0f * Fh * rcp_approx(f0 + f1);
+            const float r1 = rcp_approx(f1), s0 = q0 * r0, s1 = q1 * r1;  // f'(w), f'(w - dn)
+            float res = dn * dn * (fabsf(s1 - s0) * (1.0f / 3.0f) + s1 * s1 * fabsf(dn) * 0.25f * r1);
             // at FP64 tolerances the FP32 rounding of the step itself counts:
             // f0, f1 and the quotient are good to a few 2^-24 of F
             if constexpr (FROM64) res = fmaf(5e-7f, fabsf(Fh), res);
             const float wd = w.hi - d;
             if (res <= eps_s && wd >= 0.0f && wd <= dv) {
-                last = d;  // converged: the step is applied in FP64
+                last = d;  // converged with this step
                 break;
             }
             step = d;
@@ -168,22 +210,25 @@ __device__ __forceinline__ double ff_leaf_newton(const TAB* __restrict__ seg, in
         else
             w = ff{0.5f * (blo + bhi), 0.0f};  // safeguard (also NaN)
     }
-    // the final update in FP64
-    return ((double)w.hi + (double)w.lo) - (double)last;
+    // the final update, exact in fixed point
+    return fix_of_float(w.hi) + fix_of_float(w.lo) - fix_of_float(last);
 }
 
 // Mixed-precision sampling: table lookups and the target in FP64, the
 // quintic-Hermite guess in FP32, Newton on the leaf in float-float
 // (G8 partial integral on the shorter side, local to the leaf), and the
-// final update of v in FP64.
+// final update of v exactly, in 64-bit fixed point.  Samples per lane stay 32
+// apart: neighbours in neighbouring lanes share table lines and need the same
+// number of Newton steps.  (Consecutive samples per lane, searched for from the
+// last one's interval: 14.5 ms against 11.9 on 50,000 spatial curves; lanes that
+// take their next sample while others iterate: 14.9.)
 // Registers per thread are capped (blocks of up to SAMPLE_THREADS_MAX threads
-// still fit): left to itself the compiler gave the degree-4/5 codes 95-117
-// registers, and the occupancy lost cost more than a cap costs.  80 (6
-// blocks of 128 threads per SM), 88 for degree-5 3D: with the packed Gauss
-// sums several codes spill 12-88 bytes there, yet sampling of the uneven 1M
-// batch took 139.9 ms, against 143.7 ms with a spill-free 96 (5 blocks).
-__host__ __device__ constexpr int sample_ff_regs(int code) { return code == bs_code(5, 3) ? 88 : 80; }
-static_assert(88 * SAMPLE_THREADS_MAX <= 65536, "a block of SAMPLE_THREADS_MAX must fit one SM");
+// still fit) at 72, 7 blocks of 128 threads per SM, with up to 60 bytes of
+// spills: the kernel waits on fixed latencies and table loads more than on any
+// pipe.  Sampling of the uneven batch of 100,000 curves took 14.0 ms at 96
+// registers, 13.3 at 80 - 88, 12.8 at 72 and at 64 (the other parts as then).
+constexpr int SAMPLE_FF_REGS = 72;
+static_assert(SAMPLE_FF_REGS * SAMPLE_THREADS_MAX <= 65536, "a block of SAMPLE_THREADS_MAX must fit one SM");
 //
 // TAB = double runs the same kernel on an FP64 table (GCV_PLAIN_FP64 at
 // tolerances down to PLAIN_SPLIT_RTOL).  What it computes in float-float is
@@ -196,12 +241,12 @@ static_assert(88 * SAMPLE_THREADS_MAX <= 65536, "a block of SAMPLE_THREADS_MAX m
 // 2^-sexp, the binary exponent of its mean speed, so that curves of any
 // double magnitude fit FP32's exponent range.  The FP64 kernel was bound by
 // the FP64 pipe (91 % busy, one warp instruction per 64 issue slots); this one
-// by issue.  4,096 ellipses x 1,000 samples: 4.15 -> 0.64 ms; 10,000 planar
-// cubics x 1,024: 8.51 -> 0.96 ms.  Position errors at rtol 1e-10 .. 1e-12 on
+// by issue.  4,096 ellipses x 1,000 samples: 4.15 -> 0.48 ms; 10,000 planar
+// cubics x 1,024: 8.51 -> 0.84 ms.  Position errors at rtol 1e-10 .. 1e-12 on
 // ellipses, cubics and an uneven batch, rms and worst, are at or below the FP64
 // kernel's: the extra term of its stopping test makes it iterate further.
 template <int CODE, typename TAB>
-__global__ void __maxnreg__(sample_ff_regs(CODE)) k_sample_ff(SampleParams P, const TAB* __restrict__ coef)
+__global__ void __maxnreg__(SAMPLE_FF_REGS) k_sample_ff(SampleParams P, const TAB* __restrict__ coef)
 {
     constexpr bool FROM64 = std::is_same<TAB, double>::value;
     const Batch& b = P.b;
@@ -225,13 +270,12 @@ __global__ void __maxnreg__(sample_ff_regs(CODE)) k_sample_ff(SampleParams P, co
     for (int64_t ii = run + lane; ii < run + run_len && ii < i1; ii += 32) {
         int64_t i;
         const int c = sample_curve_hint(P, ii, i, hint);
-        const int code = CODE >= 0 ? CODE : curve_code(b, c);
-        const int64_t s0 = b.seg_off[c], s1 = b.seg_off[c + 1];
-        int64_t s;
-        double v;
+        const int s0 = (int)b.seg_off[c], s1 = (int)b.seg_off[c + 1];
+        int s;
+        long long v;  // local parameter, fixed point
         if (s1 == s0) {
             s = -1;
-            v = -1.0;
+            v = -FIX_ONE;
         } else {
             const double L = t.curve_len[c];
             const double pos = P.pos[i];
@@ -242,18 +286,18 @@ __global__ void __maxnreg__(sample_ff_regs(CODE)) k_sample_ff(SampleParams P, co
             // (FP64 tables: a NaN target is the curve's start, as !(target > 0) in k_sample)
             if (tb <= 0 || (FROM64 && tb > 0x7FF0000000000000ll)) {
                 s = s0;
-                v = -1.0;
+                v = -FIX_ONE;
             } else if (tb >= lb) {
                 s = s1 - 1;
-                v = 1.0;
+                v = FIX_ONE;
             } else {
-                s = lower_bound_key(t.seg_cum, s0, s1, dkey(target));
+                s = s0 + lower_bound_key32(t.seg_cum + s0, s1 - s0, dkey(target));
                 if (s == s1) s = s1 - 1;
                 const double prev = s > s0 ? t.seg_cum[s - 1] : 0.0;
                 const double rr = target - prev;
                 const int64_t lo = t.leaf_off[s];
                 const int cnt = t.leaf_cnt[s];
-                int64_t j = lower_bound_key(t.leaf_cum, lo, lo + cnt, dkey(rr)) - lo;
+                int j = lower_bound_key32(t.leaf_cum + lo, cnt, dkey(rr));
                 if (j >= cnt) j = cnt - 1;
                 double base = 0.0, va = -1.0;
                 float fa, qa;
@@ -262,20 +306,21 @@ __global__ void __maxnreg__(sample_ff_regs(CODE)) k_sample_ff(SampleParams P, co
                     va = t.leaf_v[lo + j - 1];
                     fa = t.leaf_f[lo + j - 1];
                     qa = t.leaf_q[lo + j - 1];
-                } else {  // the interval's start: its FP64 end values, converted once
-                    fa = (float)t.seg_f0[s];
-                    qa = (float)t.seg_q0[s];
+                } else {  // the interval's start: its end values, by their bits
+                    fa = f32_of_f64_trunc(t.seg_f0[s]);
+                    qa = f32_of_f64_trunc(t.seg_q0[s]);
                 }
                 const double vb = t.leaf_v[lo + j];
                 const double cb = t.leaf_cum[lo + j];
                 float fb = t.leaf_f[lo + j];
                 float qb = t.leaf_q[lo + j];
                 const double rd = rr - base, dSd = cb - base;  // target inside the leaf, leaf length
-                const double dvd = vb - va;                     // leaf width (exact dyadic)
+                const long long vfix = fix_of_double(va), dfix = fix_of_double(vb) - vfix;
+                const int dexp = 3 - __clzll(dfix);             // leaf width 2^dexp
                 int sexp = 0;
                 ff rl, dS;
                 if constexpr (FROM64) {
-                    sexp = exponent_of(dSd) - exponent_of(dvd);
+                    sexp = exponent_of(dSd) - dexp;
                     rl = ff_from_double_scaled(rd, sexp);
                     dS = ff_from_double_scaled(dSd, sexp);
                     fa = scale_down(fa, sexp);
@@ -286,13 +331,13 @@ __global__ void __maxnreg__(sample_ff_regs(CODE)) k_sample_ff(SampleParams P, co
                     rl = ff_from_double(rd);
                     dS = ff_from_double(dSd);
                 }
-                const float dv = (float)dvd;
+                const float dv = __int_as_float((dexp + 127) << 23);
                 const ff vaf = ff_from_double(va);
                 // quintic Hermite guess of v(S) on the leaf (FP32)
-                float sig = dS.hi > 0.0f ? rl.hi / dS.hi : 0.0f;
+                float sig = dS.hi > 0.0f ? rl.hi * rcp_approx(dS.hi) : 0.0f;
                 sig = fminf(fmaxf(sig, 0.0f), 1.0f);
                 float dvg = sig * dv;
-                const float fm = dS.hi / dv;
+                const float fm = dS.hi * rcp_approx(dv);
                 if (fa > 0.1f * fm && fb > 0.1f * fm) {
                     const float s2 = sig * sig, s3 = s2 * sig, s4 = s3 * sig, s5 = s4 * sig;
                     const float h5 = 10.0f * s3 - 15.0f * s4 + 6.0f * s5;
@@ -300,34 +345,15 @@ __global__ void __maxnreg__(sample_ff_regs(CODE)) k_sample_ff(SampleParams P, co
                     const float h4 = -4.0f * s3 + 7.0f * s4 - 3.0f * s5;
                     const float h2 = 0.5f * (s2 - 3.0f * s3 + 3.0f * s4 - s5);
                     const float h3 = 0.5f * (s3 - 2.0f * s4 + s5);
-                    const float ia = 1.0f / fa, ib = 1.0f / fb;
+                    const float ia = rcp_approx(fa), ib = rcp_approx(fb);
                     const float ka = -qa * (ia * ia) * (ia * ia), kb = -qb * (ib * ib) * (ib * ib);
                     dvg = h5 * dv + dS.hi * (h1 * ia + h4 * ib) + dS.hi * dS.hi * (h2 * ka + h3 * kb);
                     dvg = fminf(fmaxf(dvg, 0.0f), dv);
                 }
-                const TAB* seg = coef + b.coef_off[c] + (s - s0) * code_stride(code);
+                const TAB* seg = coef + b.coef_off[c] + (int64_t)(s - s0) * code_stride(CODE);
                 const float eps_s = P.eps_frac * (FROM64 ? ff_from_double_scaled(L, sexp).hi : f32_of_f64_trunc(L));
-                double wfinal;
-                if constexpr (CODE >= 0) {
-                    wfinal = ff_leaf_newton<(CODE >= 0 ? CODE : 0)>(
-                        seg, sexp, vaf, dv, rl, dS, dvg, eps_s, newton);
-                } else {
-                    switch (code) {
-#define GCV_CASE(C)                                                                                \
-    case C: wfinal = ff_leaf_newton<C>(seg, sexp, vaf, dv, rl, dS, dvg, eps_s, newton); break;
-                        GCV_FOR_EACH_CODE(GCV_CASE)
-#undef GCV_CASE
-                    default: wfinal = dvg; break;
-                    }
-                }
-                // the offset clamped to [0, dv] on the bit patterns (both
-                // non-negative there; a negative offset or NaN has its sign
-                // bit set or the largest pattern): integer compares, off the
-                // FP64 pipe, as fmin / fmax would clamp it
-                const long long wb = __double_as_longlong(wfinal);
-                if (wb < 0) wfinal = 0.0;
-                else if (wb > __double_as_longlong(dvd)) wfinal = dvd;
-                v = va + wfinal;
+                const long long w = ff_leaf_newton<CODE>(seg, sexp, vaf, dv, rl, dS, dvg, eps_s, newton);
+                v = vfix + (w < 0 ? 0 : w > dfix ? dfix : w);
             }
         }
         if (P.what == 2) {
@@ -335,15 +361,19 @@ __global__ void __maxnreg__(sample_ff_regs(CODE)) k_sample_ff(SampleParams P, co
             if (s < 0) {
                 u = b.kind[c] == 0 ? 0.0 : b.knots[b.knot_off[c] + b.degree[c]];
             } else {
-                const double t0 = t.seg_t0[s], t1 = t.seg_t1[s], hw = 0.5 * (t1 - t0);
-                // v <= 0 on the bit pattern (-0 and negatives have the sign bit)
-                u = __double_as_longlong(v) <= 0 ? fma(v + 1.0, hw, t0) : fma(v - 1.0, hw, t1);
+                // (v + 1) hw + t0 up to v = 0, (v - 1) hw + t1 above: exact at
+                // both ends, the operands chosen so that one side is evaluated
+                const double t0 = t.seg_t0[s], t1 = t.seg_t1[s];
+                const bool low = v <= 0;
+                u = fma(__ll2double_rn(v + (low ? FIX_ONE : -FIX_ONE)), (t1 - t0) * (0.5 / (double)FIX_ONE),
+                        low ? t0 : t1);
             }
             P.out[i] = u;
         } else {
             double p3[3] = {0.0, 0.0, 0.0};
             if (s >= 0) {
-                const TAB* seg = coef + b.coef_off[c] + (s - s0) * code_stride(code);
+                const TAB* seg = coef + b.coef_off[c] + (int64_t)(s - s0) * code_stride(CODE);
+                const double vd = __ll2double_rn(v) * (1.0 / (double)FIX_ONE);
                 double cd[MAX_COEF];
                 const double* pc = cd;
                 if constexpr (FROM64) {
@@ -351,16 +381,14 @@ __global__ void __maxnreg__(sample_ff_regs(CODE)) k_sample_ff(SampleParams P, co
                 } else {
                     // points from the float-float coefficients, evaluated in FP64
                     // (a B-spline stores a[0] and then b[k - 1] = k a[k])
-                    const int n = code_stride(code), dim = code_dim(code);
+                    constexpr int n = code_stride(CODE), dim = code_dim(CODE);
+#pragma unroll
                     for (int k = 0; k < n; ++k) {
                         cd[k] = (double)seg[k].x + (double)seg[k].y;
-                        if (code != 0 && k >= 2 * dim) cd[k] *= 1.0 / (double)(k / dim);
+                        if (CODE != 0 && k >= 2 * dim) cd[k] *= 1.0 / (double)(k / dim);
                     }
                 }
-                if constexpr (CODE >= 0)
-                    Eval<(CODE >= 0 ? CODE : 0)>::point(pc, v, p3);
-                else
-                    point_dyn(code, pc, v, p3);
+                Eval<CODE>::point(pc, vd, p3);
             }
             for (int k = 0; k < P.pdim; ++k) P.out[i * P.pdim + k] = p3[k];
         }
