@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <tuple>
 #include <cmath>
@@ -285,11 +286,8 @@ struct Knobs {
 // The first TUNE_TRIALS table builds (and samplings) of a batch shape not seen
 // before in the process each run one candidate; the fastest shapes, timed by
 // the context's events, are kept for that shape (curve code, precision,
-// learned form, log2 of the interval count).  The length walk is timed code
-// by code (its main pass launches once per curve code), so each code of a
-// batch that mixes codes keeps the persistent-worker count that was fastest
-// for it.  The shapes change scheduling only: every result is the same
-// under each, bit for bit.  (The half-warp-per-interval mapping of the main
+// learned form, log2 of the interval count).  The shapes change scheduling
+// only: every result is the same under each, bit for bit.  (The half-warp-per-interval mapping of the main
 // pass sums each panel's nodes in another order, so it is a user option,
 // gcv_options.mapping, not a shape the tuner may pick.)
 constexpr int TUNE_TRIALS = 3;
@@ -317,6 +315,32 @@ struct TuneKey {
 };
 static std::mutex g_tune_m;
 static std::map<TuneKey, Knobs> g_tuned;
+
+// Helper streams for the launches of a batch that mixes curve codes: one launch
+// per code and phase, independent of each other, forked from the context's
+// stream and joined to it again (gcv_ctx::stream orders everything else).  In a
+// small batch each launch is a few dozen warps and lasts as long as its slowest
+// one; side by side the phase lasts as long as the slowest launch.  Kits are
+// kept in a process-wide pool of at most FORK_KITS for the next context, since
+// creating seven streams costs more than a small batch's table.
+constexpr int FORK_HELPERS = 7;
+constexpr size_t FORK_KITS = 4;
+struct ForkKit {
+    int dev = 0;
+    cudaStream_t helper[FORK_HELPERS] = {};
+    cudaEvent_t fork = nullptr, join[FORK_HELPERS] = {};
+    ~ForkKit()
+    {
+        for (cudaStream_t h : helper)
+            if (h) cudaStreamDestroy(h);
+        for (cudaEvent_t e : join)
+            if (e) cudaEventDestroy(e);
+        if (fork) cudaEventDestroy(fork);
+    }
+};
+static std::mutex g_kit_m;
+// (never destroyed: the CUDA runtime may be gone when static objects are)
+static std::vector<std::unique_ptr<ForkKit>>& g_kits = *new std::vector<std::unique_ptr<ForkKit>>();
 
 constexpr int STREAM_EVENTS = 4;  // host-buffer sampling: events per stage, used round robin
 
@@ -395,11 +419,7 @@ struct gcv_ctx {
     // autotuner progress of this context (-1: tuned, shapes from the table)
     int len_trial = 0, smp_trial = 0;
     double len_ms[TUNE_TRIALS] = {}, smp_ms[TUNE_TRIALS] = {};
-    // per-code main-pass times of the tuning builds (ev_code: start / end of
-    // each code's main-pass launch in the last build)
-    double len_code_ms[TUNE_TRIALS][N_CODE_SLOTS] = {};
-    cudaEvent_t ev_code[N_CODE_SLOTS][2] = {};
-    bool code_timed[N_CODE_SLOTS] = {};
+    std::unique_ptr<ForkKit> kit;
     TuneKey tune_key{-9, -9, -9, -9};
     // chunked host <-> device streaming of samples
     cudaStream_t s_in = nullptr, s_out = nullptr;
@@ -534,9 +554,10 @@ void destroy_ctx(gcv_ctx* c)
     if (c->s_out) cudaStreamDestroy(c->s_out);
     for (auto& e : c->ev)
         if (e) cudaEventDestroy(e);
-    for (auto& pair : c->ev_code)
-        for (auto& e : pair)
-            if (e) cudaEventDestroy(e);
+    if (c->kit) {
+        std::lock_guard<std::mutex> g(g_kit_m);
+        if (g_kits.size() < FORK_KITS) g_kits.push_back(std::move(c->kit));
+    }
     delete c;
 }
 
@@ -613,8 +634,6 @@ gcv_status finish_create(gcv_ctx* c, const uint8_t* kind, const uint8_t* degree,
     CHECK(c->ctr.reserve(C_COUNT));
     CU(cudaMallocHost(&c->h_ctr, C_COUNT * sizeof(unsigned long long)));
     for (auto& e : c->ev) CU(cudaEventCreate(&e));
-    for (auto& pair : c->ev_code)
-        for (auto& e : pair) CU(cudaEventCreate(&e));
     if (c->n_curve > 0) {
         const Batch b = batch_view(c);
         const int blocks = (int)std::min<int64_t>((c->n_curve + 255) / 256, 65535);
@@ -727,6 +746,69 @@ gcv_status to_host(const T* src, size_t n, int where, std::vector<T>& dst)
     return GCV_OK;
 }
 
+// One phase's launches side by side: stream(k) for launch k (the context's own
+// stream among them), join() before what follows.  A phase of one launch stays
+// on the context's stream.
+class Fork {
+public:
+    Fork(gcv_ctx* c, size_t launches) : c_(c), on_(launches > 1) {}
+    ~Fork() { (void)join(); }
+    gcv_status stream(size_t k, cudaStream_t* out)
+    {
+        const int h = on_ ? (int)(k % (FORK_HELPERS + 1)) - 1 : -1;
+        *out = c_->stream;
+        if (h < 0) return GCV_OK;
+        if (!begun_) {
+            CHECK(kit());
+            CU(cudaEventRecord(c_->kit->fork, c_->stream));
+            begun_ = true;
+        }
+        if (!used_[h]) {
+            CU(cudaStreamWaitEvent(c_->kit->helper[h], c_->kit->fork, 0));
+            used_[h] = true;
+        }
+        *out = c_->kit->helper[h];
+        return GCV_OK;
+    }
+    gcv_status join()
+    {
+        gcv_status st = GCV_OK;
+        for (int h = 0; h < FORK_HELPERS; ++h) {
+            if (!used_[h]) continue;
+            used_[h] = false;
+            cudaError_t e = cudaEventRecord(c_->kit->join[h], c_->kit->helper[h]);
+            if (e == cudaSuccess) e = cudaStreamWaitEvent(c_->stream, c_->kit->join[h], 0);
+            if (e != cudaSuccess && st == GCV_OK) st = cuda_fail(e, "joining a helper stream");
+        }
+        return st;
+    }
+
+private:
+    gcv_status kit()
+    {
+        if (c_->kit) return GCV_OK;
+        const int dev = current_device();
+        {
+            std::lock_guard<std::mutex> g(g_kit_m);
+            for (auto it = g_kits.begin(); it != g_kits.end(); ++it)
+                if ((*it)->dev == dev) {
+                    c_->kit = std::move(*it);
+                    g_kits.erase(it);
+                    return GCV_OK;
+                }
+        }
+        std::unique_ptr<ForkKit> k(new ForkKit());
+        k->dev = dev;
+        for (cudaStream_t& h : k->helper) CU(cudaStreamCreateWithFlags(&h, cudaStreamNonBlocking));
+        CU(cudaEventCreateWithFlags(&k->fork, cudaEventDisableTiming));
+        for (cudaEvent_t& e : k->join) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        c_->kit = std::move(k);
+        return GCV_OK;
+    }
+    gcv_ctx* c_;
+    bool on_, begun_ = false, used_[FORK_HELPERS] = {};
+};
+
 // ------------------------------------------------------------ table build
 
 gcv_status ensure_table_buffers(gcv_ctx* c)
@@ -803,7 +885,7 @@ gcv_status read_counters(gcv_ctx* c)
 // pass; the deep passes are specialised for the common uniform batches and
 // dispatch per segment otherwise (their lists mix codes)
 template <int MODE, int PREC>
-gcv_status launch_length_code(gcv_ctx* c, int code, const LengthParams& P)
+gcv_status launch_length_code(gcv_ctx* c, int code, const LengthParams& P, cudaStream_t st)
 {
     const int sms = sm_count();
     cudaError_t e = cudaErrorInvalidValue;
@@ -817,9 +899,9 @@ gcv_status launch_length_code(gcv_ctx* c, int code, const LengthParams& P)
 #define GCV_CASE(C)                                                                                \
     case C:                                                                                        \
         if constexpr (PREC == 1)                                                                   \
-            e = half_warp ? length_launch_hw<C>(P, c->stream, sms, cap) : walk_launch<C, 1>(P, c->stream, sms, cap); \
+            e = half_warp ? length_launch_hw<C>(P, st, sms, cap) : walk_launch<C, 1>(P, st, sms, cap); \
         else                                                                                       \
-            e = walk64 ? walk_launch<C, 2>(P, c->stream, sms, cap) : length_launch<0, C, 0>(P, c->stream, sms, cap); \
+            e = walk64 ? walk_launch<C, 2>(P, st, sms, cap) : length_launch<0, C, 0>(P, st, sms, cap); \
         break;
             GCV_FOR_EACH_CODE(GCV_CASE)
 #undef GCV_CASE
@@ -828,10 +910,10 @@ gcv_status launch_length_code(gcv_ctx* c, int code, const LengthParams& P)
     } else {
         const int cap = c->knobs.deep_cap;
         switch (code) {
-        case CODE_ELLIPSE: e = length_launch<MODE, CODE_ELLIPSE, PREC>(P, c->stream, sms, cap); break;
-        case bs_code(3, 2): e = length_launch<MODE, bs_code(3, 2), PREC>(P, c->stream, sms, cap); break;
-        case bs_code(3, 3): e = length_launch<MODE, bs_code(3, 3), PREC>(P, c->stream, sms, cap); break;
-        default: e = length_launch<MODE, -1, PREC>(P, c->stream, sms, cap); break;
+        case CODE_ELLIPSE: e = length_launch<MODE, CODE_ELLIPSE, PREC>(P, st, sms, cap); break;
+        case bs_code(3, 2): e = length_launch<MODE, bs_code(3, 2), PREC>(P, st, sms, cap); break;
+        case bs_code(3, 3): e = length_launch<MODE, bs_code(3, 3), PREC>(P, st, sms, cap); break;
+        default: e = length_launch<MODE, -1, PREC>(P, st, sms, cap); break;
         }
     }
     if (e != cudaSuccess) return cuda_fail(e, "length kernel launch");
@@ -840,25 +922,17 @@ gcv_status launch_length_code(gcv_ctx* c, int code, const LengthParams& P)
 }
 
 template <int MODE>
-gcv_status launch_length(gcv_ctx* c, int code, const LengthParams& P)
+gcv_status launch_length(gcv_ctx* c, int code, const LengthParams& P, cudaStream_t st)
 {
-    return c->opt.precision == GCV_MIXED ? launch_length_code<MODE, 1>(c, code, P)
-                                         : launch_length_code<MODE, 0>(c, code, P);
+    return c->opt.precision == GCV_MIXED ? launch_length_code<MODE, 1>(c, code, P, st)
+                                         : launch_length_code<MODE, 0>(c, code, P, st);
 }
 
 // Main pass: one launch over all segments of a uniform batch, or one launch
-// per curve code over that code's range of the grouped segment list; each
-// code's launch is bracketed by its pair of timing events (as external event
-// nodes under stream capture), which the autotuner reads.
-gcv_status launch_main_pass(gcv_ctx* c, LengthParams P, bool capture = false)
+// per curve code over that code's range of the grouped segment list, side by
+// side.
+gcv_status launch_main_pass(gcv_ctx* c, LengthParams P)
 {
-    auto mark = [&](int code, int which) -> gcv_status {
-        cudaEvent_t e = c->ev_code[code_slot(code)][which];
-        CU(capture ? cudaEventRecordWithFlags(e, c->stream, cudaEventRecordExternal) : cudaEventRecord(e, c->stream));
-        c->code_timed[code_slot(code)] = true;
-        return GCV_OK;
-    };
-    for (bool& x : c->code_timed) x = false;
     // work items in the order of the coefficient table and the learned
     // start depths (segment order for one code, the grouped list otherwise)
     P.by_item = 1;
@@ -867,11 +941,10 @@ gcv_status launch_main_pass(gcv_ctx* c, LengthParams P, bool capture = false)
         P.n_items = c->n_seg;
         P.work = c->ctr.p + C_WORK;
         P.coef_base = 0;
-        CHECK(mark(c->code, 0));
-        CHECK(launch_length<0>(c, c->code, P));
-        return mark(c->code, 1);
+        return launch_length<0>(c, c->code, P, c->stream);
     }
     const uint32_t* starts = P.starts;
+    Fork fork(c, c->code_ranges.size());
     for (size_t k = 0; k < c->code_ranges.size(); ++k) {
         const CodeRange& r = c->code_ranges[k];
         if (r.end == r.begin) continue;
@@ -880,11 +953,11 @@ gcv_status launch_main_pass(gcv_ctx* c, LengthParams P, bool capture = false)
         P.coef_base = r.coef_base;
         P.starts = starts ? starts + r.begin : nullptr;
         P.work = c->ctr.p + C_WORK_CODE + k;
-        CHECK(mark(r.code, 0));
-        CHECK(launch_length<0>(c, r.code, P));
-        CHECK(mark(r.code, 1));
+        cudaStream_t st;
+        CHECK(fork.stream(k, &st));
+        CHECK(launch_length<0>(c, r.code, P, st));
     }
-    return GCV_OK;
+    return fork.join();
 }
 
 // ---------------------------------------------------------- autotuner
@@ -932,21 +1005,12 @@ int argmin3(const double* v)
     return b;
 }
 
-// the length shapes of finished trials: each code its fastest trial, the
-// deep passes the trial with the fastest length phase as a whole
+// the length shapes of finished trials: the one with the fastest length phase
 void choose_length_knobs(gcv_ctx* c, Knobs& k)
 {
-    const int all = argmin3(c->len_ms);
-    for (int sl = 0; sl < N_CODE_SLOTS; ++sl) {
-        double v[TUNE_TRIALS];
-        bool timed = true;
-        for (int i = 0; i < TUNE_TRIALS; ++i) {
-            v[i] = c->len_code_ms[i][sl];
-            timed = timed && v[i] > 0.0;
-        }
-        k.length_cap[sl] = trial_length_cap(timed ? argmin3(v) : all);
-    }
-    k.deep_cap = trial_length_cap(all);
+    const int best = trial_length_cap(argmin3(c->len_ms));
+    for (int& x : k.length_cap) x = best;
+    k.deep_cap = best;
 }
 
 void tune_finish_if_done(gcv_ctx* c)
@@ -971,13 +1035,6 @@ gcv_status tune_after_table(gcv_ctx* c)
     CU(cudaEventSynchronize(c->ev[2]));
     float ms = 0.f;
     CU(cudaEventElapsedTime(&ms, c->ev[6], c->ev[2]));
-    for (int sl = 0; sl < N_CODE_SLOTS; ++sl) {
-        float mc = 0.f;
-        c->len_code_ms[c->len_trial][sl] = 0.0;
-        if (c->code_timed[sl] && cudaEventElapsedTime(&mc, c->ev_code[sl][0], c->ev_code[sl][1]) == cudaSuccess)
-            c->len_code_ms[c->len_trial][sl] = std::max(mc, 1e-6f);
-    }
-    cudaGetLastError();
     c->len_ms[c->len_trial++] = ms;
     if (c->len_trial == TUNE_TRIALS && c->smp_trial >= 0 && c->smp_trial < TUNE_TRIALS) choose_length_knobs(c, c->knobs);
     tune_finish_if_done(c);
@@ -997,7 +1054,7 @@ gcv_status tune_after_sampling(gcv_ctx* c)
 }
 
 // feat16: the learned form's feature rows in grouped-list order (NULL otherwise)
-gcv_status launch_setup_list(gcv_ctx* c, const CodeRange& r, uint4* feat16)
+gcv_status launch_setup_list(gcv_ctx* c, const CodeRange& r, uint4* feat16, cudaStream_t st)
 {
     const int64_t n = r.end - r.begin;
     if (n <= 0) return GCV_OK;
@@ -1009,7 +1066,7 @@ gcv_status launch_setup_list(gcv_ctx* c, const CodeRange& r, uint4* feat16)
     const float rf = rtol_feature(c->opt.rtol);
     switch (r.code) {
 #define GCV_CASE(C)                                                                                \
-    case C: k_setup_list<C><<<blocks, 256, 0, c->stream>>>(b, t, list, n, f16, rf); break;
+    case C: k_setup_list<C><<<blocks, 256, 0, st>>>(b, t, list, n, f16, rf); break;
         GCV_FOR_EACH_CODE(GCV_CASE)
 #undef GCV_CASE
     default: return fail(GCV_ERR_INVALID, "no set-up kernel for curve code " + std::to_string(r.code));
@@ -1017,6 +1074,42 @@ gcv_status launch_setup_list(gcv_ctx* c, const CodeRange& r, uint4* feat16)
     CU(cudaGetLastError());
     c->stats.n_launches++;
     return GCV_OK;
+}
+
+// set-up of a batch that mixes codes
+gcv_status launch_setup_codes(gcv_ctx* c, uint4* feat16)
+{
+    Fork fork(c, c->code_ranges.size());
+    for (size_t k = 0; k < c->code_ranges.size(); ++k) {
+        cudaStream_t st;
+        CHECK(fork.stream(k, &st));
+        CHECK(launch_setup_list(c, c->code_ranges[k], feat16, st));
+    }
+    return fork.join();
+}
+
+// the network's start depths of every B-spline interval, in the order of the
+// work items (ellipse pieces keep 0)
+gcv_status launch_network(gcv_ctx* c, int max_depth)
+{
+    auto run = [&](int64_t begin, int64_t end, cudaStream_t st) -> gcv_status {
+        cudaError_t e = mlp_starts_launch_bf16(c->feat16.p + 2 * begin, nullptr, end - begin, c->mlp_w, max_depth,
+                                               c->starts.p + begin, st);
+        if (e != cudaSuccess) return cuda_fail(e, "network inference");
+        c->stats.n_launches++;
+        return GCV_OK;
+    };
+    if (c->code > 0) return run(0, c->n_seg, c->stream);
+    if (c->code == CODE_ELLIPSE) return GCV_OK;
+    Fork fork(c, c->code_ranges.size());
+    for (size_t k = 0; k < c->code_ranges.size(); ++k) {
+        const CodeRange& r = c->code_ranges[k];
+        if (r.code == CODE_ELLIPSE) continue;
+        cudaStream_t st;
+        CHECK(fork.stream(k, &st));
+        CHECK(run(r.begin, r.end, st));
+    }
+    return fork.join();
 }
 
 gcv_status build_table(gcv_ctx* c)
@@ -1038,7 +1131,7 @@ gcv_status build_table(gcv_ctx* c)
         CU(cudaGetLastError());
         c->stats.n_launches++;
     } else if (c->n_seg > 0) {
-        for (const CodeRange& r : c->code_ranges) CHECK(launch_setup_list(c, r, feat16));
+        CHECK(launch_setup_codes(c, feat16));
     }
     CU(cudaEventRecord(c->ev[1], c->stream));
     if (learned) {
@@ -1046,20 +1139,7 @@ gcv_status build_table(gcv_ctx* c)
         CHECK(c->starts.reserve((size_t)c->n_seg));
         CU(cudaMemsetAsync(c->starts.p, 0, (size_t)c->n_seg * sizeof(uint32_t), c->stream));
         const int md = mixed ? std::min(c->opt.max_depth, FF_MAX_DEPTH) : c->opt.max_depth;
-        // start depths in the order of the work items (the grouped list)
-        auto run = [&](const uint4* f16, uint32_t* starts, int64_t n) -> gcv_status {
-            cudaError_t e = mlp_starts_launch_bf16(f16, nullptr, n, c->mlp_w, md, starts, c->stream);
-            if (e != cudaSuccess) return cuda_fail(e, "network inference");
-            c->stats.n_launches++;
-            return GCV_OK;
-        };
-        if (c->code > 0) {
-            CHECK(run(c->feat16.p, c->starts.p, c->n_seg));
-        } else if (c->code < 0) {
-            for (const CodeRange& r : c->code_ranges)
-                if (r.code != CODE_ELLIPSE)
-                    CHECK(run(c->feat16.p + 2 * r.begin, c->starts.p + r.begin, r.end - r.begin));
-        }
+        CHECK(launch_network(c, md));
     }
     CU(cudaEventRecord(c->ev[6], c->stream));
     for (int attempt = 0;; ++attempt) {
@@ -1114,7 +1194,7 @@ gcv_status build_table(gcv_ctx* c)
             Q.collect = 0;
             Q.starts = nullptr;
             Q.work = c->ctr.p + C_WORK;
-            CHECK(launch_length<1>(c, c->code, Q));
+            CHECK(launch_length<1>(c, c->code, Q, c->stream));
             const int rb = (int)std::min<int64_t>((n_deep + 255) / 256, (int64_t)sm_count() * 8);
             k_deep_total<<<rb, 256, 0, c->stream>>>(c->deep_list.p, n_deep, c->leaf_cnt.p, c->ctr.p + C_DEEP_LEAVES);
             CU(cudaGetLastError());
@@ -1125,7 +1205,7 @@ gcv_status build_table(gcv_ctx* c)
             CU(cudaMemsetAsync(c->ctr.p + C_WORK, 0, sizeof(unsigned long long), c->stream));
             Q.t = table_view(c);
             Q.collect = P.collect;
-            CHECK(launch_length<2>(c, c->code, Q));
+            CHECK(launch_length<2>(c, c->code, Q, c->stream));
             CHECK(read_counters(c));
             if (c->h_ctr[C_ERR] & ERR_POOL) return fail(GCV_ERR_OVERFLOW, "leaf pool overflow in the deep pass");
             top = (int64_t)c->h_ctr[C_LEAF_TOP];
@@ -1165,7 +1245,7 @@ gcv_status build_table(gcv_ctx* c)
 
 // ---------------------------------------------------------------- sampling
 
-gcv_status launch_sampler(gcv_ctx* c, int code, const SampleParams& P, int64_t n)
+gcv_status launch_sampler(gcv_ctx* c, int code, const SampleParams& P, int64_t n, cudaStream_t st)
 {
     const int th = c->knobs.sample_threads;
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n + th - 1) / th,
@@ -1175,7 +1255,7 @@ gcv_status launch_sampler(gcv_ctx* c, int code, const SampleParams& P, int64_t n
     cudaError_t e = cudaErrorInvalidValue;
     switch (code) {
 #define GCV_CASE(C)                                                                                \
-    case C: e = mixed ? sample_launch<C, 1>(P, cf, c->stream, grid, th) : sample_launch<C, 0>(P, cf, c->stream, grid, th); break;
+    case C: e = mixed ? sample_launch<C, 1>(P, cf, st, grid, th) : sample_launch<C, 0>(P, cf, st, grid, th); break;
         GCV_FOR_EACH_CODE(GCV_CASE)
 #undef GCV_CASE
     default: return fail(GCV_ERR_INVALID, "no sampling kernel for curve code " + std::to_string(code));
@@ -1194,12 +1274,14 @@ gcv_status launch_sample_chunk(gcv_ctx* c, SampleParams P, int64_t c_lo, int64_t
         P.curve_list = nullptr;
         P.s_begin = c->h_sample_off[(size_t)c_lo];
         P.s_end = c->h_sample_off[(size_t)c_hi];
-        if (P.s_end > P.s_begin) CHECK(launch_sampler(c, c->code, P, P.s_end - P.s_begin));
+        if (P.s_end > P.s_begin) CHECK(launch_sampler(c, c->code, P, P.s_end - P.s_begin, c->stream));
         return GCV_OK;
     }
     P.curve_list = c->curve_list.p;
     P.list_off = c->list_sample_off.p;
     const int* L = c->h_curve_list.data();
+    Fork fork(c, c->curve_ranges.size());
+    size_t k = 0;
     for (const CodeRange& r : c->curve_ranges) {
         const int64_t jb = std::lower_bound(L + r.begin, L + r.end, (int)c_lo) - L;
         const int64_t je = std::lower_bound(L + r.begin, L + r.end, (int)c_hi) - L;
@@ -1207,9 +1289,11 @@ gcv_status launch_sample_chunk(gcv_ctx* c, SampleParams P, int64_t c_lo, int64_t
         if (ns == 0) continue;
         P.cb = jb;
         P.ce = je;
-        CHECK(launch_sampler(c, r.code, P, ns));
+        cudaStream_t st;
+        CHECK(fork.stream(k++, &st));
+        CHECK(launch_sampler(c, r.code, P, ns, st));
     }
-    return GCV_OK;
+    return fork.join();
 }
 
 gcv_status ensure_copy_streams(gcv_ctx* c)
@@ -1399,25 +1483,13 @@ gcv_status enqueue_table_graph(gcv_ctx* c)
         k_setup<<<blocks, 256, 0, c->stream>>>(b, table_view(c), feat16, rtol_feature(c->opt.rtol));
         CU(cudaGetLastError());
     } else if (c->n_seg > 0) {
-        for (const CodeRange& r : c->code_ranges) CHECK(launch_setup_list(c, r, feat16));
+        CHECK(launch_setup_codes(c, feat16));
     }
     CU(cudaEventRecordWithFlags(c->ev[1], c->stream, cudaEventRecordExternal));
     if (learned) {
         CU(cudaMemsetAsync(c->starts.p, 0, (size_t)c->n_seg * sizeof(uint32_t), c->stream));
         const int md = mixed ? std::min(c->opt.max_depth, FF_MAX_DEPTH) : c->opt.max_depth;
-        // start depths in the order of the work items (the grouped list)
-        auto run = [&](const uint4* f16, uint32_t* starts, int64_t n) -> gcv_status {
-            cudaError_t e = mlp_starts_launch_bf16(f16, nullptr, n, c->mlp_w, md, starts, c->stream);
-            if (e != cudaSuccess) return cuda_fail(e, "network inference");
-            return GCV_OK;
-        };
-        if (c->code > 0) {
-            CHECK(run(c->feat16.p, c->starts.p, c->n_seg));
-        } else if (c->code < 0) {
-            for (const CodeRange& r : c->code_ranges)
-                if (r.code != CODE_ELLIPSE)
-                    CHECK(run(c->feat16.p + 2 * r.begin, c->starts.p + r.begin, r.end - r.begin));
-        }
+        CHECK(launch_network(c, md));
     }
     CU(cudaEventRecordWithFlags(c->ev[6], c->stream, cudaEventRecordExternal));
     if (c->n_seg > 0) {
@@ -1429,7 +1501,7 @@ gcv_status enqueue_table_graph(gcv_ctx* c)
         P.collect = c->opt.collect_stats;
         P.coef_ff = c->coef_ff.p;
         P.starts = learned ? c->starts.p : nullptr;
-        CHECK(launch_main_pass(c, P, true));
+        CHECK(launch_main_pass(c, P));
         // deep passes over the deep list, its length read on the device
         LengthParams Q = P;
         Q.list = c->deep_list.p;
@@ -1439,10 +1511,10 @@ gcv_status enqueue_table_graph(gcv_ctx* c)
         Q.starts = nullptr;
         Q.collect = 0;
         CU(cudaMemsetAsync(c->ctr.p + C_WORK, 0, sizeof(unsigned long long), c->stream));
-        CHECK(launch_length<1>(c, c->code, Q));
+        CHECK(launch_length<1>(c, c->code, Q, c->stream));
         Q.collect = P.collect;
         CU(cudaMemsetAsync(c->ctr.p + C_WORK, 0, sizeof(unsigned long long), c->stream));
-        CHECK(launch_length<2>(c, c->code, Q));
+        CHECK(launch_length<2>(c, c->code, Q, c->stream));
     }
     CU(cudaEventRecordWithFlags(c->ev[2], c->stream, cudaEventRecordExternal));
     const int64_t tiles = (c->n_seg + SCAN_TILE - 1) / SCAN_TILE;
@@ -1499,16 +1571,21 @@ gcv_status enqueue_sampling_graph(gcv_ctx* c, const int* d_counts, const double*
     if (c->code >= 0) {
         P.s_begin = 0;
         P.s_end_dev = c->sample_off.p + c->n_curve;
-        CHECK(launch_sampler(c, c->code, P, nominal));
+        CHECK(launch_sampler(c, c->code, P, nominal, c->stream));
     } else {
         CHECK(enqueue_count_scan(c, d_counts, c->curve_list.p, c->list_sample_off.p));
         P.curve_list = c->curve_list.p;
         P.list_off = c->list_sample_off.p;
+        Fork fork(c, c->curve_ranges.size());
+        size_t k = 0;
         for (const CodeRange& r : c->curve_ranges) {
             P.cb = r.begin;
             P.ce = r.end;
-            CHECK(launch_sampler(c, r.code, P, nominal));
+            cudaStream_t st;
+            CHECK(fork.stream(k++, &st));
+            CHECK(launch_sampler(c, r.code, P, nominal, st));
         }
+        CHECK(fork.join());
     }
     CU(cudaEventRecordWithFlags(c->ev[5], c->stream, cudaEventRecordExternal));
     return GCV_OK;
@@ -2174,6 +2251,10 @@ gcv_status gcv_host_free(void* p)
 
 gcv_status gcv_release_cached_memory(int64_t* bytes)
 {
+    {
+        std::lock_guard<std::mutex> g(g_kit_m);
+        g_kits.clear();
+    }
     const size_t n = release_cache(-1);
     if (bytes) *bytes = (int64_t)n;
     return GCV_OK;

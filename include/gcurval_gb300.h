@@ -263,7 +263,7 @@ gcv_status gcv_measure_fma_peak(int which, double* tflops);
  * samples/sample1_ellipse/main.cpp:147-155).  An allocation that finds the
  * GPU full frees the cache first.  Set GCV_NO_MEMORY_CACHE=1 in the
  * environment to free buffers at once instead.  This call frees the cached
- * buffers of every device; *bytes (may be NULL) receives how many bytes. */
+ * buffers of every device (and the few idle helper streams kept beside them); *bytes (may be NULL) receives how many bytes. */
 gcv_status gcv_release_cached_memory(int64_t* bytes);
 
 /* Page-locked host memory for the host-side arrays of gcv_create_batch and
