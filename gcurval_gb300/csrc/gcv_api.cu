@@ -287,9 +287,7 @@ struct Knobs {
 // before in the process each run one candidate; the fastest shapes, timed by
 // the context's events, are kept for that shape (curve code, precision,
 // learned form, log2 of the interval count).  The shapes change scheduling
-// only: every result is the same under each, bit for bit.  (The half-warp-per-interval mapping of the main
-// pass sums each panel's nodes in another order, so it is a user option,
-// gcv_options.mapping, not a shape the tuner may pick.)
+// only: every result is the same under each, bit for bit.
 constexpr int TUNE_TRIALS = 3;
 inline int trial_length_cap(int i) { return i == 1 ? 4 : (i == 2 ? 6 : 32); }
 inline Knobs trial_knobs(int i)
@@ -1028,13 +1026,14 @@ void tune_finish_if_done(gcv_ctx* c)
     }
 }
 
-// record the length passes' time (events ev[6] -> ev[2]) of a tuning build
+// record the length passes' time (events ev[7] -> ev[2]: without an attempt that
+// the leaf pool was too small for) of a tuning build
 gcv_status tune_after_table(gcv_ctx* c)
 {
     if (c->len_trial < 0 || c->len_trial >= TUNE_TRIALS) return GCV_OK;
     CU(cudaEventSynchronize(c->ev[2]));
     float ms = 0.f;
-    CU(cudaEventElapsedTime(&ms, c->ev[6], c->ev[2]));
+    CU(cudaEventElapsedTime(&ms, c->ev[7], c->ev[2]));
     c->len_ms[c->len_trial++] = ms;
     if (c->len_trial == TUNE_TRIALS && c->smp_trial >= 0 && c->smp_trial < TUNE_TRIALS) choose_length_knobs(c, c->knobs);
     tune_finish_if_done(c);
@@ -1144,6 +1143,7 @@ gcv_status build_table(gcv_ctx* c)
     CU(cudaEventRecord(c->ev[6], c->stream));
     for (int attempt = 0;; ++attempt) {
         if (attempt > 8) return fail(GCV_ERR_OVERFLOW, "deep list kept overflowing");
+        CU(cudaEventRecord(c->ev[7], c->stream));
         // keep the set-up's error bits, clear the rest
         CU(cudaMemsetAsync(c->ctr.p, 0, C_ERR * sizeof(unsigned long long), c->stream));
         CU(cudaMemsetAsync(c->ctr.p + C_WORK_CODE, 0, (C_COUNT - C_WORK_CODE) * sizeof(unsigned long long), c->stream));
@@ -1492,6 +1492,7 @@ gcv_status enqueue_table_graph(gcv_ctx* c)
         CHECK(launch_network(c, md));
     }
     CU(cudaEventRecordWithFlags(c->ev[6], c->stream, cudaEventRecordExternal));
+    CU(cudaEventRecordWithFlags(c->ev[7], c->stream, cudaEventRecordExternal));
     if (c->n_seg > 0) {
         LengthParams P{};
         P.b = b;

@@ -1,6 +1,6 @@
 // Device-side building blocks of the arc-length library: quadrature
-// constants, curve evaluators on per-knot-interval polynomials, the symbolic
-// de Boor set-up of those polynomials, and warp helpers.
+// constants, curve evaluators on per-knot-interval polynomials (set up by
+// gcv_setup.cuh), and warp helpers.
 //
 // Every knot interval ("segment") is mapped to a local variable v in [-1, 1]:
 //   B-spline  t = t0 + (v + 1) * hw,  hw = (k[span+1] - k[span]) / 2
@@ -67,29 +67,6 @@ __host__ __device__ constexpr double gl8_w(int i)
 }
 
 constexpr double PI = 3.141592653589793238462643383279502884;
-
-// Node of half-warp lane `hl` (0..15): lanes 0..6 take -x_k, lane 7 the
-// centre, lanes 8..14 +x_{14-hl}; lane 15 the panel's right end (weights 0).
-__host__ __device__ inline void gk_lane(int hl, double& x, double& wk, double& wg)
-{
-    if (hl < 7) {
-        x = -gk_x(hl);
-        wk = gk_wk(hl);
-        wg = gk_wg(hl);
-    } else if (hl == 7) {
-        x = 0.0;
-        wk = gk_wk(7);
-        wg = gk_wg(7);
-    } else if (hl < 15) {
-        x = gk_x(14 - hl);
-        wk = gk_wk(14 - hl);
-        wg = gk_wg(14 - hl);
-    } else {
-        x = 1.0;
-        wk = 0.0;
-        wg = 0.0;
-    }
-}
 
 // ------------------------------------------------------------ curve codes
 // 0 = ellipse; B-splines 16 + 4 p + D for degree p in 1..5 and D in {2, 3}.
@@ -296,90 +273,7 @@ __device__ __forceinline__ void point_dyn(int code, const double* __restrict__ s
     }
 }
 
-// ------------------------------------------------- symbolic de Boor set-up
-// Power-basis coefficients in v of the B-spline piece on knot span `span`
-// (k[span] < k[span+1]): the reference's basis recursion
-// (samples/sample2_bspline/BSpline.h:26-96, b_spline_func_value /
-// b_spline_derv_o1 / to_point) run on polynomials in v instead of numbers,
-// with u = m + w v, m the span midpoint and w its half width.  The
-// denominators right[r+1] + left[j-r] are knot differences and do not depend
-// on u.  Output: the position polynomial a[k][d], k = 0..P; the derivative
-// dC/dv is b[k][d] = (k + 1) a[k + 1][d] (see Eval::load_speed).
-template <int P, int D>
-__device__ void bspline_setup(const double* __restrict__ kv, const double* __restrict__ cp, int span,
-                              double* out)
-{
-    const double ka = kv[span], kb = kv[span + 1];
-    const double m = 0.5 * (ka + kb), w = 0.5 * (kb - ka);
-    // N[r][k]: basis polynomial r, coefficient of v^k (degree <= P)
-    double N[P + 1][P + 1];
-#pragma unroll
-    for (int r = 0; r <= P; ++r)
-#pragma unroll
-        for (int k = 0; k <= P; ++k) N[r][k] = 0.0;
-    N[0][0] = 1.0;
-    // at step j the basis polynomials N[0..j-1] have degree j - 1 and the
-    // new ones degree j: the loops run over those coefficients only
-#pragma unroll
-    for (int j = 1; j <= P; ++j) {
-        double saved[P + 1];
-#pragma unroll
-        for (int k = 0; k <= j; ++k) saved[k] = 0.0;
-#pragma unroll
-        for (int r = 0; r < j; ++r) {
-            const double kr = kv[span + r + 1];      // right[r+1] = kr - u
-            const double kl = kv[span + 1 - j + r];  // left[j-r]  = u - kl
-            const double inv = 1.0 / (kr - kl);
-            double temp[P + 1];
-#pragma unroll
-            for (int k = 0; k < j; ++k) temp[k] = N[r][k] * inv;
-            const double ra = kr - m, la = m - kl;  // right = ra - w v, left = la + w v
-#pragma unroll
-            for (int k = j; k >= 0; --k) {
-                if (k == j) {  // only the v * temp[j-1] terms reach degree j
-                    N[r][k] = saved[k] - w * temp[k - 1];
-                    saved[k] = w * temp[k - 1];
-                } else if (k == 0) {
-                    N[r][k] = saved[k] + ra * temp[k];
-                    saved[k] = la * temp[k];
-                } else {
-                    N[r][k] = saved[k] + (ra * temp[k] - w * temp[k - 1]);
-                    saved[k] = la * temp[k] + w * temp[k - 1];
-                }
-            }
-        }
-#pragma unroll
-        for (int k = 0; k <= j; ++k) N[j][k] = saved[k];
-    }
-    // position: C(v) = sum_i P_{span-P+i} N_i(v).  The basis sums to one, so
-    // combining differences P_i - P_0 and adding P_0 back to the constant
-    // term keeps the higher coefficients free of cancellation against |P|.
-    const double* c0 = cp + (size_t)(span - P) * D;
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-        const double q = c0[d];
-#pragma unroll
-        for (int k = 0; k <= P; ++k) {
-            double acc = 0.0;
-#pragma unroll
-            for (int i = 1; i <= P; ++i) acc = fma(c0[i * D + d] - q, N[i][k], acc);
-            out[k * D + d] = k == 0 ? acc + q : acc;
-        }
-    }
-}
-
 // ------------------------------------------------------------ warp helpers
-__device__ __forceinline__ double half_sum(double x, unsigned mask)
-{
-    // xor butterfly inside a 16-lane half: partners add a+b and b+a, so every
-    // lane ends with the bitwise-same total
-    x += __shfl_xor_sync(mask, x, 8);
-    x += __shfl_xor_sync(mask, x, 4);
-    x += __shfl_xor_sync(mask, x, 2);
-    x += __shfl_xor_sync(mask, x, 1);
-    return x;
-}
-
 // Non-negative doubles order like their bit patterns: binary searches on
 // cumulative lengths compare 64-bit integers instead of using the FP64 pipe.
 __device__ __forceinline__ long long dkey(double x) { return __double_as_longlong(x); }

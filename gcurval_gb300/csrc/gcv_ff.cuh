@@ -97,6 +97,15 @@ __device__ __forceinline__ long long fix_of_double(double x)
 }
 __device__ __forceinline__ long long fix_of_float(float x) { return __float2ll_rn(x * 1152921504606846976.0f); }
 
+// float -> double from the bit pattern (the FP64 pipe's conversion for zeros,
+// denormals, infinities and NaN)
+__device__ __forceinline__ double double_of_float(float x)
+{
+    const unsigned b = __float_as_uint(x), e = (b >> 23) & 0xFFu;
+    if (e == 0u || e == 0xFFu) return (double)x;
+    return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7FFFFFFFu) >> 3) + (896u << 20))), (int)(b << 29));
+}
+
 // reciprocal to an ulp, for factors that carry FP32 rounding anyway
 __device__ __forceinline__ float rcp_approx(float x) { return __fdividef(1.0f, x); }
 

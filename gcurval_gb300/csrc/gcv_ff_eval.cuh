@@ -159,7 +159,7 @@ struct EvalFF {
     static constexpr int D = code_dim(CODE);
     // A, B, w0 (ellipse piece) or the derivative polynomial
     // b[k][d] = (k + 1) a[k + 1][d], stored after the midpoint position a[0]
-    // (bspline_setup_ff)
+    // (gcv_setup.cuh)
     __device__ __forceinline__ static void load(const float2* __restrict__ seg, ff* r)
     {
         if constexpr (CODE == 0) {
@@ -303,85 +303,6 @@ struct EvalFF {
     }
 };
 
-// ------------------------------------------- symbolic de Boor set-up (FF)
-// bspline_setup (gcv_device.cuh) in float-float arithmetic, for tables built
-// for the mixed path: the same polynomial recursion in v on the FP32 pipes.
-// FP64 is used only to centre the data: knots relative to the span midpoint
-// m and control points relative to the first one of the span (differences
-// that carry the cancellation), each converted once to float-float.  The
-// constant term (the position at the midpoint) is formed in float-float.
-template <int P, int D>
-__device__ void bspline_setup_ff(const double* __restrict__ kv, const double* __restrict__ cp, int span, float2* out)
-{
-    const double ka = kv[span], kb = kv[span + 1];
-    const double m = 0.5 * (ka + kb);
-    const ff w = ff_from_double(0.5 * (kb - ka));
-    // knots span-P+1 .. span+P relative to m
-    ff dk[2 * P];
-#pragma unroll
-    for (int i = 0; i < 2 * P; ++i) dk[i] = ff_from_double(kv[span - P + 1 + i] - m);
-    // N[r][k]: basis polynomial r, coefficient of v^k
-    ff N[P + 1][P + 1];
-    N[0][0] = ff{1.0f, 0.0f};
-#pragma unroll
-    for (int j = 1; j <= P; ++j) {
-        ff saved[P + 1];
-#pragma unroll
-        for (int r = 0; r < j; ++r) {
-            const ff ra = dk[r + P];                // k[span + r + 1] - m
-            const ff la = ff_neg(dk[r + P - j]);    // m - k[span + 1 - j + r]
-            const ff inv = ff_recip(ff_add(ra, la));
-            ff temp[P + 1];
-#pragma unroll
-            for (int k = 0; k < j; ++k) temp[k] = ff_mul(N[r][k], inv);
-#pragma unroll
-            for (int k = j; k >= 0; --k) {
-                const ff a = r == 0 ? ff{0.0f, 0.0f} : saved[k];
-                if (k == j) {
-                    const ff wt = ff_mul(w, temp[k - 1]);
-                    N[r][k] = r == 0 ? ff_neg(wt) : ff_add(a, ff_neg(wt));
-                    saved[k] = wt;
-                } else if (k == 0) {
-                    const ff rt = ff_mul(ra, temp[0]);
-                    N[r][k] = r == 0 ? rt : ff_add(a, rt);
-                    saved[k] = ff_mul(la, temp[0]);
-                } else {
-                    const ff wt = ff_mul(w, temp[k - 1]);
-                    const ff rt = ff_fma(ra, temp[k], ff_neg(wt));
-                    N[r][k] = r == 0 ? rt : ff_add(a, rt);
-                    saved[k] = ff_fma(la, temp[k], wt);
-                }
-            }
-        }
-#pragma unroll
-        for (int k = 0; k <= j; ++k) N[j][k] = saved[k];
-    }
-    // C(v) = P_0 + sum_{i >= 1} (P_i - P_0) N_i(v)  (the basis sums to one)
-    const double* c0 = cp + (size_t)(span - P) * D;
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-        const double q = c0[d];
-        ff dp[P];
-#pragma unroll
-        for (int i = 1; i <= P; ++i) dp[i - 1] = ff_from_double(c0[i * D + d] - q);
-#pragma unroll
-        for (int k = 0; k <= P; ++k) {
-            ff acc{0.0f, 0.0f};
-#pragma unroll
-            for (int i = 1; i <= P; ++i) acc = i == 1 ? ff_mul(dp[0], N[1][k]) : ff_fma(dp[i - 1], N[i][k], acc);
-            // the position at the midpoint, P_0 + acc, in float-float (it
-            // only enters points, never the speed); the higher terms are
-            // stored as the derivative's coefficients k a_k, which the walk
-            // and the sampler read without rescaling
-            if (k == 0)
-                acc = ff_add(ff_from_double(q), acc);
-            else if (k > 1)
-                acc = ff_mul_f(acc, float(k));
-            out[k * D + d] = make_float2(acc.hi, acc.lo);
-        }
-    }
-}
-
 // B-spline panels by node pairs.  The speed polynomials p_d (degree P - 1 in
 // v) are shifted to the panel's midpoint m and scaled to its half width h:
 // b_j = h^j p_d^(j)(m) / j!, so p_d(m + h x) = sum_j b_j x^j on x in [-1, 1]
@@ -450,16 +371,22 @@ __host__ __device__ constexpr double gk_pair_wg(int i) { return i < 7 ? gk_wg(i)
 static __constant__ GkStep2 c_gk_step2[4] = {GCV_GK_STEP2(0), GCV_GK_STEP2(1), GCV_GK_STEP2(2), GCV_GK_STEP2(3)};
 #undef GCV_GK_STEP2
 
+// the midpoint of panel (k, depth), built exactly from the integer k
+__device__ __forceinline__ ff panel_mid(unsigned long long k, int depth)
+{
+    const float hw = __int_as_float((127 - depth) << 23);  // 2^-depth, exact
+    const float kh = (float)(unsigned)(k >> 24), kl = (float)(unsigned)(k & 0xFFFFFFull);
+    const float sh = __int_as_float((127 + 25 - depth) << 23), sl = 2.0f * hw;  // 2^(25-depth), 2^(1-depth)
+    return ff_add_f(ff_add_f(two_sum(-1.0f, kh * sh), kl * sl), hw);
+}
+
 // An ellipse piece's panel by angle addition (AngleTable), two node pairs per
 // packed step as in panel_k15_ff_pairs.  r: A, B, w0.
 __device__ __forceinline__ void panel_k15_ff_ellipse(const ff* r, unsigned long long k, int depth, ff& K, ff& G)
 {
     const float hw = __int_as_float((127 - depth) << 23);  // 2^-depth, exact
-    const float kh = (float)(unsigned)(k >> 24), kl = (float)(unsigned)(k & 0xFFFFFFull);
-    const float sh = __int_as_float((127 + 25 - depth) << 23), sl = 2.0f * hw;
-    const ff mid = ff_add_f(ff_add_f(two_sum(-1.0f, kh * sh), kl * sl), hw);
     ff sm, cm;
-    ff_sincospi(ff_add_f(ff_scale(mid, (float)ELLIPSE_PIECE_SCALE), r[2].hi), sm, cm);
+    ff_sincospi(ff_add_f(ff_scale(panel_mid(k, depth), (float)ELLIPSE_PIECE_SCALE), r[2].hi), sm, cm);
     const ff2 s2 = splat(sm), c2 = splat(cm), A = splat(r[0]), B = splat(r[1]);
     const float4* tab = reinterpret_cast<const float4*>(c_angle.ff[depth]);
     ff2 kk2{}, gg2{};
@@ -479,16 +406,12 @@ __device__ __forceinline__ void panel_k15_ff_ellipse(const ff* r, unsigned long 
     G = ff_scale(ff_add(lane0(gg2), lane1(gg2)), hw);
 }
 
-// b: the interval's speed coefficients on entry, shifted in place
-template <int CODE>
-__device__ __forceinline__ void panel_k15_ff_pairs(ff* b, unsigned long long k, int depth, ff& K, ff& G)
+// b: the interval's speed coefficients on entry, shifted to the panel's midpoint
+// and scaled to its half width in place
+template <int P, int D>
+__device__ __forceinline__ void panel_shift(ff* b, unsigned long long k, int depth)
 {
-    constexpr int P = code_degree(CODE), D = code_dim(CODE);
-    const float hw = __int_as_float((127 - depth) << 23);  // 2^-depth, exact
-    const float kh = (float)(unsigned)(k >> 24), kl = (float)(unsigned)(k & 0xFFFFFFull);
-    const float sh = __int_as_float((127 + 25 - depth) << 23), sl = 2.0f * hw;  // 2^(25-depth), 2^(1-depth)
-    const ff vlo = ff_add_f(two_sum(-1.0f, kh * sh), kl * sl);
-    const ff mid = ff_add_f(vlo, hw);
+    const ff mid = panel_mid(k, depth);
     // Taylor shift to mid: after pass i, b[i] holds p^(i)(mid) / i!
 #pragma unroll
     for (int i = 0; i < P - 1; ++i)
@@ -496,6 +419,7 @@ __device__ __forceinline__ void panel_k15_ff_pairs(ff* b, unsigned long long k, 
         for (int j = P - 2; j >= i; --j)
 #pragma unroll
             for (int d = 0; d < D; ++d) b[j * D + d] = ff_fma(b[(j + 1) * D + d], mid, b[j * D + d]);
+    const float hw = __int_as_float((127 - depth) << 23);
     float sc = hw;
 #pragma unroll
     for (int j = 1; j < P; ++j) {
@@ -503,6 +427,14 @@ __device__ __forceinline__ void panel_k15_ff_pairs(ff* b, unsigned long long k, 
         for (int d = 0; d < D; ++d) b[j * D + d] = ff_scale(b[j * D + d], sc);
         sc *= hw;
     }
+}
+
+template <int CODE>
+__device__ __forceinline__ void panel_k15_ff_pairs(ff* b, unsigned long long k, int depth, ff& K, ff& G)
+{
+    constexpr int P = code_degree(CODE), D = code_dim(CODE);
+    const float hw = __int_as_float((127 - depth) << 23);
+    panel_shift<P, D>(b, k, depth);
     // the node pairs two at a time in packed lanes (the centre in the last
     // step's second lane); the two lanes' sums are added at the end
     ff2 kk2{}, gg2{};

@@ -3,6 +3,7 @@
 // instantiates them, and by the header-only plugin path.
 #pragma once
 
+#include "gcv_setup.cuh"
 #include "gcv_table.cuh"
 
 namespace gcv {

@@ -1,38 +1,80 @@
 // The length pass with one half-warp per knot interval (float-float panels):
 // the alternative mapping to k_walk's one lane per panel, chosen by the
-// caller through gcv_options.mapping (GCV_MAP_HALF_WARP).  It is not an
-// autotuner choice: the two mappings sum K15 and G7 in different orders, and
-// a tuner's choice must leave every result bit-identical.
+// caller through gcv_options.mapping (GCV_MAP_HALF_WARP).
 //
-// The 16 lanes of a half-warp walk one interval's dyadic panels together:
-// in each panel lane hl evaluates one node (gk_lane: the 15 Kronrod nodes,
-// lane 15 idle), the half-warp sums K15 and G7 by shuffles, and the walk's
-// state (panel (k, depth), running sums, tolerance) is the same in all its
-// lanes.  Lane 0 of the half stages accepted leaves in shared memory; the
-// lanes write them out together when the interval is done.  The acceptance
-// test, the learned start, the leaf table and the deep-list hand-over are
-// those of k_walk<CODE, 1> (intervals of more than LCAP leaves go to the deep
-// passes here), so both mappings build the same table (up
-// to the summation order of K15 and G7).
+// The 16 lanes of a half-warp walk one interval's dyadic panels together: in
+// each panel a lane evaluates one node (the seven Kronrod pairs and the centre,
+// panel_ff_half), the nodes are gathered by shuffles and summed in k_walk's
+// order, and the walk's state (panel (k, depth), running sums, tolerance) is
+// the same in all lanes.  Lane 0 of the half stages accepted leaves in shared
+// memory; the lanes write them out together when the interval is done.  The
+// acceptance test, the learned start and the leaf table are those of
+// k_walk<CODE, 1> (intervals of more than LCAP leaves go to the deep passes
+// here), so both mappings build the same table up to float-float rounding (the
+// square roots are scalar here and packed there): lengths differ by at most
+// 6e-15 relative, curve parameters by 7e-13, over 1,500 uneven curves.
 //
-// Per panel this mapping spends 16 lanes on one node each plus the
-// shuffle reductions, where k_length spends one lane on seven node pairs
-// (gcv_ff_eval.cuh, panel_k15_ff_pairs); it holds far less state per lane
-// and finishes each interval 16 times sooner.
+// Per panel this mapping spends 16 lanes on one node each, every one of which
+// shifts the polynomials and adds up all pairs, where k_walk spends one lane on
+// all of them; it finishes an interval's panel sooner.
 #pragma once
 
 #include "gcv_length_impl.cuh"  // chord_of and the shared parameter block
 
 namespace gcv {
 
-// float-float sum over the 16 lanes of each half-warp (every lane of the
-// warp takes part), then lane 0's result for the whole half
-__device__ __forceinline__ ff half_warp_sum(ff a, int half_base)
+// K15 and G7 of a panel by the 16 lanes of a half-warp: lane hl evaluates one
+// node of pair hl % 8 (the eighth pair is the centre), every lane then adds the
+// pairs up in panel_ff's order, so the two agree to the rounding of
+// the square root.  Every lane of the warp takes part.
+template <int CODE>
+__device__ __forceinline__ void panel_ff_half(ff* r, unsigned long long k, int depth, int hl, int half_base, ff& K, ff& G)
 {
+    const unsigned FULL = 0xffffffffu;
+    const int i = hl & 7;
+    const bool plus = hl >= 8;
+    ff f;
+    if constexpr (CODE == 0) {
+        ff sm, cm;
+        ff_sincospi(ff_add_f(ff_scale(panel_mid(k, depth), (float)ELLIPSE_PIECE_SCALE), r[2].hi), sm, cm);
+        const float4 a = __ldg(reinterpret_cast<const float4*>(c_angle.ff[depth]) + i);
+        const ff sd{a.x, a.y}, s = ff_fma(cm, plus ? sd : ff_neg(sd), ff_mul(sm, ff{a.z, a.w}));
+        f = ff_sqrt(ff_fma(r[0], ff_mul(s, s), r[1]));
+    } else {
+        constexpr int P = code_degree(CODE), D = code_dim(CODE), N = P - 1;
+        constexpr int JE = (N % 2 == 0) ? N : N - 1, JO = (N % 2 == 1) ? N : N - 1;
+        panel_shift<P, D>(r, k, depth);
+        const GkStep2 c = c_gk_step2[i >> 1];
+        const ff x = i & 1 ? ff{c.xh.y, c.xl.y} : ff{c.xh.x, c.xl.x};
+        const ff x2 = i & 1 ? ff{c.x2h.y, c.x2l.y} : ff{c.x2h.x, c.x2l.x};
+        ff sum{0.0f, 0.0f};
 #pragma unroll
-    for (int o = 8; o > 0; o >>= 1)
-        a = ff_add(a, ff{__shfl_xor_sync(0xffffffffu, a.hi, o), __shfl_xor_sync(0xffffffffu, a.lo, o)});
-    return ff{__shfl_sync(0xffffffffu, a.hi, half_base), __shfl_sync(0xffffffffu, a.lo, half_base)};
+        for (int d = 0; d < D; ++d) {
+            ff e = r[JE * D + d];
+#pragma unroll
+            for (int j = JE - 2; j >= 0; j -= 2) e = ff_fma(e, x2, r[j * D + d]);
+            if constexpr (JO >= 1) {
+                ff o = r[JO * D + d];
+#pragma unroll
+                for (int j = JO - 2; j >= 1; j -= 2) o = ff_fma(o, x2, r[j * D + d]);
+                o = ff_mul(o, x);
+                e = ff_add(e, plus ? o : ff_neg(o));
+            }
+            sum = d == 0 ? ff_mul(e, e) : ff_fma(e, e, sum);
+        }
+        f = ff_sqrt(sum);
+    }
+    const ff pair = ff_add(f, ff{__shfl_xor_sync(FULL, f.hi, 8), __shfl_xor_sync(FULL, f.lo, 8)});
+    ff kk[2] = {}, gg[2] = {};
+#pragma unroll
+    for (int p = 0; p < 8; ++p) {
+        const ff s{__shfl_sync(FULL, pair.hi, half_base + p), __shfl_sync(FULL, pair.lo, half_base + p)};
+        kk[p & 1] = ff_fma(to_ff(split_const(gk_pair_wk(p))), s, kk[p & 1]);
+        gg[p & 1] = ff_fma(to_ff(split_const(gk_pair_wg(p))), s, gg[p & 1]);
+    }
+    const float hw = __int_as_float((127 - depth) << 23);
+    K = ff_scale(ff_add(kk[0], kk[1]), hw);
+    G = ff_scale(ff_add(gg[0], gg[1]), hw);
 }
 
 template <int CODE>
@@ -49,11 +91,6 @@ __global__ void __launch_bounds__(LK_THREADS) k_length_hw(LengthParams P)
     const int lane = threadIdx.x & 31, hl = lane & 15, half_base = lane & 16, half = threadIdx.x >> 4;
     const unsigned half_mask = half_base ? 0xffff0000u : 0x0000ffffu;
     const double eps50 = 50.0 * 1.4210854715202004e-14;  // round-off floor: 50 float-float units
-
-    // this lane's node and weights
-    double xd, wkd, wgd;
-    gk_lane(hl, xd, wkd, wgd);
-    const ff xn = ff_from_double(xd), wk = ff_from_double(wkd), wg = ff_from_double(wgd);
 
     const int64_t n_items = P.n_items_dev ? (int64_t)*P.n_items_dev : P.n_items;
     bool active = false, exhausted = false;
@@ -121,23 +158,15 @@ __global__ void __launch_bounds__(LK_THREADS) k_length_hw(LengthParams P)
         }
         // ---- one panel per active half: each lane one node
         const float hwf = __int_as_float((127 - depth) << 23);  // 2^-depth
-        ff Kf{0.0f, 0.0f}, Gf{0.0f, 0.0f};
-        if (active && hl < 15) {
-            const float kh = (float)(unsigned)(k >> 24), kl = (float)(unsigned)(k & 0xFFFFFFull);
-            const float sh = __int_as_float((127 + 25 - depth) << 23), sl = 2.0f * hwf;
-            const ff vlo = ff_add_f(two_sum(-1.0f, kh * sh), kl * sl);
-            const ff v = ff_add(ff_add_f(vlo, hwf), ff_scale(xn, hwf));
-            ff rl[MAX_COEF];
-            EvalFF<CODE>::load(cff, rl);
-            const ff f = EvalFF<CODE>::speed(rl, v);
-            Kf = ff_mul(wk, f);
-            Gf = ff_mul(wg, f);
-        }
-        Kf = half_warp_sum(Kf, half_base);
-        Gf = half_warp_sum(Gf, half_base);
+        ff Kf, Gf, rl[MAX_COEF];
         if (active) {
-            Kf = ff_scale(Kf, hwf);
-            Gf = ff_scale(Gf, hwf);
+            EvalFF<CODE>::load(cff, rl);
+        } else {
+#pragma unroll
+            for (ff& x : rl) x = ff{0.0f, 0.0f};
+        }
+        panel_ff_half<CODE>(rl, k, depth, hl, half_base, Kf, Gf);
+        if (active) {
             if (depth == 0) {
                 tol_unit = P.rtol * fabs(ff_to_double(Kf));
                 tol_f = (float)tol_unit;

@@ -11,7 +11,7 @@
 namespace gcv {
 
 // set-up of one B-spline interval for a mixed-path table: float-float
-// coefficients straight from the float-float recursion
+// coefficients straight from the float-float expansion
 template <int P, int D>
 __device__ void setup_bspline_seg_ff(const Batch& b, const Table& t, int64_t s, int64_t c)
 {
@@ -21,18 +21,22 @@ __device__ void setup_bspline_seg_ff(const Batch& b, const Table& t, int64_t s, 
     const double* cp = b.ctrl + b.ctrl_off[c];
     const int span = int(j) + P;
     float2* at = t.coef_ff + b.coef_off[c] + j * N;
-    const double ka = kv[span], kb = kv[span + 1];
-    if (!(kb >= ka)) raise_err(t, ERR_BAD_KNOTS);
-    if (kb > ka) {
-        bspline_setup_ff<P, D>(kv, cp, span, at);
+    const double ka = kv[span], kb = kv[span + 1], width = kb - ka;
+    // kb > ka and !(kb >= ka) from the sign of the difference (its bit pattern:
+    // off the FP64 pipe), the values themselves where it is NaN
+    const long long wb = __double_as_longlong(width);
+    const bool nan = (wb & 0x7FFFFFFFFFFFFFFFll) > 0x7FF0000000000000ll;
+    if (nan ? !(kb >= ka) : wb < 0) raise_err(t, ERR_BAD_KNOTS);
+    if (!nan && wb > 0) {
+        bspline_setup_ff<P, D>(kv, cp, span, width, at);
         t.seg_t0[s] = ka;
         t.seg_t1[s] = kb;
         ff r[P * D];
         float q0;
         EvalFF<bs_code(P, D)>::load(at, r);
         // the start speed and slope only shape the sampler's first guess: FP32
-        t.seg_f0[s] = (double)EvalFF<bs_code(P, D)>::speed_slope32(r, -1.0f, q0);
-        t.seg_q0[s] = (double)q0;
+        t.seg_f0[s] = double_of_float(EvalFF<bs_code(P, D)>::speed_slope32(r, -1.0f, q0));
+        t.seg_q0[s] = double_of_float(q0);
     } else {
 #pragma unroll
         for (int i = 0; i < N; ++i) at[i] = make_float2(0.0f, 0.0f);

@@ -84,8 +84,8 @@ typedef struct gcv_options {
                              GCV_MAP_LANE (default) one thread per panel, a warp
                              sharing its intervals' panels, or
                              GCV_MAP_HALF_WARP 16 threads per knot interval, one panel node
-                             each; the same table up to the summation order of each
-                             panel's nodes (float-float rounding); no effect on GCV_PLAIN_FP64 */
+                             each; the same table up to
+                             float-float rounding; no effect on GCV_PLAIN_FP64 */
     int host_in_place;    /* nonzero: gcv_create_batch with GCV_HOST does not copy page-locked
                              knot and control arrays (gcv_host_alloc, cudaMallocHost,
                              cudaHostRegister); every table build reads them in place over the
