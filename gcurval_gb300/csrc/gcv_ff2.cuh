@@ -72,13 +72,33 @@ __device__ __forceinline__ ff2 ff2_fma(ff2 a, ff2 b, ff2 c)
     return fast_two_sum2(s.hi, add2(s.lo, add2(t, c.lo)));
 }
 
-// ff_sqrt, lane by lane (0 for a zero lane, NaN for a negative one)
-__device__ __forceinline__ ff2 ff2_sqrt(ff2 a)
+// ff_fma_open, ff_mul_open and a sum left unnormalised, lane by lane
+__device__ __forceinline__ ff2 ff2_fma_open(ff2 a, ff2 b, ff2 c)
+{
+    const float2 p = mul2(a.hi, b.hi);
+    const float2 t = fma2(a.hi, b.lo, fma2(a.lo, b.hi, fma2(a.hi, b.hi, neg2(p))));
+    const ff2 s = two_sum2(p, c.hi);
+    return ff2{s.hi, add2(s.lo, add2(t, c.lo))};
+}
+__device__ __forceinline__ ff2 ff2_mul_open(ff2 a, ff2 b)
+{
+    const float2 p = mul2(a.hi, b.hi);
+    return ff2{p, fma2(a.hi, b.lo, fma2(a.lo, b.hi, fma2(a.hi, b.hi, neg2(p))))};
+}
+__device__ __forceinline__ ff2 ff2_add_open(ff2 a, ff2 b)
+{
+    const ff2 s = two_sum2(a.hi, b.hi);
+    return ff2{s.hi, add2(s.lo, add2(a.lo, b.lo))};
+}
+
+// ff_sqrt without the last normalisation, lane by lane (0 for a zero lane, NaN for a negative one)
+__device__ __forceinline__ ff2 ff2_sqrt_open(ff2 a)
 {
     const float2 y = make_float2(rsqrtf(a.hi.x), rsqrtf(a.hi.y));
     const float2 s = mul2(a.hi, y);
     const float2 r = add2(fma2(neg2(s), s, a.hi), a.lo);
-    ff2 q = fast_two_sum2(s, mul2(r, make_float2(0.5f * y.x, 0.5f * y.y)));
+    const float2 c = mul2(r, make_float2(0.5f * y.x, 0.5f * y.y));
+    ff2 q{s, fma2(mul2(c, make_float2(1.5f, 1.5f)), mul2(c, y), c)};
     if (!(a.hi.x > 0.0f)) {
         q.hi.x = a.hi.x == 0.0f ? 0.0f : __fsqrt_rn(a.hi.x);
         q.lo.x = 0.0f;

@@ -80,19 +80,24 @@ __host__ __device__ constexpr double series_cospi(double x)
 // sin(pi (w_m -+ d_i)) = sin(pi w_m) cos(pi d_i) -+ cos(pi w_m) sin(pi d_i).
 // The offsets depend on the depth alone, so their sines and cosines are a
 // table, and a panel evaluates one sine and cosine instead of fifteen.
+// Order of the panels' node pairs: those of the Gauss rule first (1, 3, 5, and the
+// centre, 7), then the Kronrod-only ones
+__host__ __device__ constexpr int gk_pair(int j) { return j < 4 ? 2 * j + 1 : 2 * j - 8; }
+__host__ __device__ constexpr double gk_pair_x(int j) { return gk_pair(j) < 7 ? gk_x(gk_pair(j)) : 0.0; }
+
 constexpr int ANGLE_DEPTHS = 49;  // 0 .. MAX_DEPTH_LIMIT
 struct alignas(16) AngleTable {
     double sc[ANGLE_DEPTHS][8][2];  // pair i: sin(pi d_i), 1 - cos(pi d_i); entry 7 is the centre
-    float ff[ANGLE_DEPTHS][8][4];   // float-float sine and cosine: sin hi, lo, cos hi, lo
+    float ff[ANGLE_DEPTHS][8][4];   // float-float sine and cosine of pair gk_pair(i): sin hi, lo, cos hi, lo
     __host__ __device__ constexpr AngleTable() : sc(), ff()
     {
         double h = ELLIPSE_PIECE_SCALE;
         for (int d = 0; d < ANGLE_DEPTHS; ++d, h *= 0.5)
             for (int i = 0; i < 8; ++i) {
-                const double x = i < 7 ? h * gk_x(i) : 0.0;
-                const double s = series_sinpi(x), c = series_cospi(x), h2 = series_sinpi(0.5 * x);
-                sc[d][i][0] = s;
+                const double x = i < 7 ? h * gk_x(i) : 0.0, h2 = series_sinpi(0.5 * x);
+                sc[d][i][0] = series_sinpi(x);
                 sc[d][i][1] = 2.0 * h2 * h2;
+                const double s = series_sinpi(h * gk_pair_x(i)), c = series_cospi(h * gk_pair_x(i));
                 ff[d][i][0] = split_const(s).hi;
                 ff[d][i][1] = split_const(s).lo;
                 ff[d][i][2] = split_const(c).hi;
@@ -129,8 +134,9 @@ __device__ __forceinline__ void ff_sincospi(ff x, ff& s, ff& c)
     const ff2 U = splat(ff_mul(u, u));
     ff2 p = pack(to_ff(split_const(sinpi_coef(SINCOS_TERMS - 1))), to_ff(split_const(cospi_coef(SINCOS_TERMS - 1))));
 #pragma unroll
-    for (int k = SINCOS_TERMS - 2; k >= 0; --k)
-        p = ff2_fma(p, U, pack(to_ff(split_const(sinpi_coef(k))), to_ff(split_const(cospi_coef(k)))));
+    for (int k = SINCOS_TERMS - 2; k >= 1; --k)
+        p = ff2_fma_open(p, U, pack(to_ff(split_const(sinpi_coef(k))), to_ff(split_const(cospi_coef(k)))));
+    p = ff2_fma(p, U, pack(to_ff(split_const(sinpi_coef(0))), to_ff(split_const(cospi_coef(0)))));
     const ff a = ff_mul(lane0(p), u), b = lane1(p);
     s = swap ? b : a;
     c = swap ? a : b;
@@ -146,8 +152,9 @@ __device__ __forceinline__ void ff_sincospi_small(ff d, ff& s, ff& c)
     const ff2 U = splat(ff_mul(d, d));
     ff2 p = pack(to_ff(split_const(sinpi_coef(SMALL_TERMS - 1))), to_ff(split_const(cospi_coef(SMALL_TERMS - 1))));
 #pragma unroll
-    for (int k = SMALL_TERMS - 2; k >= 0; --k)
-        p = ff2_fma(p, U, pack(to_ff(split_const(sinpi_coef(k))), to_ff(split_const(cospi_coef(k)))));
+    for (int k = SMALL_TERMS - 2; k >= 1; --k)
+        p = ff2_fma_open(p, U, pack(to_ff(split_const(sinpi_coef(k))), to_ff(split_const(cospi_coef(k)))));
+    p = ff2_fma(p, U, pack(to_ff(split_const(sinpi_coef(0))), to_ff(split_const(cospi_coef(0)))));
     s = ff_mul(lane0(p), d);
     c = lane1(p);
 }
@@ -222,10 +229,11 @@ struct EvalFF {
         for (int d = 0; d < D; ++d) {
             ff2 acc = splat(r[(P - 1) * D + d]);
 #pragma unroll
-            for (int k = P - 2; k >= 0; --k) acc = ff2_fma(acc, v, splat(r[k * D + d]));
-            s = d == 0 ? ff2_mul(acc, acc) : ff2_fma(acc, acc, s);
+            for (int k = P - 2; k >= 1; --k) acc = ff2_fma_open(acc, v, splat(r[k * D + d]));
+            if constexpr (P > 1) acc = ff2_fma(acc, v, splat(r[d]));
+            s = d == 0 ? ff2_mul_open(acc, acc) : (d + 1 < D ? ff2_fma_open(acc, acc, s) : ff2_fma(acc, acc, s));
         }
-        return ff2_sqrt(s);
+        return ff2_sqrt_open(s);
     }
     // Speed rounded to FP32 and q at a float-float point (B-splines): the
     // components in float-float (Horner at the full point), their norm in FP32
@@ -330,35 +338,33 @@ __device__ __forceinline__ void ff_node_pair2(const ff* b, ff2 x, ff2 x2, ff2& f
     for (int d = 0; d < D; ++d) {
         ff2 e = splat(b[JE * D + d]);
 #pragma unroll
-        for (int j = JE - 2; j >= 0; j -= 2) e = ff2_fma(e, x2, splat(b[j * D + d]));
+        for (int j = JE - 2; j >= 0; j -= 2) e = ff2_fma_open(e, x2, splat(b[j * D + d]));
         ff2 lo_ = e, hi_ = e;
         if constexpr (JO >= 1) {
             ff2 o = splat(b[JO * D + d]);
 #pragma unroll
-            for (int j = JO - 2; j >= 1; j -= 2) o = ff2_fma(o, x2, splat(b[j * D + d]));
-            o = ff2_mul(o, x);
+            for (int j = JO - 2; j >= 1; j -= 2) o = ff2_fma_open(o, x2, splat(b[j * D + d]));
+            o = ff2_mul_open(o, x);
             lo_ = ff2_add(e, ff2_neg(o));
             hi_ = ff2_add(e, o);
         }
-        sm = d == 0 ? ff2_mul(lo_, lo_) : ff2_fma(lo_, lo_, sm);
-        sp = d == 0 ? ff2_mul(hi_, hi_) : ff2_fma(hi_, hi_, sp);
+        sm = d == 0 ? ff2_mul_open(lo_, lo_) : (d + 1 < D ? ff2_fma_open(lo_, lo_, sm) : ff2_fma(lo_, lo_, sm));
+        sp = d == 0 ? ff2_mul_open(hi_, hi_) : (d + 1 < D ? ff2_fma_open(hi_, hi_, sp) : ff2_fma(hi_, hi_, sp));
     }
-    fm = ff2_sqrt(sm);
-    fp = ff2_sqrt(sp);
+    fm = ff2_sqrt_open(sm);
+    fp = ff2_sqrt_open(sp);
 }
 
-// The seven Kronrod node pairs and the centre as four packed steps: step j
-// holds pairs 2j and 2j + 1, and the eighth lane is the centre node (x = 0:
-// both of its "nodes" are the centre, so it carries half the centre
-// weights).  Per step: x, x^2, the Kronrod weights and the Gauss weights
-// (zero on the Kronrod-only pairs), each as the hi / lo float pairs of both
-// lanes.
+// The seven Kronrod node pairs and the centre as four packed steps.  The first
+// two hold the pairs that are Gauss nodes too, so that only they add to G; the
+// eighth lane is the centre node (x = 0: both of its "nodes" are the centre, so it
+// carries half the centre weights).  Per step: x, x^2, the Kronrod weights and
+// the Gauss weights, each as the hi / lo float pairs of both lanes.
 struct GkStep2 {
     float2 xh, xl, x2h, x2l, wkh, wkl, wgh, wgl;
 };
-__host__ __device__ constexpr double gk_pair_x(int i) { return i < 7 ? gk_x(i) : 0.0; }
-__host__ __device__ constexpr double gk_pair_wk(int i) { return i < 7 ? gk_wk(i) : 0.5 * gk_wk(7); }
-__host__ __device__ constexpr double gk_pair_wg(int i) { return i < 7 ? gk_wg(i) : 0.5 * gk_wg(7); }
+__host__ __device__ constexpr double gk_pair_wk(int j) { return gk_pair(j) < 7 ? gk_wk(gk_pair(j)) : 0.5 * gk_wk(7); }
+__host__ __device__ constexpr double gk_pair_wg(int j) { return gk_pair(j) < 7 ? gk_wg(gk_pair(j)) : 0.5 * gk_wg(7); }
 #define GCV_GK_STEP2(j)                                                                                          \
     {{split_const(gk_pair_x(2 * j)).hi, split_const(gk_pair_x(2 * j + 1)).hi},                                  \
      {split_const(gk_pair_x(2 * j)).lo, split_const(gk_pair_x(2 * j + 1)).lo},                                  \
@@ -370,6 +376,13 @@ __host__ __device__ constexpr double gk_pair_wg(int i) { return i < 7 ? gk_wg(i)
      {split_const(gk_pair_wg(2 * j)).lo, split_const(gk_pair_wg(2 * j + 1)).lo}}
 static __constant__ GkStep2 c_gk_step2[4] = {GCV_GK_STEP2(0), GCV_GK_STEP2(1), GCV_GK_STEP2(2), GCV_GK_STEP2(3)};
 #undef GCV_GK_STEP2
+// step j's sums of node pairs into K and G
+__device__ __forceinline__ void gk_add(int j, ff2 sum, ff2& kk2, ff2& gg2)
+{
+    const GkStep2& c = c_gk_step2[j];
+    kk2 = ff2_fma(ff2{c.wkh, c.wkl}, sum, kk2);
+    if (j < 2) gg2 = ff2_fma(ff2{c.wgh, c.wgl}, sum, gg2);
+}
 
 // the midpoint of panel (k, depth), built exactly from the integer k
 __device__ __forceinline__ ff panel_mid(unsigned long long k, int depth)
@@ -394,13 +407,11 @@ __device__ __forceinline__ void panel_k15_ff_ellipse(const ff* r, unsigned long 
     for (int j = 0; j < 4; ++j) {
         const float4 a = __ldg(tab + 2 * j), b = __ldg(tab + 2 * j + 1);
         const ff2 sd{make_float2(a.x, b.x), make_float2(a.y, b.y)}, cd{make_float2(a.z, b.z), make_float2(a.w, b.w)};
-        const ff2 p = ff2_mul(s2, cd);
+        const ff2 p = ff2_mul_open(s2, cd);
         const ff2 up = ff2_fma(c2, sd, p), dn = ff2_fma(c2, ff2_neg(sd), p);
-        const ff2 fm = ff2_sqrt(ff2_fma(A, ff2_mul(dn, dn), B)), fp = ff2_sqrt(ff2_fma(A, ff2_mul(up, up), B));
-        const ff2 sum = ff2_add(fm, fp);
-        const GkStep2 c = c_gk_step2[j];
-        kk2 = ff2_fma(ff2{c.wkh, c.wkl}, sum, kk2);
-        gg2 = ff2_fma(ff2{c.wgh, c.wgl}, sum, gg2);
+        const ff2 fm = ff2_sqrt_open(ff2_fma(A, ff2_mul_open(dn, dn), B));
+        const ff2 fp = ff2_sqrt_open(ff2_fma(A, ff2_mul_open(up, up), B));
+        gk_add(j, ff2_add_open(fm, fp), kk2, gg2);
     }
     K = ff_scale(ff_add(lane0(kk2), lane1(kk2)), hw);
     G = ff_scale(ff_add(lane0(gg2), lane1(gg2)), hw);
@@ -418,7 +429,7 @@ __device__ __forceinline__ void panel_shift(ff* b, unsigned long long k, int dep
 #pragma unroll
         for (int j = P - 2; j >= i; --j)
 #pragma unroll
-            for (int d = 0; d < D; ++d) b[j * D + d] = ff_fma(b[(j + 1) * D + d], mid, b[j * D + d]);
+            for (int d = 0; d < D; ++d) b[j * D + d] = ff_fma_open(b[(j + 1) * D + d], mid, b[j * D + d]);
     const float hw = __int_as_float((127 - depth) << 23);
     float sc = hw;
 #pragma unroll
@@ -444,12 +455,10 @@ __device__ __forceinline__ void panel_k15_ff_pairs(ff* b, unsigned long long k, 
     // unrolled, 13.0 rolled).
 #pragma unroll 1
     for (int j = 0; j < 4; ++j) {
-        const GkStep2 c = c_gk_step2[j];
+        const GkStep2& c = c_gk_step2[j];
         ff2 fm, fp;
         ff_node_pair2<P, D>(b, ff2{c.xh, c.xl}, ff2{c.x2h, c.x2l}, fm, fp);
-        const ff2 sum = ff2_add(fm, fp);
-        kk2 = ff2_fma(ff2{c.wkh, c.wkl}, sum, kk2);
-        gg2 = ff2_fma(ff2{c.wgh, c.wgl}, sum, gg2);  // zero weights on the Kronrod-only pairs
+        gk_add(j, ff2_add_open(fm, fp), kk2, gg2);
     }
     const ff kk = ff_add(lane0(kk2), lane1(kk2));
     const ff gg = ff_add(lane0(gg2), lane1(gg2));

@@ -38,8 +38,8 @@ __device__ __forceinline__ void panel_ff_half(ff* r, unsigned long long k, int d
         ff sm, cm;
         ff_sincospi(ff_add_f(ff_scale(panel_mid(k, depth), (float)ELLIPSE_PIECE_SCALE), r[2].hi), sm, cm);
         const float4 a = __ldg(reinterpret_cast<const float4*>(c_angle.ff[depth]) + i);
-        const ff sd{a.x, a.y}, s = ff_fma(cm, plus ? sd : ff_neg(sd), ff_mul(sm, ff{a.z, a.w}));
-        f = ff_sqrt(ff_fma(r[0], ff_mul(s, s), r[1]));
+        const ff sd{a.x, a.y}, s = ff_fma(cm, plus ? sd : ff_neg(sd), ff_mul_open(sm, ff{a.z, a.w}));
+        f = ff_sqrt(ff_fma(r[0], ff_mul_open(s, s), r[1]));
     } else {
         constexpr int P = code_degree(CODE), D = code_dim(CODE), N = P - 1;
         constexpr int JE = (N % 2 == 0) ? N : N - 1, JO = (N % 2 == 1) ? N : N - 1;
@@ -52,15 +52,15 @@ __device__ __forceinline__ void panel_ff_half(ff* r, unsigned long long k, int d
         for (int d = 0; d < D; ++d) {
             ff e = r[JE * D + d];
 #pragma unroll
-            for (int j = JE - 2; j >= 0; j -= 2) e = ff_fma(e, x2, r[j * D + d]);
+            for (int j = JE - 2; j >= 0; j -= 2) e = ff_fma_open(e, x2, r[j * D + d]);
             if constexpr (JO >= 1) {
                 ff o = r[JO * D + d];
 #pragma unroll
-                for (int j = JO - 2; j >= 1; j -= 2) o = ff_fma(o, x2, r[j * D + d]);
-                o = ff_mul(o, x);
+                for (int j = JO - 2; j >= 1; j -= 2) o = ff_fma_open(o, x2, r[j * D + d]);
+                o = ff_mul_open(o, x);
                 e = ff_add(e, plus ? o : ff_neg(o));
             }
-            sum = d == 0 ? ff_mul(e, e) : ff_fma(e, e, sum);
+            sum = d == 0 ? ff_mul_open(e, e) : (d + 1 < D ? ff_fma_open(e, e, sum) : ff_fma(e, e, sum));
         }
         f = ff_sqrt(sum);
     }
@@ -70,7 +70,7 @@ __device__ __forceinline__ void panel_ff_half(ff* r, unsigned long long k, int d
     for (int p = 0; p < 8; ++p) {
         const ff s{__shfl_sync(FULL, pair.hi, half_base + p), __shfl_sync(FULL, pair.lo, half_base + p)};
         kk[p & 1] = ff_fma(to_ff(split_const(gk_pair_wk(p))), s, kk[p & 1]);
-        gg[p & 1] = ff_fma(to_ff(split_const(gk_pair_wg(p))), s, gg[p & 1]);
+        if (p < 4) gg[p & 1] = ff_fma(to_ff(split_const(gk_pair_wg(p))), s, gg[p & 1]);
     }
     const float hw = __int_as_float((127 - depth) << 23);
     K = ff_scale(ff_add(kk[0], kk[1]), hw);

@@ -44,8 +44,8 @@ static __constant__ float2 c_gl8_ff[12] = {
 // (gl8_pairs) rather than by evaluating each node: the B-spline codes of
 // degree x dimension below 10.  The larger codes hold more coefficients than
 // their register cap leaves room for beside the pairs' temporaries: sampling of
-// 50,000 spatial cubics and quintics took 11.0 ms with pairs below 8, 10.8
-// below 10, 10.9 for every code (with the pairs' loop rolled).
+// 50,000 spatial cubics and quintics took 10.4 ms with pairs below 8, 10.2
+// below 10, 11.1 for every code.
 __host__ __device__ constexpr bool sample_node_pairs(int code)
 {
     return code > 0 && code_degree(code) * code_dim(code) < 10;
@@ -67,7 +67,7 @@ __device__ __forceinline__ ff gl8_pairs(ff* b, ff m, ff h)
 #pragma unroll
         for (int j = P - 2; j >= i; --j)
 #pragma unroll
-            for (int d = 0; d < D; ++d) b[j * D + d] = ff_fma(b[(j + 1) * D + d], m, b[j * D + d]);
+            for (int d = 0; d < D; ++d) b[j * D + d] = ff_fma_open(b[(j + 1) * D + d], m, b[j * D + d]);
     // pairs (0, 1) and (2, 3) in packed lanes
     const ff2 h2 = splat(h);
     ff2 I2{};
@@ -76,7 +76,7 @@ __device__ __forceinline__ ff gl8_pairs(ff* b, ff m, ff h)
         const ff2 X = ff2_mul(h2, pack(to_ff(split_const(gl8_x(k))), to_ff(split_const(gl8_x(k + 1)))));
         ff2 fm, fp;
         ff_node_pair2<P, D>(b, X, ff2_mul(X, X), fm, fp);
-        I2 = ff2_fma(pack(to_ff(split_const(gl8_w(k))), to_ff(split_const(gl8_w(k + 1)))), ff2_add(fm, fp), I2);
+        I2 = ff2_fma(pack(to_ff(split_const(gl8_w(k))), to_ff(split_const(gl8_w(k + 1)))), ff2_add_open(fm, fp), I2);
     }
     return ff_add(lane0(I2), lane1(I2));
 }
@@ -97,9 +97,9 @@ __device__ __forceinline__ ff gl8_ellipse(const ff* r, const EllipseMid& e, ff h
     for (int k = 0; k < 4; ++k) {
         ff sd, cd;
         ff_sincospi_small(ff_mul(h8, ff{c_gl8_ff[4 + k].x, c_gl8_ff[4 + k].y}), sd, cd);
-        const ff q = ff_mul(e.cm, sd);
-        const ff2 s = ff2_add(splat(ff_mul(e.sm, cd)), pack(ff_neg(q), q));
-        const ff2 f = ff2_sqrt(ff2_fma(A, ff2_mul(s, s), B));
+        const ff q = ff_mul_open(e.cm, sd);
+        const ff2 s = ff2_add(splat(ff_mul_open(e.sm, cd)), pack(ff_neg(q), q));
+        const ff2 f = ff2_sqrt_open(ff2_fma(A, ff2_mul_open(s, s), B));
         I = ff_fma(ff{c_gl8_ff[8 + k].x, c_gl8_ff[8 + k].y}, ff_add(lane0(f), lane1(f)), I);
     }
     return I;
@@ -194,9 +194,9 @@ __device__ __forceinline__ long long ff_leaf_newton(const TAB* __restrict__ seg,
             const float d = 2.0f * Fh * rcp_approx(f0 + f1);
             const float r1 = rcp_approx(f1), s0 = q0 * r0, s1 = q1 * r1;  // f'(w), f'(w - dn)
             float res = dn * dn * (fabsf(s1 - s0) * (1.0f / 3.0f) + s1 * s1 * fabsf(dn) * 0.25f * r1);
-            // at FP64 tolerances the FP32 rounding of the step itself counts:
+            // at tight tolerances the FP32 rounding of the step itself counts:
             // f0, f1 and the quotient are good to a few 2^-24 of F
-            if constexpr (FROM64) res = fmaf(5e-7f, fabsf(Fh), res);
+            res = fmaf(5e-7f, fabsf(Fh), res);
             const float wd = w.hi - d;
             if (res <= eps_s && wd >= 0.0f && wd <= dv) {
                 last = d;  // converged with this step
@@ -223,11 +223,12 @@ __device__ __forceinline__ long long ff_leaf_newton(const TAB* __restrict__ seg,
 // last one's interval: 14.5 ms against 11.9 on 50,000 spatial curves; lanes that
 // take their next sample while others iterate: 14.9.)
 // Registers per thread are capped (blocks of up to SAMPLE_THREADS_MAX threads
-// still fit) at 72, 7 blocks of 128 threads per SM, with up to 60 bytes of
-// spills: the kernel waits on fixed latencies and table loads more than on any
-// pipe.  Sampling of the uneven batch of 100,000 curves took 14.0 ms at 96
-// registers, 13.3 at 80 - 88, 12.8 at 72 and at 64 (the other parts as then).
-constexpr int SAMPLE_FF_REGS = 72;
+// still fit) at 64, 8 blocks of 128 threads per SM, at the price of spills: the
+// kernel waits on fixed latencies and table loads more than on any
+// pipe.  Sampling of the uneven batch of 100,000 curves took 11.76 ms at 80
+// registers, 11.40 at 72, 11.24 at 64; unnormalised inner steps (gcv_ff.cuh)
+// were worth 0.47 ms of it.
+constexpr int SAMPLE_FF_REGS = 64;
 static_assert(SAMPLE_FF_REGS * SAMPLE_THREADS_MAX <= 65536, "a block of SAMPLE_THREADS_MAX must fit one SM");
 //
 // TAB = double runs the same kernel on an FP64 table (GCV_PLAIN_FP64 at
@@ -241,8 +242,8 @@ static_assert(SAMPLE_FF_REGS * SAMPLE_THREADS_MAX <= 65536, "a block of SAMPLE_T
 // 2^-sexp, the binary exponent of its mean speed, so that curves of any
 // double magnitude fit FP32's exponent range.  The FP64 kernel was bound by
 // the FP64 pipe (91 % busy, one warp instruction per 64 issue slots); this one
-// by issue.  4,096 ellipses x 1,000 samples: 4.15 -> 0.48 ms; 10,000 planar
-// cubics x 1,024: 8.51 -> 0.84 ms.  Position errors at rtol 1e-10 .. 1e-12 on
+// by issue.  4,096 ellipses x 1,000 samples: 4.15 -> 0.45 ms; 10,000 planar
+// cubics x 1,024: 8.51 -> 0.82 ms.  Position errors at rtol 1e-10 .. 1e-12 on
 // ellipses, cubics and an uneven batch, rms and worst, are at or below the FP64
 // kernel's: the extra term of its stopping test makes it iterate further.
 template <int CODE, typename TAB>

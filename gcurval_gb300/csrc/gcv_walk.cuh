@@ -20,10 +20,11 @@
 // and hands intervals of more than 16 leaves to two more passes that walk them
 // again, one lane each; here an interval of L leaves takes as many rounds as
 // its deepest leaf has levels.  Against it: FP64 tables, 10,000 cubics 3.28 ->
-// 0.76 ms, 1,237 spatial curves (175k intervals) 3.16 -> 0.45 ms, 4,096 ellipses
-// 0.35 -> 0.08 ms, 64 ellipses 0.24 -> 0.05 ms; mixed, 301 uneven curves 1.41 ->
-// 0.41 ms, 50,000 spatial 2.68 -> 1.97 ms, 100,000 uneven with learned starts
-// 14.2 -> 12.6 ms.
+// 0.74 ms, 1,237 spatial curves (175k intervals) 3.16 -> 0.40 ms, 4,096 ellipses
+// 0.35 -> 0.07 ms, 64 ellipses 0.24 -> 0.05 ms; mixed, 301 uneven curves 1.41 ->
+// 0.24 ms, 50,000 spatial 2.68 -> 1.73 ms, 100,000 uneven with learned starts
+// 14.2 -> 11.0 ms (of these two, 1.97 and 12.3 before the panels' inner steps were
+// left unnormalised, gcv_ff.cuh).
 #pragma once
 
 #include "gcv_length_impl.cuh"
@@ -109,12 +110,12 @@ __device__ __noinline__ bool accept_fp64(const double* __restrict__ seg, unsigne
     return fabs(K - G) <= fmax(tol * hw, 50.0 * 2.220446049250313e-16 * fabs(K));
 }
 
-// Resident blocks per SM asked for, per curve code: 12 (at most 80 registers)
-// for degree 3-5 in 3D, 14 (72) for the others.  The walk of the uneven batch of
-// 100,000 curves took 13.0 ms at 10 / 12, 12.7 at 12 / 14, 14.0 at 8 / 8.
+// Resident blocks per SM asked for, per curve code: 14 (at most 72 registers)
+// for degree 3-5 in 3D, 16 (64) for the others.  The walk of the uneven batch of
+// 100,000 curves took 11.5 ms at 10 / 12, 11.15 at 12 / 14, 11.0 at 14 / 16.
 __host__ __device__ constexpr int walk_blocks(int code)
 {
-    return code > 0 && code_dim(code) == 3 && code_degree(code) >= 3 ? 12 : 14;
+    return code > 0 && code_dim(code) == 3 && code_degree(code) >= 3 ? 14 : 16;
 }
 
 // PREC 1: float-float table, K15 in float-float; PREC 2: FP64 table, the
