@@ -28,9 +28,16 @@ namespace gcv {
 // Newton on one leaf in float-float, in the local offset w = v - va in
 // [0, dv]: F(w) = S(va + w) - S(va) - rl with the partial integral taken by
 // 8-point Gauss over the shorter side of the leaf, bracketed by bisection.
-// Second-order steps and the stopping test of leaf_newton (gcv_kernels.cuh):
-// d = 2 F / (f0 + f1) with f1 the speed at the Newton point, stop when
-// dn^2 (|f'(w - dn) - f'(w)| / 3 + |f'|^2 |dn| / (4 f)) <= eps_s.
+// From F and the speed f0 at w, the Newton point w - dn; from the speeds there (f1)
+// and half way (fm), all in FP32, the length between by a rule of order seven
+// (Simpson's and the end-corrected trapezoidal rule combined, their difference E
+// the error's measure), what of F that leaves, and its own second-order step.
+// It stops when the estimated residual of that step is below eps_s.  With the
+// second-order step d = 2 F / (f0 + f1) alone, 9 % of the samples of 50,000 spatial
+// curves took another iteration, so most warps did; now 0.7 %: 10.2 -> 8.5 ms,
+// the uneven batch of 100,000 curves 11.3 -> 9.9, 4,096 ellipses 0.45 -> 0.41, and
+// positions are off by a fifth as much (7e-12 to 9e-12 rms at rtol 5e-9, from
+// 2.4e-11 to 3.5e-11).
 // Returns the final offset in units of 2^-60.
 // 8-point Gauss nodes (-x0..-x3, x0..x3) then weights w0..w3, float-float
 #define GCV_FFC(x) {split_const(x).hi, split_const(x).lo}
@@ -106,14 +113,32 @@ __device__ __forceinline__ ff gl8_ellipse(const ff* r, const EllipseMid& e, ff h
 }
 // speed to FP32 accuracy and q = f f' at the offset x from the midpoint (the
 // square of the speed in float-float: on a thin ellipse's tips it cancels)
-__device__ __forceinline__ float speed_slope_ellipse(const ff* r, const EllipseMid& e, ff x, float& q)
+// near: A, f^2, and the sine and cosine of the doubled angle there, for
+// speed_slope_near
+__device__ __forceinline__ float speed_slope_ellipse(const ff* r, const EllipseMid& e, ff x, float& q, float* near)
 {
     ff sd, cd;
     ff_sincospi_small(ff_scale(x, (float)ELLIPSE_PIECE_SCALE), sd, cd);
     const ff s = ff_fma(e.cm, sd, ff_mul(e.sm, cd));
     const float c = fmaf(e.cm.hi, cd.hi, -e.sm.hi * sd.hi);
     q = (float)(PI * ELLIPSE_PIECE_SCALE) * r[0].hi * s.hi * c;
-    return sqrtf(ff_fma(r[0], ff_mul(s, s), r[1]).hi);
+    near[0] = r[0].hi;
+    near[1] = ff_fma(r[0], ff_mul(s, s), r[1]).hi;
+    near[2] = 2.0f * s.hi * c;
+    near[3] = 1.0f - 2.0f * s.hi * s.hi;
+    return sqrtf(near[1]);
+}
+// the same at the distance x from there: A (sin^2(a + d) - sin^2 a) = A sin(2 a +
+// d) sin d, all in FP32
+__device__ __forceinline__ float speed_slope_near_ellipse(const float* near, float x, float& q)
+{
+    const float d = (float)(PI * ELLIPSE_PIECE_SCALE) * x, d2 = d * d;
+    const float sd = d * fmaf(d2, fmaf(d2, 1.0f / 120.0f, -1.0f / 6.0f), 1.0f);
+    const float vd = d2 * fmaf(d2, -1.0f / 24.0f, 0.5f);  // 1 - cos d
+    const float s1 = near[2] + (near[3] * sd - near[2] * vd);  // sin(2 a + d)
+    const float c1 = near[3] - (near[2] * sd + near[3] * vd);
+    q = (float)(0.5 * PI * ELLIPSE_PIECE_SCALE) * near[0] * (s1 + (c1 * sd - s1 * vd));
+    return sqrtf(fmaf(near[0] * s1, sd, near[1]));
 }
 
 // TAB: the coefficient table's element: float2 (float-float, mixed tables) or
@@ -170,35 +195,43 @@ __device__ __forceinline__ long long ff_leaf_newton(const TAB* __restrict__ seg,
         // +-h2 of the summed side that is w
         float q0, f0, near_w[MAX_COEF];
         if constexpr (C == 0)
-            f0 = speed_slope_ellipse(r, em, from_left ? h2 : ff_neg(h2), q0);
+            f0 = speed_slope_ellipse(r, em, from_left ? h2 : ff_neg(h2), q0, near_w);
         else if constexpr (PAIRS)
             f0 = EvalFF<C>::speed_slope_f(r, from_left ? h2 : ff_neg(h2), q0, near_w);
         else
             f0 = EvalFF<C>::speed_slope_f(r, ff_add(vaf, w), q0, near_w);
         const float r0 = rcp_approx(f0), dn = Fh * r0;
         float step = dn;
-        // the second-order step only from a Newton point inside the closed
+        // the higher-order step only from a Newton point inside the closed
         // bracket (a step below one FP32 ulp of w leaves w.hi - dn == w.hi,
         // which must still converge); a Newton point outside it would take
         // f1 from the polynomial extrapolated past the leaf
         const float wn = w.hi - dn;
         if (wn >= blo && wn <= bhi) {
-            // for the ellipse at the offset (w - dn) - (a0 + h2) from m2; for
-            // B-splines by the FP32 Taylor expansion at w (full evaluations
-            // of f1 were 7-9 % of the sampler's instructions)
-            float q1, f1;
-            if constexpr (C == 0)
-                f1 = speed_slope_ellipse(r, em, ff_add(ff_add_f(w, -dn), ff_neg(ff_add(a0, h2))), q1);
-            else
+            // the speeds at w - dn and half way in FP32 from what is known at w
+            float q1, qm, f1, fm;
+            if constexpr (C == 0) {
+                f1 = speed_slope_near_ellipse(near_w, -dn, q1);
+                fm = speed_slope_near_ellipse(near_w, -0.5f * dn, qm);
+            } else {
                 f1 = EvalFF<C>::speed_slope_near(near_w, -dn, q1);
-            const float d = 2.0f * Fh * rcp_approx(f0 + f1);
-            const float r1 = rcp_approx(f1), s0 = q0 * r0, s1 = q1 * r1;  // f'(w), f'(w - dn)
-            float res = dn * dn * (fabsf(s1 - s0) * (1.0f / 3.0f) + s1 * s1 * fabsf(dn) * 0.25f * r1);
+                fm = EvalFF<C>::speed_slope_near(near_w, -0.5f * dn, qm);
+            }
+            const float r1 = rcp_approx(f1), s1 = q1 * r1, ds = s1 - q0 * r0;  // f'(w - dn), less f'(w)
+            // the length between the two less dn f0: Simpson's rule, and the
+            // trapezoidal rule with end correction less that; the errors are as -1 to 4
+            const float simpson = dn * (1.0f / 6.0f) * (4.0f * (fm - f0) + (f1 - f0));
+            const float E = dn * (0.5f * (f1 - f0) + dn * (1.0f / 12.0f) * ds) - simpson;
+            const float rest = fmaf(-dn, f0, Fh) - simpson - 0.2f * E;
+            const float d0 = rest * r1, d = dn + fmaf(0.5f * s1 * r1, d0 * d0, d0);
+            float res = 0.2f * fabsf(E) + d0 * d0 * (0.5f * s1 * s1 * r1 * fabsf(d0) + (0.25f / 6.0f) * fabsf(ds));
             // at tight tolerances the FP32 rounding of the step itself counts:
-            // f0, f1 and the quotient are good to a few 2^-24 of F
-            res = fmaf(5e-7f, fabsf(Fh), res);
+            // the speeds and the quotients are good to a few 2^-24 of F (at most
+            // 1.3e-7 was seen; 5e-7 takes 10,000 cubics at rtol 1e-10 from
+            // 0.77 to 0.79 ms, 2.5e-7 to 0.75, but with errors as large as the FP64 kernel's)
+            res = fmaf(3.5e-7f, fabsf(Fh), res);
             const float wd = w.hi - d;
-            if (res <= eps_s && wd >= 0.0f && wd <= dv) {
+            if (res <= eps_s && fabsf(d0) <= 0.25f * fabsf(dn) && wd >= 0.0f && wd <= dv) {
                 last = d;  // converged with this step
                 break;
             }
@@ -242,8 +275,8 @@ static_assert(SAMPLE_FF_REGS * SAMPLE_THREADS_MAX <= 65536, "a block of SAMPLE_T
 // 2^-sexp, the binary exponent of its mean speed, so that curves of any
 // double magnitude fit FP32's exponent range.  The FP64 kernel was bound by
 // the FP64 pipe (91 % busy, one warp instruction per 64 issue slots); this one
-// by issue.  4,096 ellipses x 1,000 samples: 4.15 -> 0.45 ms; 10,000 planar
-// cubics x 1,024: 8.51 -> 0.82 ms.  Position errors at rtol 1e-10 .. 1e-12 on
+// by issue.  4,096 ellipses x 1,000 samples: 4.15 -> 0.41 ms; 10,000 planar
+// cubics x 1,024: 8.51 -> 0.77 ms.  Position errors at rtol 1e-10 .. 1e-12 on
 // ellipses, cubics and an uneven batch, rms and worst, are at or below the FP64
 // kernel's: the extra term of its stopping test makes it iterate further.
 template <int CODE, typename TAB>
