@@ -841,9 +841,9 @@ gcv_status ensure_table_buffers(gcv_ctx* c)
     if (c->deep_list.n == 0) CHECK(c->deep_list.reserve(ns / 16 + 1024));
     const size_t tiles = (ns + SCAN_TILE - 1) / SCAN_TILE;
     CHECK(c->scan_status.reserve(tiles));
-    CHECK(c->scan_flag.reserve(tiles));
-    CHECK(c->scan_hi.reserve(tiles));
-    CHECK(c->scan_lo.reserve(tiles));
+    CHECK(c->scan_flag.reserve(2 * tiles));
+    CHECK(c->scan_hi.reserve(2 * tiles));
+    CHECK(c->scan_lo.reserve(2 * tiles));
     return GCV_OK;
 }
 

@@ -60,7 +60,7 @@ struct Table {
     int64_t deep_cap;
     unsigned long long* ctr;
     int* scan_status;  // per scan tile: 0 none, 1 aggregate, 2 inclusive
-    int* scan_flag;
+    int* scan_flag;    // per scan tile its own sum, then (n_tiles further) the inclusive one
     double* scan_hi;
     double* scan_lo;
 };

@@ -247,15 +247,17 @@ static __global__ void __launch_bounds__(SCAN_THREADS) k_scan(Batch b, Table t, 
                     break;
                 }
                 __threadfence();
-                const SegVal pj{__ldcg(t.scan_flag + j), DD{__ldcg(t.scan_hi + j), __ldcg(t.scan_lo + j)}};
+                const int64_t e = st == 2 ? n_tiles + j : j;
+                const SegVal pj{__ldcg(t.scan_flag + e), DD{__ldcg(t.scan_hi + e), __ldcg(t.scan_lo + e)}};
                 pre = seg_combine(pj, pre);
                 if (st == 2 || pj.flag) done = true;
             }
         }
         const SegVal incl = seg_combine(pre, tile_agg);
-        t.scan_flag[tile] = 1;
-        t.scan_hi[tile] = incl.v.hi;
-        t.scan_lo[tile] = incl.v.lo;
+        // beside the tile's own sum, which a later tile may be reading
+        t.scan_flag[n_tiles + tile] = 1;
+        t.scan_hi[n_tiles + tile] = incl.v.hi;
+        t.scan_lo[n_tiles + tile] = incl.v.lo;
         __threadfence();
         atomicExch(t.scan_status + tile, 2);
         s_prefix = pre;
