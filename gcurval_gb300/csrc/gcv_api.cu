@@ -839,11 +839,28 @@ gcv_status ensure_table_buffers(gcv_ctx* c)
         CHECK(c->leaf_q.reserve((size_t)c->leaf_cap));
     }
     if (c->deep_list.n == 0) CHECK(c->deep_list.reserve(ns / 16 + 1024));
-    const size_t tiles = (ns + SCAN_TILE - 1) / SCAN_TILE;
-    CHECK(c->scan_status.reserve(tiles));
+    const size_t tiles = (size_t)scan_tiles((int64_t)ns);
+    CHECK(c->scan_status.reserve(tiles + 1));
     CHECK(c->scan_flag.reserve(2 * tiles));
     CHECK(c->scan_hi.reserve(2 * tiles));
     CHECK(c->scan_lo.reserve(2 * tiles));
+    return GCV_OK;
+}
+
+// prefix sums of the interval lengths and the curves' lengths, on the context's stream
+gcv_status launch_scan(gcv_ctx* c, const Batch& b)
+{
+    const int64_t tiles = scan_tiles(c->n_seg);
+    if (tiles > 0) {
+        CU(cudaMemsetAsync(c->scan_status.p, 0, (size_t)(tiles + 1) * sizeof(int), c->stream));
+        if (scan_items(c->n_seg) == 4)
+            k_scan<4><<<(unsigned)tiles, SCAN_THREADS, 0, c->stream>>>(b, table_view(c), tiles);
+        else
+            k_scan<32><<<(unsigned)tiles, SCAN_THREADS, 0, c->stream>>>(b, table_view(c), tiles);
+        CU(cudaGetLastError());
+    } else if (c->n_curve > 0) {
+        CU(cudaMemsetAsync(c->curve_len.p, 0, (size_t)c->n_curve * sizeof(double), c->stream));
+    }
     return GCV_OK;
 }
 
@@ -1217,19 +1234,8 @@ gcv_status build_table(gcv_ctx* c)
         break;
     }
     CU(cudaEventRecord(c->ev[2], c->stream));
-    const int64_t tiles = (c->n_seg + SCAN_TILE - 1) / SCAN_TILE;
-    if (tiles > 0) {
-        CU(cudaMemsetAsync(c->scan_status.p, 0, (size_t)tiles * sizeof(int), c->stream));
-        CU(cudaMemsetAsync(c->ctr.p + C_SCAN_TILE, 0, sizeof(unsigned long long), c->stream));
-        k_scan<<<(unsigned)tiles, SCAN_THREADS, 0, c->stream>>>(b, table_view(c), tiles);
-        CU(cudaGetLastError());
-        c->stats.n_launches++;
-    }
-    if (c->n_curve > 0) {
-        k_curve_len<<<(unsigned)std::min<int64_t>((c->n_curve + 255) / 256, 65535), 256, 0, c->stream>>>(b, table_view(c));
-        CU(cudaGetLastError());
-        c->stats.n_launches++;
-    }
+    CHECK(launch_scan(c, b));
+    if (c->n_seg > 0) c->stats.n_launches++;
     CU(cudaEventRecord(c->ev[3], c->stream));
     c->ev_table = true;
     if (learned) {
@@ -1518,16 +1524,7 @@ gcv_status enqueue_table_graph(gcv_ctx* c)
         CHECK(launch_length<2>(c, c->code, Q, c->stream));
     }
     CU(cudaEventRecordWithFlags(c->ev[2], c->stream, cudaEventRecordExternal));
-    const int64_t tiles = (c->n_seg + SCAN_TILE - 1) / SCAN_TILE;
-    if (tiles > 0) {
-        CU(cudaMemsetAsync(c->scan_status.p, 0, (size_t)tiles * sizeof(int), c->stream));
-        k_scan<<<(unsigned)tiles, SCAN_THREADS, 0, c->stream>>>(b, table_view(c), tiles);
-        CU(cudaGetLastError());
-    }
-    if (c->n_curve > 0) {
-        k_curve_len<<<(unsigned)std::min<int64_t>((c->n_curve + 255) / 256, 65535), 256, 0, c->stream>>>(b, table_view(c));
-        CU(cudaGetLastError());
-    }
+    CHECK(launch_scan(c, b));
     CU(cudaEventRecordWithFlags(c->ev[3], c->stream, cudaEventRecordExternal));
     return GCV_OK;
 }

@@ -32,7 +32,6 @@ enum Counter {
     C_NEWTON = 5,
     C_ERR = 6,        // error bits (ERR_*)
     C_NONFINITE = 7,
-    C_SCAN_TILE = 8,  // scan tile ticket
     C_DEEP_LEAVES = 9,  // leaves of the deep list's intervals (count pass)
     C_WORK_CODE = 16,   // work-queue heads of the per-code main-pass launches
     C_COUNT = 32
@@ -59,7 +58,7 @@ struct Table {
     int* deep_list;
     int64_t deep_cap;
     unsigned long long* ctr;
-    int* scan_status;  // per scan tile: 0 none, 1 aggregate, 2 inclusive
+    int* scan_status;  // per scan tile: 0 none, 1 aggregate, 2 inclusive; then the tile ticket
     int* scan_flag;    // per scan tile its own sum, then (n_tiles further) the inclusive one
     double* scan_hi;
     double* scan_lo;

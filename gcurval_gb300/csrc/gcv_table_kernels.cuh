@@ -134,8 +134,18 @@ static __global__ void k_deep_total(const int* __restrict__ list, int64_t n, con
 // replacing the reference's per-segment Brent-Kung scan plus one thread per
 // curve doing a sequential Kahan sum (gcurval/detail/cuda/kernel/generic.inl.cuh:52-137).
 constexpr int SCAN_THREADS = 256;
-constexpr int SCAN_ITEMS = 32;
-constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
+// Lengths per thread, by the number of knot intervals: 32 keep the look-back
+// short, 4 give small batches more blocks and short serial sums.  With 4 against
+// 32 (launch, clearing and curve lengths included): 130k intervals 17 against 31 us,
+// 610k 23 against 33, 1.0M 35 against 33 (65 against 49 as one curve), 7.0M 133
+// against 114, 47M 940 against 630.  The look-back takes 32 tiles at a time: thread by
+// thread a curve over a thousand tiles would wait for a thousand reads.
+constexpr int64_t SCAN_SHORT = 3 << 18;
+constexpr int scan_items(int64_t n_seg) { return n_seg <= SCAN_SHORT ? 4 : 32; }
+constexpr int64_t scan_tiles(int64_t n_seg)
+{
+    return (n_seg + SCAN_THREADS * scan_items(n_seg) - 1) / (SCAN_THREADS * scan_items(n_seg));
+}
 constexpr long long SCAN_SPIN_LIMIT = 1ll << 22;
 
 struct SegVal {
@@ -157,13 +167,17 @@ __device__ __forceinline__ SegVal shfl_up_sv(const SegVal& x, int d)
     return y;
 }
 
+// Also writes every curve's length (0 for curves without intervals).
+// scan_status: n_tiles states, then the tile ticket; all 0 at the launch.
+template <int SCAN_ITEMS>
 static __global__ void __launch_bounds__(SCAN_THREADS) k_scan(Batch b, Table t, int64_t n_tiles)
 {
+    constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
     __shared__ int s_tile;
     __shared__ SegVal s_warp[SCAN_THREADS / 32];
     __shared__ SegVal s_prefix;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) s_tile = (int)atomicAdd(t.ctr + C_SCAN_TILE, 1ull);
+    if (threadIdx.x == 0) s_tile = atomicAdd(t.scan_status + n_tiles, 1);
     __syncthreads();
     const int64_t tile = s_tile;
     if (tile >= n_tiles) return;
@@ -222,45 +236,60 @@ static __global__ void __launch_bounds__(SCAN_THREADS) k_scan(Batch b, Table t, 
     SegVal excl = lane == 0 ? SegVal{0, DD{0.0, 0.0}} : SegVal{ex_flag, DD{ex_v, 0.0}};
     if (warp > 0) excl = lane == 0 ? s_warp[warp - 1] : seg_combine(s_warp[warp - 1], excl);
 
-    // decoupled look-back by thread 0
-    if (threadIdx.x == 0) {
+    // decoupled look-back by warp 0, 32 tiles at a time
+    if (warp == 0) {
         const SegVal tile_agg = s_warp[SCAN_THREADS / 32 - 1];
-        SegVal pre{0, DD{0.0, 0.0}};
-        if (tile == 0) {
-            pre = SegVal{1, DD{0.0, 0.0}};
-        } else {
+        SegVal pre{tile == 0, DD{0.0, 0.0}};
+        if (tile > 0 && lane == 0) {
             t.scan_flag[tile] = tile_agg.flag;
             t.scan_hi[tile] = tile_agg.v.hi;
             t.scan_lo[tile] = tile_agg.v.lo;
             __threadfence();
             atomicExch(t.scan_status + tile, 1);
-            bool done = false;
-            for (int64_t j = tile - 1; j >= 0 && !done; --j) {
-                int st = 0;
-                for (long long it = 0; it < SCAN_SPIN_LIMIT; ++it) {
-                    st = atomicAdd(t.scan_status + j, 0);
-                    if (st) break;
-                    __nanosleep(64);
+        }
+        bool done = tile == 0;
+        for (int64_t top = tile - 1; top >= 0 && !done; top -= 32) {
+            // lane l looks at tile top - l; wanted are the tiles up to the first
+            // (`stop`) that knows its inclusive sum or has a curve's start
+            const int64_t j = top - lane;
+            SegVal pj{1, DD{0.0, 0.0}};
+            int st = j < 0 ? 2 : 0, stop = 0;
+            for (long long it = 0;; ++it) {
+                if (st == 0 && (st = atomicAdd(t.scan_status + j, 0)) != 0) {
+                    __threadfence();
+                    const int64_t e = st == 2 ? n_tiles + j : j;
+                    pj = SegVal{__ldcg(t.scan_flag + e), DD{__ldcg(t.scan_hi + e), __ldcg(t.scan_lo + e)}};
                 }
-                if (!st) {
-                    raise_err(t, ERR_SCAN_TIMEOUT);
+                const unsigned ready = __ballot_sync(0xffffffffu, st != 0);
+                const unsigned ends = __ballot_sync(0xffffffffu, st == 2 || (st == 1 && pj.flag));
+                stop = ends ? __ffs(ends) - 1 : 31;
+                done = ends != 0u;
+                if ((~ready & (0xffffffffu >> (31 - stop))) == 0u) break;
+                if (it == SCAN_SPIN_LIMIT) {
+                    if (lane == 0) raise_err(t, ERR_SCAN_TIMEOUT);
+                    done = true;
                     break;
                 }
-                __threadfence();
-                const int64_t e = st == 2 ? n_tiles + j : j;
-                const SegVal pj{__ldcg(t.scan_flag + e), DD{__ldcg(t.scan_hi + e), __ldcg(t.scan_lo + e)}};
-                pre = seg_combine(pj, pre);
-                if (st == 2 || pj.flag) done = true;
+                __nanosleep(64);
             }
+            const int flag = __shfl_sync(0xffffffffu, pj.flag, stop);
+            if (lane > stop || st == 0) pj.v = DD{0.0, 0.0};
+            if (stop > 0)
+                for (int o = 16; o > 0; o >>= 1)
+                    pj.v = dd_add(pj.v, DD{__shfl_xor_sync(0xffffffffu, pj.v.hi, o), __shfl_xor_sync(0xffffffffu, pj.v.lo, o)});
+            const DD sum{__shfl_sync(0xffffffffu, pj.v.hi, 0), __shfl_sync(0xffffffffu, pj.v.lo, 0)};
+            pre = SegVal{flag, dd_add(sum, pre.v)};
         }
-        const SegVal incl = seg_combine(pre, tile_agg);
-        // beside the tile's own sum, which a later tile may be reading
-        t.scan_flag[n_tiles + tile] = 1;
-        t.scan_hi[n_tiles + tile] = incl.v.hi;
-        t.scan_lo[n_tiles + tile] = incl.v.lo;
-        __threadfence();
-        atomicExch(t.scan_status + tile, 2);
-        s_prefix = pre;
+        if (lane == 0) {
+            // beside the tile's own sum, which a later tile may be reading
+            const SegVal incl = seg_combine(pre, tile_agg);
+            t.scan_flag[n_tiles + tile] = 1;
+            t.scan_hi[n_tiles + tile] = incl.v.hi;
+            t.scan_lo[n_tiles + tile] = incl.v.lo;
+            __threadfence();
+            atomicExch(t.scan_status + tile, 2);
+            s_prefix = pre;
+        }
     }
     __syncthreads();
     // items before the thread's first curve start add the exclusive prefix
@@ -269,16 +298,18 @@ static __global__ void __launch_bounds__(SCAN_THREADS) k_scan(Batch b, Table t, 
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k) {
         const int64_t s = base + k;
-        if (s < b.n_seg) t.seg_cum[s] = k < first_head ? pre.v.hi + (pre.v.lo + part[k]) : part[k];
-    }
-}
-
-static __global__ void k_curve_len(Batch b, Table t)
-{
-    for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < b.n_curve;
-         c += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t e = b.seg_off[c + 1];
-        t.curve_len[c] = e > b.seg_off[c] ? t.seg_cum[e - 1] : 0.0;
+        if (s >= b.n_seg) break;
+        const double cum = k < first_head ? pre.v.hi + (pre.v.lo + part[k]) : part[k];
+        t.seg_cum[s] = cum;
+        const bool end = s + 1 == b.n_seg;
+        const bool last = end || (k + 1 < SCAN_ITEMS ? heads >> (k + 1) & 1u : b.seg_curve[s + 1] != b.seg_curve[s]);
+        if (last) {
+            const int c = b.seg_curve[s], next = end ? (int)b.n_curve : b.seg_curve[s + 1];
+            t.curve_len[c] = cum;
+            for (int q = c + 1; q < next; ++q) t.curve_len[q] = 0.0;
+        }
+        if (s == 0)
+            for (int q = 0; q < b.seg_curve[0]; ++q) t.curve_len[q] = 0.0;
     }
 }
 

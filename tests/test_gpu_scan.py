@@ -1,5 +1,5 @@
 """Prefix sums of interval lengths and the curves' lengths they write: interval
-counts at the edges of tiles (1,024 intervals, 8,192 from 1,048,577 intervals on),
+counts at the edges of tiles (1,024 intervals, 8,192 from 786,433 intervals on),
 curves that span several tiles, runs of curves within one tile, and curves without
 intervals (a single control point) before, between and after others.
 
@@ -36,8 +36,8 @@ CASES = {
     "tiles of single intervals": [1] * 2049,
     "curves over several tiles": [5000, 1, 1, 3000, 7],
     "heads at every place": list(range(1, 70)),
-    "most for short tiles": [1 << 20],
-    "one more": [(1 << 20) - 5, 3, 3],
+    "most for short tiles": [3 << 18],
+    "one more": [(3 << 18) - 5, 3, 3],
     "without intervals": [0, 0, 3, 0, 2000, 0, 0, 0, 1, 0],
     "none with intervals": [0, 0, 0],
     "long tiles": [8192 * 3, 8191, 1, 1] + [777] * 1400,
