@@ -48,6 +48,13 @@ def _is_device(a) -> bool:
     return hasattr(a, "is_cuda") and bool(a.is_cuda)
 
 
+def _finish_current_stream(a):
+    """Waits for the work queued on the torch stream that is current on a's device."""
+    import torch
+
+    torch.cuda.current_stream(a.device).synchronize()
+
+
 def _is_f32(a) -> bool:
     """A float32 numpy array or torch tensor."""
     dt = getattr(a, "dtype", None)
@@ -303,24 +310,41 @@ class ArclengthCalculateGpu:
         pos = sample_position if in_dev else np.ascontiguousarray(sample_position, self.dtype)
         if _is_f32(pos) != self.f32 or _is_f32(out) != self.f32:
             raise ValueError(f"positions and output must be {np.dtype(self.dtype).name} for this context")
-        total = self._check_counts(n, int(pos.shape[0]))
+        n_pos = int(pos.shape[0])
         width = 1 if what == GCV_RETURN_US else self.point_dim
         n_out = int(out.numel()) if hasattr(out, "numel") else int(out.size)
-        if n_out < total * width:
-            raise ValueError(f"output holds {n_out} values, {total * width} needed")
-        into = self._lib.gcv_arclength_reverse_into_f32 if self.f32 else self._lib.gcv_arclength_reverse_into
-        check(into(self._h, _ptr(n), _ptr(pos), int(bool(is_relative)), GCV_DEVICE if in_dev else GCV_HOST,
-                   int(what), _ptr(out), GCV_DEVICE if _is_device(out) else GCV_HOST))
+        total = ctypes.c_int64(n_pos)
+        if in_dev and n_out >= n_pos * width and str(n.dtype) == "torch.int32" and n.is_contiguous():
+            # the library sums the counts as it stages them (a sum on the device
+            # and its transfer cost 30 us); what it waited for on the
+            # caller's stream is waited for here
+            self._check_shape(n)
+            _finish_current_stream(n)
+        else:
+            total.value = self._check_counts(n, n_pos)
+        st = 0
+        if n_out >= total.value * width:
+            st = self._lib.gcv_arclength_reverse_sized(
+                self._h, _ptr(n), _ptr(pos), n_pos, int(bool(is_relative)), GCV_DEVICE if in_dev else GCV_HOST, int(what),
+                _ptr(out), n_out, GCV_DEVICE if _is_device(out) else GCV_HOST, int(self.f32), ctypes.byref(total))
+        if total.value != n_pos:
+            raise ValueError(f"sample counts add up to {total.value}, {n_pos} positions given")
+        if n_out < total.value * width:
+            raise ValueError(f"output holds {n_out} values, {total.value * width} needed")
+        check(st)
         return out
 
     def clearArclength(self):
         check(self._lib.gcv_clear_arclength(self._h))
 
+    def _check_shape(self, n):
+        if tuple(n.shape) != (self.n_curve,):
+            raise ValueError(f"{n.shape[0] if len(n.shape) else 0} sample counts for {self.n_curve} curves")
+
     def _check_counts(self, n, n_positions: int) -> int:
         """The C ABI reads n_curve counts and their sum of positions through raw
         pointers, as the reference does; check the sizes before handing them over."""
-        if tuple(n.shape) != (self.n_curve,):
-            raise ValueError(f"{n.shape[0] if len(n.shape) else 0} sample counts for {self.n_curve} curves")
+        self._check_shape(n)
         total = int(n.sum())
         if total != n_positions:
             raise ValueError(f"sample counts add up to {total}, {n_positions} positions given")

@@ -117,6 +117,8 @@ _SIGS = {
                                                _P, ctypes.c_int, ctypes.POINTER(Options)]),
     "gcv_get_all_curve_arclengths_f32": (ctypes.c_int, [_P, _P, ctypes.c_int]),
     "gcv_get_arclength_f32": (ctypes.c_int, [_P, ctypes.c_int, ctypes.POINTER(ctypes.c_float)]),
+    "gcv_arclength_reverse_sized": (ctypes.c_int, [_P, _P, _P, ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_int, _P,
+                                                   ctypes.c_int64, ctypes.c_int, ctypes.c_int, _P]),
     "gcv_arclength_reverse_into_f32": (ctypes.c_int, [_P, _P, _P, ctypes.c_int, ctypes.c_int, ctypes.c_int, _P,
                                                       ctypes.c_int]),
     "gcv_arclength_reverse_f32": (ctypes.c_int, [_P, _P, _P, ctypes.c_int, ctypes.c_int, ctypes.c_int,

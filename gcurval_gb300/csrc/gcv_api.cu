@@ -1597,11 +1597,24 @@ void drop_graph(gcv_ctx* c)
     c->graph = nullptr;
 }
 
-gcv_status stage_counts(gcv_ctx* c, const int* n_ptrs, int in_where, int64_t* total)
+// what a caller's positions and output buffers hold; `total` receives the sum of the counts
+struct SampleSizes {
+    int64_t positions, outputs;
+    int width;
+    int64_t* total;
+};
+gcv_status stage_counts(gcv_ctx* c, const int* n_ptrs, int in_where, int64_t* total, const SampleSizes* sizes)
 {
     const int64_t n = c->n_curve;
     std::vector<int> cnt;
     CHECK(to_host(n_ptrs, (size_t)n, in_where, cnt));
+    if (sizes) {
+        int64_t sum = 0;
+        for (const int x : cnt) sum += x;
+        *sizes->total = sum;
+        if (sum != sizes->positions) return fail(GCV_ERR_INVALID, "sample counts do not add up to the positions given");
+        if (sizes->outputs < sum * sizes->width) return fail(GCV_ERR_INVALID, "output too small");
+    }
     std::vector<int64_t>& off = c->h_sample_off;
     off.assign((size_t)n + 1, 0);
     for (int64_t i = 0; i < n; ++i) {
@@ -1909,8 +1922,8 @@ gcv_status gcv_clear_arclength(gcv_ctx* ctx)
     return GCV_OK;
 }
 
-gcv_status gcv_arclength_reverse_into(gcv_ctx* ctx, const int* n_ptrs_for_curves, const double* sample_position,
-                                      int is_relative, int in_where, int what, double* out, int out_where)
+static gcv_status reverse_into(gcv_ctx* ctx, const int* n_ptrs_for_curves, const double* sample_position, int is_relative,
+                               int in_where, int what, double* out, int out_where, const SampleSizes* sizes)
 {
     if (!ctx) return fail(GCV_ERR_INVALID, "ctx is NULL");
     if (!ctx->table_ready) return fail(GCV_ERR_STATE, "createArclengthTable has not run");
@@ -1919,7 +1932,7 @@ gcv_status gcv_arclength_reverse_into(gcv_ctx* ctx, const int* n_ptrs_for_curves
     if (out_where != GCV_HOST && out_where != GCV_DEVICE) return fail(GCV_ERR_INVALID, "bad out_where");
     if (ctx->n_curve > 0 && !n_ptrs_for_curves) return fail(GCV_ERR_INVALID, "n_ptrs_for_curves is NULL");
     int64_t total = 0;
-    CHECK(stage_counts(ctx, n_ptrs_for_curves, in_where, &total));
+    CHECK(stage_counts(ctx, n_ptrs_for_curves, in_where, &total, sizes));
     if (total == 0) return GCV_OK;
     if (!sample_position || !out) return fail(GCV_ERR_INVALID, "NULL positions or output");
     // Page-locked host buffers are read and written by the sampling kernels
@@ -1952,6 +1965,12 @@ gcv_status gcv_arclength_reverse_into(gcv_ctx* ctx, const int* n_ptrs_for_curves
     CHECK(run_sampling(ctx, ctx->sample_off.p, d_pos, total, is_relative ? 1 : 0, what, d_out, h_pos, h_out));
     if (out_where == GCV_HOST) CU(cudaStreamSynchronize(ctx->stream));
     return GCV_OK;
+}
+
+gcv_status gcv_arclength_reverse_into(gcv_ctx* ctx, const int* n_ptrs_for_curves, const double* sample_position,
+                                      int is_relative, int in_where, int what, double* out, int out_where)
+{
+    return reverse_into(ctx, n_ptrs_for_curves, sample_position, is_relative, in_where, what, out, out_where, nullptr);
 }
 
 gcv_status gcv_arclength_reverse(gcv_ctx* ctx, const int* n_ptrs_for_curves, const double* sample_position,
@@ -2104,8 +2123,9 @@ gcv_status gcv_get_arclength_f32(gcv_ctx* ctx, int cid, float* out)
     return GCV_OK;
 }
 
-gcv_status gcv_arclength_reverse_into_f32(gcv_ctx* ctx, const int* n_ptrs_for_curves, const float* sample_position,
-                                          int is_relative, int in_where, int what, float* out, int out_where)
+static gcv_status reverse_into_f32(gcv_ctx* ctx, const int* n_ptrs_for_curves, const float* sample_position,
+                                   int is_relative, int in_where, int what, float* out, int out_where,
+                                   const SampleSizes* sizes)
 {
     if (!ctx) return fail(GCV_ERR_INVALID, "ctx is NULL");
     if (!ctx->table_ready) return fail(GCV_ERR_STATE, "createArclengthTable has not run");
@@ -2114,7 +2134,7 @@ gcv_status gcv_arclength_reverse_into_f32(gcv_ctx* ctx, const int* n_ptrs_for_cu
     if (out_where != GCV_HOST && out_where != GCV_DEVICE) return fail(GCV_ERR_INVALID, "bad out_where");
     if (ctx->n_curve > 0 && !n_ptrs_for_curves) return fail(GCV_ERR_INVALID, "n_ptrs_for_curves is NULL");
     int64_t total = 0;
-    CHECK(stage_counts(ctx, n_ptrs_for_curves, in_where, &total));
+    CHECK(stage_counts(ctx, n_ptrs_for_curves, in_where, &total, sizes));
     if (total == 0) return GCV_OK;
     if (!sample_position || !out) return fail(GCV_ERR_INVALID, "NULL positions or output");
     const int width = what == GCV_RETURN_US ? 1 : ctx->point_dim;
@@ -2141,6 +2161,25 @@ gcv_status gcv_arclength_reverse_into_f32(gcv_ctx* ctx, const int* n_ptrs_for_cu
         CU(cudaStreamSynchronize(ctx->stream));
     }
     return GCV_OK;
+}
+
+gcv_status gcv_arclength_reverse_into_f32(gcv_ctx* ctx, const int* n_ptrs_for_curves, const float* sample_position,
+                                          int is_relative, int in_where, int what, float* out, int out_where)
+{
+    return reverse_into_f32(ctx, n_ptrs_for_curves, sample_position, is_relative, in_where, what, out, out_where,
+                            nullptr);
+}
+
+gcv_status gcv_arclength_reverse_sized(gcv_ctx* ctx, const int* n_ptrs_for_curves, const void* sample_position,
+                                       int64_t n_positions, int is_relative, int in_where, int what, void* out,
+                                       int64_t n_out, int out_where, int f32, int64_t* total)
+{
+    if (!ctx || !total) return fail(GCV_ERR_INVALID, "NULL argument");
+    const SampleSizes sizes{n_positions, n_out, what == GCV_RETURN_US ? 1 : ctx->point_dim, total};
+    return f32 ? reverse_into_f32(ctx, n_ptrs_for_curves, (const float*)sample_position, is_relative, in_where, what,
+                                  (float*)out, out_where, &sizes)
+               : reverse_into(ctx, n_ptrs_for_curves, (const double*)sample_position, is_relative, in_where, what,
+                              (double*)out, out_where, &sizes);
 }
 
 gcv_status gcv_arclength_reverse_f32(gcv_ctx* ctx, const int* n_ptrs_for_curves, const float* sample_position,
@@ -2392,7 +2431,7 @@ gcv_status gcv_step_graph(gcv_ctx* ctx, const int* d_counts, const double* d_pos
         drop_graph(c);
         CHECK(build_table(c));
         int64_t total = 0;
-        CHECK(stage_counts(c, d_counts, GCV_DEVICE, &total));
+        CHECK(stage_counts(c, d_counts, GCV_DEVICE, &total, nullptr));
         CHECK(run_sampling(c, c->sample_off.p, const_cast<double*>(d_pos), total, is_relative, what, d_out));
         CU(cudaStreamSynchronize(c->stream));
         c->h_len_valid = false;

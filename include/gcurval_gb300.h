@@ -301,6 +301,14 @@ gcv_status gcv_get_all_curve_arclengths_f32(gcv_ctx* ctx, float* out, int where)
 gcv_status gcv_get_arclength_f32(gcv_ctx* ctx, int cid, float* out);
 gcv_status gcv_arclength_reverse_into_f32(gcv_ctx* ctx, const int* n_ptrs_for_curves, const float* sample_position,
                                           int is_relative, int in_where, int what, float* out, int out_where);
+/* gcv_arclength_reverse_into (f32 = 0) or its FP32 form (f32 = 1) with the
+ * buffers' sizes: n_positions positions and room for n_out values.  *total
+ * receives the sum of the counts.  GCV_ERR_INVALID, with nothing launched, when
+ * it is not n_positions or when the output does not hold the result: one
+ * reading of device counts checks and uses them. */
+gcv_status gcv_arclength_reverse_sized(gcv_ctx* ctx, const int* n_ptrs_for_curves, const void* sample_position,
+                                       int64_t n_positions, int is_relative, int in_where, int what, void* out,
+                                       int64_t n_out, int out_where, int f32, int64_t* total);
 gcv_status gcv_arclength_reverse_f32(gcv_ctx* ctx, const int* n_ptrs_for_curves, const float* sample_position,
                                      int is_relative, int where, int what, gcv_result_f32* result);
 gcv_status gcv_free_result_f32(gcv_result_f32* result);
