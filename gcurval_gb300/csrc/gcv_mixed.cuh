@@ -28,16 +28,19 @@ namespace gcv {
 // Newton on one leaf in float-float, in the local offset w = v - va in
 // [0, dv]: F(w) = S(va + w) - S(va) - rl with the partial integral taken by
 // 8-point Gauss over the shorter side of the leaf, bracketed by bisection.
-// From F and the speed f0 at w, the Newton point w - dn; from the speeds there (f1)
-// and half way (fm), all in FP32, the length between by a rule of order seven
-// (Simpson's and the end-corrected trapezoidal rule combined, their difference E
-// the error's measure), what of F that leaves, and its own second-order step.
-// It stops when the estimated residual of that step is below eps_s.  With the
-// second-order step d = 2 F / (f0 + f1) alone, 9 % of the samples of 50,000 spatial
-// curves took another iteration, so most warps did; now 0.7 %: 10.2 -> 8.5 ms,
-// the uneven batch of 100,000 curves 11.3 -> 9.9, 4,096 ellipses 0.45 -> 0.41, and
-// positions are off by a fifth as much (7e-12 to 9e-12 rms at rtol 5e-9, from
-// 2.4e-11 to 3.5e-11).
+// From F and the speed f0 at w, the Newton point w - dn; with the speed f1 there
+// the second-order step d = 2 F / (f0 + f1), and the stopping test of leaf_newton
+// (gcv_kernels.cuh): dn^2 (|f'(w - dn) - f'(w)| / 3 + |f'|^2 |dn| / (4 f)) <= eps_s.
+// Where that is not enough, the speed half way (fm, in FP32 like f1) gives the
+// length of the step by a rule of order seven (Simpson's and the end-corrected
+// trapezoidal rule combined, their difference E the error's measure), and what of
+// F that leaves its own second-order step: taken when its residual is below eps_t,
+// which stands for what another iteration would leave.  Without it 9 % of the
+// samples of 50,000 spatial curves took another iteration, so most warps did; now
+// 4 %: 10.2 -> 9.0 ms, the uneven batch of 100,000 curves 11.3 -> 10.3, 4,096
+// ellipses 0.45 -> 0.42, 10,000 cubics at rtol 1e-10 0.82 -> 0.80.  (Taken wherever
+// its residual is below eps_s itself: 8.5, 9.9, 0.41, 0.77 ms, but with samples off by
+// eps_s where an iteration left rounding.)
 // Returns the final offset in units of 2^-60.
 // 8-point Gauss nodes (-x0..-x3, x0..x3) then weights w0..w3, float-float
 #define GCV_FFC(x) {split_const(x).hi, split_const(x).lo}
@@ -145,7 +148,7 @@ __device__ __forceinline__ float speed_slope_near_ellipse(const float* near, flo
 // double (FP64 tables; lengths then come scaled by 2^-sexp, see k_sample_ff).
 template <int C, typename TAB>
 __device__ __forceinline__ long long ff_leaf_newton(const TAB* __restrict__ seg, int sexp, ff vaf, float dv, ff rl, ff dS,
-                                                 float dvg, float eps_s, unsigned long long& newton)
+                                                 float dvg, float eps_s, float eps_t, unsigned long long& newton)
 {
     constexpr bool FROM64 = std::is_same<TAB, double>::value;
     constexpr bool PAIRS = sample_node_pairs(C);
@@ -208,30 +211,42 @@ __device__ __forceinline__ long long ff_leaf_newton(const TAB* __restrict__ seg,
         // f1 from the polynomial extrapolated past the leaf
         const float wn = w.hi - dn;
         if (wn >= blo && wn <= bhi) {
-            // the speeds at w - dn and half way in FP32 from what is known at w
-            float q1, qm, f1, fm;
-            if constexpr (C == 0) {
+            // the speed at w - dn in FP32 from what is known at w
+            float q1, f1;
+            if constexpr (C == 0)
                 f1 = speed_slope_near_ellipse(near_w, -dn, q1);
-                fm = speed_slope_near_ellipse(near_w, -0.5f * dn, qm);
-            } else {
+            else
                 f1 = EvalFF<C>::speed_slope_near(near_w, -dn, q1);
-                fm = EvalFF<C>::speed_slope_near(near_w, -0.5f * dn, qm);
-            }
+            float d = 2.0f * Fh * rcp_approx(f0 + f1);
             const float r1 = rcp_approx(f1), s1 = q1 * r1, ds = s1 - q0 * r0;  // f'(w - dn), less f'(w)
-            // the length between the two less dn f0: Simpson's rule, and the
-            // trapezoidal rule with end correction less that; the errors are as -1 to 4
-            const float simpson = dn * (1.0f / 6.0f) * (4.0f * (fm - f0) + (f1 - f0));
-            const float E = dn * (0.5f * (f1 - f0) + dn * (1.0f / 12.0f) * ds) - simpson;
-            const float rest = fmaf(-dn, f0, Fh) - simpson - 0.2f * E;
-            const float d0 = rest * r1, d = dn + fmaf(0.5f * s1 * r1, d0 * d0, d0);
-            float res = 0.2f * fabsf(E) + d0 * d0 * (0.5f * s1 * s1 * r1 * fabsf(d0) + (0.25f / 6.0f) * fabsf(ds));
+            float res = dn * dn * (fabsf(ds) * (1.0f / 3.0f) + s1 * s1 * fabsf(dn) * 0.25f * r1);
             // at tight tolerances the FP32 rounding of the step itself counts:
             // the speeds and the quotients are good to a few 2^-24 of F (at most
-            // 1.3e-7 was seen; 5e-7 takes 10,000 cubics at rtol 1e-10 from
-            // 0.77 to 0.79 ms, 2.5e-7 to 0.75, but with errors as large as the FP64 kernel's)
-            res = fmaf(3.5e-7f, fabsf(Fh), res);
+            // 1.3e-7 was seen; with 3.5e-7 the errors at rtol 1e-11 came out a
+            // tenth above the FP64 kernel's)
+            const float noise = 5e-7f * fabsf(Fh);
+            bool ok = (eps_t < eps_s ? res : res + noise) <= eps_s;
+            // only where the speed changes little over the step: past a cusp E can be
+            // small by accident
+            if (!ok && fabsf(f1 - f0) + fabsf(ds * dn) <= 0.3f * f0) {
+                // the speed half way; the length between w - dn and w less dn f0
+                // by Simpson's rule, and the trapezoidal rule with end correction
+                // less that; their errors are as -1 to 4
+                float qm, fm;
+                if constexpr (C == 0)
+                    fm = speed_slope_near_ellipse(near_w, -0.5f * dn, qm);
+                else
+                    fm = EvalFF<C>::speed_slope_near(near_w, -0.5f * dn, qm);
+                const float simpson = dn * (1.0f / 6.0f) * (4.0f * (fm - f0) + (f1 - f0));
+                const float E = dn * (0.5f * (f1 - f0) + dn * (1.0f / 12.0f) * ds) - simpson;
+                const float rest = fmaf(-dn, f0, Fh) - simpson - 0.2f * E;
+                const float d0 = rest * r1;
+                d = dn + fmaf(0.5f * s1 * r1, d0 * d0, d0);
+                res = 0.2f * fabsf(E) + d0 * d0 * (0.5f * s1 * s1 * r1 * fabsf(d0) + (0.25f / 6.0f) * fabsf(ds));
+                ok = res + noise <= eps_t && fabsf(d0) <= 0.25f * fabsf(dn);
+            }
             const float wd = w.hi - d;
-            if (res <= eps_s && fabsf(d0) <= 0.25f * fabsf(dn) && wd >= 0.0f && wd <= dv) {
+            if (ok && wd >= 0.0f && wd <= dv) {
                 last = d;  // converged with this step
                 break;
             }
@@ -263,6 +278,8 @@ __device__ __forceinline__ long long ff_leaf_newton(const TAB* __restrict__ seg,
 // were worth 0.47 ms of it.
 constexpr int SAMPLE_FF_REGS = 64;
 static_assert(SAMPLE_FF_REGS * SAMPLE_THREADS_MAX <= 65536, "a block of SAMPLE_THREADS_MAX must fit one SM");
+// residual, of the curve's length, that counts as an iterate's (at least eps_frac)
+constexpr float SAMPLE_TIGHT = 1e-10f;
 //
 // TAB = double runs the same kernel on an FP64 table (GCV_PLAIN_FP64 at
 // tolerances down to PLAIN_SPLIT_RTOL).  What it computes in float-float is
@@ -275,8 +292,8 @@ static_assert(SAMPLE_FF_REGS * SAMPLE_THREADS_MAX <= 65536, "a block of SAMPLE_T
 // 2^-sexp, the binary exponent of its mean speed, so that curves of any
 // double magnitude fit FP32's exponent range.  The FP64 kernel was bound by
 // the FP64 pipe (91 % busy, one warp instruction per 64 issue slots); this one
-// by issue.  4,096 ellipses x 1,000 samples: 4.15 -> 0.41 ms; 10,000 planar
-// cubics x 1,024: 8.51 -> 0.77 ms.  Position errors at rtol 1e-10 .. 1e-12 on
+// by issue.  4,096 ellipses x 1,000 samples: 4.15 -> 0.42 ms; 10,000 planar
+// cubics x 1,024: 8.51 -> 0.80 ms.  Position errors at rtol 1e-10 .. 1e-12 on
 // ellipses, cubics and an uneven batch, rms and worst, are at or below the FP64
 // kernel's: the extra term of its stopping test makes it iterate further.
 template <int CODE, typename TAB>
@@ -296,6 +313,7 @@ __global__ void __maxnreg__(SAMPLE_FF_REGS) k_sample_ff(SampleParams P, const TA
     // nine launches: 750 us and 185 us)
     const int64_t per = (i1 - i0) / P.min_runs & ~(int64_t)31;
     const int run_len = per >= SAMPLE_RUN ? SAMPLE_RUN : (per < 32 ? 32 : (int)per);
+    const float tight = fminf(1.0f, SAMPLE_TIGHT / P.eps_frac);
     CurveHint hint;
     const int lane = threadIdx.x & 31;
     const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -386,7 +404,7 @@ __global__ void __maxnreg__(SAMPLE_FF_REGS) k_sample_ff(SampleParams P, const TA
                 }
                 const TAB* seg = coef + b.coef_off[c] + (int64_t)(s - s0) * code_stride(CODE);
                 const float eps_s = P.eps_frac * (FROM64 ? ff_from_double_scaled(L, sexp).hi : f32_of_f64_trunc(L));
-                const long long w = ff_leaf_newton<CODE>(seg, sexp, vaf, dv, rl, dS, dvg, eps_s, newton);
+                const long long w = ff_leaf_newton<CODE>(seg, sexp, vaf, dv, rl, dS, dvg, eps_s, tight * eps_s, newton);
                 v = vfix + (w < 0 ? 0 : w > dfix ? dfix : w);
             }
         }
