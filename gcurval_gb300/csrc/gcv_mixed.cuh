@@ -37,7 +37,7 @@ namespace gcv {
 // F that leaves its own second-order step: taken when its residual is below eps_t,
 // which stands for what another iteration would leave.  Without it 9 % of the
 // samples of 50,000 spatial curves took another iteration, so most warps did; now
-// 4 %: 10.2 -> 9.0 ms, the uneven batch of 100,000 curves 11.3 -> 10.3, 4,096
+// 6 %: 10.2 -> 9.58 ms, the uneven batch of 100,000 curves 11.3 -> 10.6, 4,096
 // ellipses 0.45 -> 0.42, 10,000 cubics at rtol 1e-10 0.82 -> 0.80.  (Taken wherever
 // its residual is below eps_s itself: 8.5, 9.9, 0.41, 0.77 ms, but with samples off by
 // eps_s where an iteration left rounding.)
@@ -279,7 +279,7 @@ __device__ __forceinline__ long long ff_leaf_newton(const TAB* __restrict__ seg,
 constexpr int SAMPLE_FF_REGS = 64;
 static_assert(SAMPLE_FF_REGS * SAMPLE_THREADS_MAX <= 65536, "a block of SAMPLE_THREADS_MAX must fit one SM");
 // residual, of the curve's length, that counts as an iterate's (at least eps_frac)
-constexpr float SAMPLE_TIGHT = 1e-10f;
+constexpr float SAMPLE_TIGHT = 4e-11f;
 //
 // TAB = double runs the same kernel on an FP64 table (GCV_PLAIN_FP64 at
 // tolerances down to PLAIN_SPLIT_RTOL).  What it computes in float-float is
