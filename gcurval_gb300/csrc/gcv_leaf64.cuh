@@ -15,6 +15,13 @@
 //     instructions per node, the sum good to FP64 rounding.
 // A planar cubic's panel takes about 90 FP64 instructions, against about 300 of
 // panel_k15; an ellipse's about 145 against about 650.
+//
+// The polynomial q is good to a rounding of its largest coefficients, so where the
+// speed at a node is a small part of the panel's largest (LEAF_LOW) its root is
+// not: next to a zero of even order, whose speeds are smooth and whose panel is
+// accepted whole, lengths were off by up to 4e-10.  Such panels are summed once more
+// by leaf_k15_nodes, from the speeds' components (none of the 44,000 leaves of random
+// planar and spatial cubics and uneven curves).
 #pragma once
 
 #include "gcv_ff_eval.cuh"
@@ -68,23 +75,34 @@ __device__ __forceinline__ double kronrod_root(double x, float wf, float& corr)
     corr = live ? fmaf(wf * hy, rf, corr) : corr;
     return S;
 }
-// the Kronrod pair i with squared speeds x0, x1
-__device__ __forceinline__ void kronrod_pair(double x0, double x1, int i, double& acc, float& corr)
+// the Kronrod pair i with squared speeds x0, x1; low: the smallest one's leading bits
+__device__ __forceinline__ void kronrod_pair(double x0, double x1, int i, double& acc, float& corr, int& low)
 {
     const float wf = c_gk_wf[i];
+    low = min(low, min(__double2hiint(x0), __double2hiint(x1)));
     const double S0 = kronrod_root(x0, wf, corr), S1 = kronrod_root(x1, wf, corr);
     acc = fma(c_gk_w[i], S0 + S1, acc);
 }
 
+// A squared speed below 2^-LEAF_LOW of q's largest coefficient (or below
+// kronrod_root's range) is taken from its components.  Above it q's rounding
+// moves a speed by at most 2^(LEAF_LOW / 2 - 1) units of q's, and a node's weight is a
+// fifth of the panel or less: a few units of the panel's sum.
+constexpr int LEAF_LOW = 8;
+
 // seg: the interval's FP64 table entry; sexp: the binary exponent that brings
-// its speeds near 1; panel (k, depth).  The integral over the panel of v.
+// its speeds near 1; panel (k, depth).  The integral over the panel of v;
+// `again`: leaf_k15_nodes has to give it.
 template <int CODE>
-__device__ __forceinline__ double leaf_k15(const double* __restrict__ seg, int sexp, unsigned long long k, int depth)
+__device__ __forceinline__ double leaf_k15(const double* __restrict__ seg, int sexp, unsigned long long k, int depth,
+                                           bool& again)
 {
     const double hw = pow2_neg(depth);
     const double mid = fma(__ull2double_rn(k), 2.0 * hw, -1.0) + hw;
     double acc = 0.0, centre;
     float corr = 0.0f;
+    int low = 0x7FFFFFFF;
+    again = false;
     if constexpr (CODE == 0) {
         const double B = scale_exp(seg[1], 2 * sexp);
         double A = scale_exp(seg[0], 2 * sexp), sm, cm;
@@ -98,7 +116,7 @@ __device__ __forceinline__ double leaf_k15(const double* __restrict__ seg, int s
         for (int i = 0; i < 7; ++i) {
             const double sd = __ldg(&tab[i][0]), p = fma(-sm, __ldg(&tab[i][1]), sm);
             const double up = fma(cm, sd, p), dn = fma(-cm, sd, p);
-            kronrod_pair(fma(A * up, up, B), fma(A * dn, dn, B), i, acc, corr);
+            kronrod_pair(fma(A * up, up, B), fma(A * dn, dn, B), i, acc, corr, low);
         }
         centre = fma(A * sm, sm, B);
     } else {
@@ -148,12 +166,42 @@ __device__ __forceinline__ double leaf_k15(const double* __restrict__ seg, int s
 #pragma unroll
                 for (int m = 2 * N - 3; m >= 1; m -= 2) O = fma(O, z, q[m]);
             }
-            kronrod_pair(N > 0 ? fma(x, O, E) : E, N > 0 ? fma(-x, O, E) : E, i, acc, corr);
+            kronrod_pair(N > 0 ? fma(x, O, E) : E, N > 0 ? fma(-x, O, E) : E, i, acc, corr, low);
         }
         centre = q[0];
+        int top = 0;
+#pragma unroll
+        for (int m = 0; m <= 2 * N; ++m) top = max(top, __double2hiint(q[m]) & 0x7FFFFFFF);
+        low = min(low, __double2hiint(centre));
+        again = top != 0 && low < max(top - (LEAF_LOW << 20), (1023 - 70) << 20);
     }
     acc = fma(gk_wk(7), kronrod_root(centre, (float)gk_wk(7), corr), acc);
     return scale_exp((acc + (double)corr) * hw, -sexp);
+}
+
+// The same panel of a B-spline piece by 16 lanes, one node each (the centre twice,
+// with half its weight), every speed from its components in FP64 throughout: its
+// error is a rounding of the interval's largest speed.  Every lane of the warp takes
+// part; the result is the same in the 16.
+template <int CODE>
+__device__ __noinline__ double leaf_k15_nodes(const double* __restrict__ seg, int sexp, unsigned long long k, int depth)
+{
+    constexpr int P = code_degree(CODE), D = code_dim(CODE);
+    const int i = threadIdx.x & 7;
+    const double hw = pow2_neg(depth), x = i < 7 ? c_gk_x[i] : 0.0, w = i < 7 ? c_gk_w[i] : 0.5 * gk_wk(7);
+    const double v = fma(threadIdx.x & 8 ? hw : -hw, x, fma(__ull2double_rn(k), 2.0 * hw, -1.0) + hw);
+    double s = 0.0;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+        double p = scale_exp(seg[P * D + d], sexp) * double(P);
+#pragma unroll
+        for (int j = P - 2; j >= 0; --j) p = fma(p, v, scale_exp(seg[(j + 1) * D + d], sexp) * double(j + 1));
+        s = fma(p, p, s);
+    }
+    double f = w * sqrt(s);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
+    return scale_exp(f * hw, -sexp);
 }
 
 }  // namespace gcv

@@ -406,13 +406,30 @@ __global__ void __launch_bounds__(WK_THREADS, PREC == 3 ? 6 : walk_blocks(CODE))
             }
             __syncwarp(FULL);
             if constexpr (PREC >= 2) {
-                for (int g = lane; g < total; g += 32) {
-                    const int q = W.order[g], qs = W.slot[q];
-                    const ff kf = unpack_ff(W.val[q]);
-                    double K = ff_to_double(kf);
-                    if (W.fits[qs] && isfinite(kf.hi))
-                        K = leaf_k15<CODE>(coef64(qs), W.sexp[qs], W.key[q] & WK_K_MASK, wk_depth(W.key[q]));
-                    W.val[q] = K;
+                for (int g0 = 0; g0 < total; g0 += 32) {
+                    const int g = g0 + lane, q = g < total ? W.order[g] : 0;
+                    bool again = false;
+                    if (g < total) {
+                        const int qs = W.slot[q];
+                        const ff kf = unpack_ff(W.val[q]);
+                        double K = ff_to_double(kf);
+                        if (W.fits[qs] && isfinite(kf.hi))
+                            K = leaf_k15<CODE>(coef64(qs), W.sexp[qs], W.key[q] & WK_K_MASK, wk_depth(W.key[q]), again);
+                        if (!again) W.val[q] = K;
+                    }
+                    if constexpr (CODE > 0) {
+                        // two leaves at a time, 16 lanes each (the last one by both halves)
+                        for (unsigned m = __ballot_sync(FULL, again); m;) {
+                            const int a = __ffs(m) - 1;
+                            m &= m - 1;
+                            const int b = m ? __ffs(m) - 1 : a;
+                            m &= m - 1;
+                            const int qa = __shfl_sync(FULL, q, lane < 16 ? a : b), qs = W.slot[qa];
+                            const double K =
+                                leaf_k15_nodes<CODE>(coef64(qs), W.sexp[qs], W.key[qa] & WK_K_MASK, wk_depth(W.key[qa]));
+                            if ((lane & 15) == 0) W.val[qa] = K;
+                        }
+                    }
                 }
                 __syncwarp(FULL);
             }
