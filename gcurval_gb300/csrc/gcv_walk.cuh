@@ -85,7 +85,7 @@ template <int CODE>
 __device__ __forceinline__ int interval_exponent(const double* __restrict__ seg)
 {
     if constexpr (CODE == 0) {
-        return exponent_of(fmax(seg[3], seg[4]) * (PI * ELLIPSE_PIECE_SCALE));
+        return exponent_of(fmax(fabs(seg[3]), fabs(seg[4])) * (PI * ELLIPSE_PIECE_SCALE));  // axes of either sign
     } else {
         constexpr int D = code_dim(CODE);
         int m = 0;
