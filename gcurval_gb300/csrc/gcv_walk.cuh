@@ -250,16 +250,22 @@ __global__ void __launch_bounds__(WK_THREADS, PREC == 3 ? 6 : walk_blocks(CODE))
         // keeps the left one in place, the right one is a new node behind it
         auto split_nodes = [&](bool split, bool right_flag, bool left_to_stack) {
             if (split) {
+                // the split's two nodes for the one are counted first: of the splits that
+                // an interval wants at once, those beyond its limit see it, so it
+                // is given up if and only if its tree has more leaves than
+                // the limit, whichever rounds its splits fall in
                 const bool learned = CODE > 0 && W.dq[sl] != 0u;
-                if (W.count[sl] >> 16 >= (learned ? LCAP : WK_LEAVES)) {
+                if (atomicAdd(&W.count[sl], 0x10001) >> 16 >= (learned ? LCAP : WK_LEAVES)) {
                     W.dead[sl] = learned ? WK_PLAIN : WK_DEEP;
                     dead = true;
                     split = false;
+                    atomicSub(&W.count[sl], 0x10001);
                 }
             }
             __syncwarp(FULL);
             const int rank = __popc(__ballot_sync(FULL, split) & lt_mask);
             const bool none_left = split && rank >= nfree;
+            if (none_left) atomicSub(&W.count[sl], 0x10001);
             split = split && !none_left;
             const int cnt = __popc(__ballot_sync(FULL, split));
             if (split) {
@@ -269,7 +275,6 @@ __global__ void __launch_bounds__(WK_THREADS, PREC == 3 ? 6 : walk_blocks(CODE))
                 W.slot[right] = (unsigned char)sl;
                 W.next[right] = W.next[nd];
                 W.next[nd] = (unsigned char)right;
-                atomicAdd(&W.count[sl], 0x10001);
                 if (left_to_stack) {
                     W.key[nd] = wk_key(k, depth, false);
                     W.stack[nstack + 2 * rank] = (unsigned char)right;
