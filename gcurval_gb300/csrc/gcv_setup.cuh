@@ -15,6 +15,9 @@
 // kinds of step share the difference.  The position at m follows from the same
 // interpolated values: replacing the knots of P_0 by m one after another,
 //   C(m) = P_0 + sum_r (m - t_r) g(m^r, t_{r+2} ..).
+// g is carried times w and (m - t_r) over w, so that nothing has the units of a
+// control point over a knot: with Q_j itself, knots in units of 1e-30 under
+// coordinates of 1e9 overflowed in float-float.
 // For degree 5 in 3D that is about 3,200 instructions in float-float, against
 // 5,600 of the basis recursion on polynomials it replaces (whose code also missed
 // the instruction cache); planar cubics take about 95 instead of 190 FP64
@@ -71,7 +74,8 @@ struct SpanKnots {
     static constexpr int N = P - 1;
     T w;                     // half width
     T t[2 * P];              // knots span - P + 1 .. span + P
-    T rq[P];                 // 1 / (t[j + P] - t[j]): the derivative's control points
+    T rq[P];                 // w / (t[j + P] - t[j]): w times the derivative's control points
+    T tw[P > 1 ? P - 1 : 1];  // (m - t[r]) / w; 1 for r = P - 1
     T alpha[N * P / 2 + 1];  // step s, pair j: (m - t_lo) / (t_hi - t_lo)
     T beta[N * P / 2 + 1];   // w / (t_hi - t_lo)
     // pairs of the steps before s (step s has N - s)
@@ -97,7 +101,12 @@ struct SpanKnots {
             }
         }
 #pragma unroll
-        for (int j = 0; j < P; ++j) rq[j] = n_recip(n_sub(t[j + P], t[j]));
+        for (int j = 0; j < P; ++j) rq[j] = n_mul(w, n_recip(n_sub(t[j + P], t[j])));
+        if constexpr (P > 1) {
+            const T rw = n_recip(w);
+#pragma unroll
+            for (int r = 0; r < P - 1; ++r) tw[r] = n_mul(neg(t[r]), rw);
+        }
 #pragma unroll
         for (int s = 0; s < N; ++s)
 #pragma unroll
@@ -137,7 +146,7 @@ __device__ __forceinline__ void polar_both(const SpanKnots<P, T>& k, const T* in
     }
 }
 
-// q: the P control points; out[l] = g(m^(N-l), w^l); lead[r] = g(m^r, t_{r+2} ..), the
+// q: the P control points times w; out[l] = w g(m^(N-l), w^l); lead[r] = w g(m^r, t_{r+2} ..), the
 // first of the values interpolated r times
 template <int P, typename T>
 __device__ __forceinline__ void polar_tree(const SpanKnots<P, T>& k, const T* q, T* out, T* lead)
@@ -188,9 +197,9 @@ __device__ __forceinline__ T expand_dim(const SpanKnots<P, T>& k, const double* 
         q[j] = n_mul(q[j], k.rq[j]);
     }
     polar_tree<P>(k, q, out, lead);
-    T a = n_mul(SpanKnots<P, T>::neg(k.t[0]), lead[0]);
+    T a = lead[P - 1];
 #pragma unroll
-    for (int r = 1; r < P; ++r) a = n_fma(SpanKnots<P, T>::neg(k.t[r]), lead[r], a);
+    for (int r = 0; r < P - 1; ++r) a = n_fma(k.tw[r], lead[r], a);
     return a;
 }
 
@@ -208,7 +217,7 @@ __device__ __forceinline__ void bspline_setup(const double* __restrict__ kv, con
         double g[P];
         out[d] = c0[d] + expand_dim<P, D>(k, c0, d, g);
 #pragma unroll
-        for (int l = 0; l < P; ++l) out[(l + 1) * D + d] = n_times(k.w, binomial(P, l + 1)) * g[l];
+        for (int l = 0; l < P; ++l) out[(l + 1) * D + d] = n_times(g[l], binomial(P, l + 1));
     }
 }
 
@@ -230,7 +239,7 @@ __device__ __forceinline__ void bspline_setup_ff(const double* __restrict__ kv, 
         out[d] = make_float2(a.hi, a.lo);
 #pragma unroll
         for (int l = 0; l < P; ++l) {
-            const ff b = ff_mul(n_times(k.w, P * binomial(P - 1, l)), g[l]);
+            const ff b = n_times(g[l], P * binomial(P - 1, l));
             out[(l + 1) * D + d] = make_float2(b.hi, b.lo);
         }
     }
