@@ -95,6 +95,13 @@ __device__ __forceinline__ long long fix_of_double(double x)
     const long long v = sh >= 0 ? (long long)(m << (sh & 15)) : (sh > -53 ? (long long)(m >> -sh) : 0ll);
     return (long long)b < 0 ? -v : v;
 }
+// back, the scaling by the exponent bits: with the unit in a factor, knot spans below
+// 2^-960 became denormals and their parameters lost digits
+__device__ __forceinline__ double double_of_fix(long long v)
+{
+    const double x = __ll2double_rn(v);
+    return __hiloint2double(__double2hiint(x) - (v != 0 ? 60 << 20 : 0), __double2loint(x));
+}
 __device__ __forceinline__ long long fix_of_float(float x) { return __float2ll_rn(x * 1152921504606846976.0f); }
 
 // float -> double from the bit pattern (the FP64 pipe's conversion for zeros,

@@ -417,15 +417,14 @@ __global__ void __maxnreg__(SAMPLE_FF_REGS) k_sample_ff(SampleParams P, const TA
                 // both ends, the operands chosen so that one side is evaluated
                 const double t0 = t.seg_t0[s], t1 = t.seg_t1[s];
                 const bool low = v <= 0;
-                u = fma(__ll2double_rn(v + (low ? FIX_ONE : -FIX_ONE)), (t1 - t0) * (0.5 / (double)FIX_ONE),
-                        low ? t0 : t1);
+                u = fma(double_of_fix(v + (low ? FIX_ONE : -FIX_ONE)), 0.5 * (t1 - t0), low ? t0 : t1);
             }
             P.out[i] = u;
         } else {
             double p3[3] = {0.0, 0.0, 0.0};
             if (s >= 0) {
                 const TAB* seg = coef + b.coef_off[c] + (int64_t)(s - s0) * code_stride(CODE);
-                const double vd = __ll2double_rn(v) * (1.0 / (double)FIX_ONE);
+                const double vd = double_of_fix(v);
                 double cd[MAX_COEF];
                 const double* pc = cd;
                 if constexpr (FROM64) {
