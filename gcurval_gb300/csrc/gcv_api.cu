@@ -1564,6 +1564,7 @@ gcv_status enqueue_sampling_graph(gcv_ctx* c, const int* d_counts, const double*
     P.rtol = c->opt.rtol;
     P.eps_frac = (float)(SAMPLE_EPS_FRAC * c->opt.rtol);
     P.min_runs = sm_count() * SAMPLE_RUNS_PER_SM;
+    P.err = c->ctr.p + C_ERR;
     // grids for any sample count: the kernels loop over their ranges
     const int64_t nominal = (int64_t)sm_count() * c->knobs.sample_blocks_per_sm * c->knobs.sample_threads;
     if (c->code >= 0) {

@@ -104,6 +104,7 @@ struct SampleParams {
     int64_t cb, ce;
     int64_t s_begin, s_end;  // sample range of the launch when curve_list is NULL
     const int64_t* s_end_dev;  // when set: the end of that range, read on the device
+    const unsigned long long* err;  // when set (captured steps): the table's error word, see sample_range
     int min_runs;  // k_sample_ff: runs the launch should at least consist of (shorter runs then)
 };
 
@@ -113,6 +114,10 @@ __device__ __forceinline__ void sample_range(const SampleParams& P, int64_t& i0,
 {
     i0 = P.curve_list ? P.list_off[P.cb] : P.s_begin;
     i1 = P.curve_list ? P.list_off[P.ce] : (P.s_end_dev ? *P.s_end_dev : P.s_end);
+    // A captured step samples before the host has seen that a pool was too small.
+    // The table then holds intervals whose leaves lie outside the pool or were
+    // never written: nothing is sampled, and the host runs the step once more.
+    if (P.err && (*P.err & (ERR_POOL | ERR_DEEP_LIST))) i1 = i0;
 }
 __device__ __forceinline__ int sample_curve(const SampleParams& P, int64_t i, int64_t& gi)
 {

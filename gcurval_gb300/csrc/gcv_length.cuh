@@ -44,8 +44,8 @@ struct LengthParams {
     int collect;
     const int* list;  // segments to process; NULL: segments 0 .. n_items - 1
     int64_t n_items;
-    const unsigned long long* n_items_dev;  // when set: the item count, read on the device
-                                            // (graph launches; n_items then sizes the grid)
+    const unsigned long long* n_items_dev;  // when set: the item count, read on the device (captured
+                                            // steps; n_items is then the list's size: see length_items)
     const float2* coef_ff;  // float-float copy of the coefficients (PREC 1)
     unsigned long long* work;  // work-queue head of this launch (starts at 0)
     const uint32_t* starts;    // learned quarter start depths per segment (NULL: plain walk)
@@ -57,6 +57,15 @@ struct LengthParams {
     int by_item;
     int64_t coef_base;
 };
+
+// Items of a launch.  The count on the device is of the intervals that wanted a place
+// in the list, which may be more than it has.
+__device__ __forceinline__ int64_t length_items(const LengthParams& P)
+{
+    if (!P.n_items_dev) return P.n_items;
+    const int64_t n = (int64_t)*P.n_items_dev;
+    return n < P.n_items ? n : P.n_items;
+}
 
 // Launches k_length<MODE, CODE, PREC> over P (persistent grid sized from the
 // occupancy, capped at blocks_per_sm_cap per SM, and sm_count); defined with the kernel in gcv_length_impl.cuh and

@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(LK_THREADS) k_length_hw(LengthParams P)
     const unsigned half_mask = half_base ? 0xffff0000u : 0x0000ffffu;
     const double eps50 = 50.0 * 1.4210854715202004e-14;  // round-off floor: 50 float-float units
 
-    const int64_t n_items = P.n_items_dev ? (int64_t)*P.n_items_dev : P.n_items;
+    const int64_t n_items = length_items(P);
     bool active = false, exhausted = false;
     int64_t s = 0;
     const float2* cff = nullptr;

@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(LK_THREADS) k_length(LengthParams P)
     // (FP64: 2^-52; float-float: ~2^-46)
     const double eps50 = PREC == 1 ? 50.0 * 1.4210854715202004e-14 : 50.0 * 2.220446049250313e-16;
 
-    const int64_t n_items = P.n_items_dev ? (int64_t)*P.n_items_dev : P.n_items;
+    const int64_t n_items = length_items(P);
     bool active = false, exhausted = false;
     int64_t s = 0, pool = 0;
     int code = CODE >= 0 ? CODE : 0;
