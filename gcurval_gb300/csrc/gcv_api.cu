@@ -411,6 +411,7 @@ struct gcv_ctx {
         int is_relative, what, learned;
         gcv_options opt;
     } gargs{};
+    std::vector<const void*> gbufs;  // the captured step's device buffers (step_buffers)
     DBuf<int64_t> scan_blk;
     int64_t graph_kernels = 0;
     Knobs knobs, gknobs;  // launch shapes in use / in the captured step
@@ -1590,6 +1591,20 @@ gcv_status enqueue_sampling_graph(gcv_ctx* c, const int* d_counts, const double*
     return GCV_OK;
 }
 
+// The device buffers whose addresses a captured step holds.  An ordinary build in
+// between may have replaced some (a larger leaf pool or deep list, the other
+// precision's coefficients): such a step is captured again.
+std::vector<const void*> step_buffers(const gcv_ctx* c)
+{
+    return {c->kind.p,      c->degree.p,    c->dim.p,       c->knot_off.p,   c->ctrl_off.p, c->knots.p,
+            c->ctrl.p,      c->seg_off.p,   c->coef_off.p,  c->seg_curve.p,  c->seg_list.p, c->curve_list.p,
+            c->mlp_w,       c->starts.p,    c->feat16.p,    c->coef.p,       c->coef_ff.p,  c->seg_t0.p,
+            c->seg_t1.p,    c->seg_f0.p,    c->seg_q0.p,    c->seg_len.p,    c->seg_cum.p,  c->curve_len.p,
+            c->leaf_off.p,  c->leaf_cnt.p,  c->leaf_v.p,    c->leaf_cum.p,   c->leaf_f.p,   c->leaf_q.p,
+            c->deep_list.p, c->ctr.p,       c->scan_status.p, c->scan_flag.p, c->scan_hi.p, c->scan_lo.p,
+            c->sample_off.p, c->list_sample_off.p, c->scan_blk.p};
+}
+
 void drop_graph(gcv_ctx* c)
 {
     if (c->gexec) cudaGraphExecDestroy(c->gexec);
@@ -2361,7 +2376,7 @@ gcv_status gcv_step_graph(gcv_ctx* ctx, const int* d_counts, const double* d_pos
     const bool same = c->gexec && c->gknobs == c->knobs && c->gargs.counts == d_counts && c->gargs.pos == d_pos && c->gargs.out == d_out &&
                       c->gargs.is_relative == is_relative && c->gargs.what == what &&
                       c->gargs.learned == (c->opt.learned && c->mlp_w ? 1 : 0) &&
-                      std::memcmp(&c->gargs.opt, &c->opt, sizeof(gcv_options)) == 0;
+                      std::memcmp(&c->gargs.opt, &c->opt, sizeof(gcv_options)) == 0 && c->gbufs == step_buffers(c);
     if (!same) {
         drop_graph(c);
         CHECK(c->sample_off.reserve((size_t)c->n_curve + 1));
@@ -2401,6 +2416,7 @@ gcv_status gcv_step_graph(gcv_ctx* ctx, const int* d_counts, const double* d_pos
         c->gargs.what = what;
         c->gargs.learned = c->opt.learned && c->mlp_w ? 1 : 0;
         std::memcpy(&c->gargs.opt, &c->opt, sizeof(gcv_options));
+        c->gbufs = step_buffers(c);
         c->gknobs = c->knobs;
         // kernels per replay, for the launch count
         size_t nn = 0;
