@@ -166,10 +166,35 @@ __global__ void __launch_bounds__(256) k_sgemm(GemmArgs g)
     }
 }
 
-// g[i] = the sum of the chunks' partial gradients, in chunk order
-__global__ void k_sum_partials(const float* __restrict__ part, int chunks, int count, float* __restrict__ g)
+constexpr int SUM_THREADS = 128;
+constexpr int LOSS_THREADS = 64;  // rows per block of k_loss
+constexpr int LOSS_BLOCKS = 152 * 32;
+int loss_blocks(int n) { return std::min((n + LOSS_THREADS - 1) / LOSS_THREADS, LOSS_BLOCKS); }
+
+// g[i] = the sum of the chunks' partial gradients, in chunk order; the last block adds
+// up the loss of k_loss's blocks, in a fixed order and in FP64 (added by FP32 atomics,
+// the loss of 8,192 rows differed by 2e-7 from call to call)
+__global__ void __launch_bounds__(SUM_THREADS) k_sum_partials(const float* __restrict__ part, int chunks, int count,
+                                                              float* __restrict__ g, const float* __restrict__ loss_part,
+                                                              int n_loss, float* __restrict__ loss3)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.x + 1 == gridDim.x) {
+        __shared__ double s_l[SUM_THREADS];
+        for (int k = 0; k < 3; ++k) {
+            double l = 0.0;
+            for (int b = threadIdx.x; b < n_loss; b += SUM_THREADS) l += (double)loss_part[3 * b + k];
+            s_l[threadIdx.x] = l;
+            __syncthreads();
+            for (int o = SUM_THREADS / 2; o > 0; o >>= 1) {
+                if (threadIdx.x < o) s_l[threadIdx.x] += s_l[threadIdx.x + o];
+                __syncthreads();
+            }
+            if (threadIdx.x == 0) loss3[k] = (float)s_l[0];
+            __syncthreads();
+        }
+        return;
+    }
+    const int i = blockIdx.x * SUM_THREADS + threadIdx.x;
     if (i >= count) return;
     float s = 0.0f;
 #pragma unroll 8
@@ -177,10 +202,11 @@ __global__ void k_sum_partials(const float* __restrict__ part, int chunks, int c
     g[i] = s;
 }
 
-// loss parts (sums over the batch) and dOut = d(mean loss) / d out
-__global__ void k_loss(const float* out, const int* depth, const float* share, const float* tg, int n, float* dOut,
-                       float* loss3)
+// loss parts (sums over the block's rows) and dOut = d(mean loss) / d out
+__global__ void __launch_bounds__(LOSS_THREADS) k_loss(const float* out, const int* depth, const float* share,
+                                                       const float* tg, int n, float* dOut, float* loss_part)
 {
+    __shared__ float s_l[LOSS_THREADS / 32][3];
     float l0 = 0.0f, l1 = 0.0f, l2 = 0.0f;
     const float inv = 1.0f / (float)n;
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x) {
@@ -219,10 +245,13 @@ __global__ void k_loss(const float* out, const int* depth, const float* share, c
         l2 += __shfl_xor_sync(0xffffffffu, l2, o);
     }
     if ((threadIdx.x & 31) == 0) {
-        atomicAdd(loss3 + 0, l0);
-        atomicAdd(loss3 + 1, l1);
-        atomicAdd(loss3 + 2, l2);
+        s_l[threadIdx.x >> 5][0] = l0;
+        s_l[threadIdx.x >> 5][1] = l1;
+        s_l[threadIdx.x >> 5][2] = l2;
     }
+    __syncthreads();
+    static_assert(LOSS_THREADS == 64, "two warps' sums");
+    if (threadIdx.x < 3) loss_part[3 * blockIdx.x + threadIdx.x] = s_l[0][threadIdx.x] + s_l[1][threadIdx.x];
 }
 
 __global__ void k_adam(float* w, const float* g, float* m, float* v, int count, float lr, float b1, float b2, float eps,
@@ -264,6 +293,7 @@ struct gcv_mlp_trainer {
     float *w = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
     float *Z[3] = {}, *H[3] = {}, *out = nullptr, *dOut = nullptr, *dA = nullptr, *dB = nullptr, *loss3 = nullptr;
     float* part = nullptr;  // GRAD_CHUNKS partial gradients, each packed like w
+    float* loss_part = nullptr;  // the loss parts of k_loss's blocks
     long long step = 0;
 };
 
@@ -304,9 +334,7 @@ void forward(gcv_mlp_trainer* tr, const float* X, int n)
 // loss and gradients of the mean loss into tr->g
 void backward(gcv_mlp_trainer* tr, const float* X, const int* depth, const float* share, const float* tg, int n)
 {
-    cudaMemsetAsync(tr->loss3, 0, 3 * sizeof(float), tr->st);
-    k_loss<<<(unsigned)std::min<size_t>(((size_t)n + 63) / 64, 152 * 32), 64, 0, tr->st>>>(tr->out, depth, share, tg, n,
-                                                                                          tr->dOut, tr->loss3);
+    k_loss<<<loss_blocks(n), LOSS_THREADS, 0, tr->st>>>(tr->out, depth, share, tg, n, tr->dOut, tr->loss_part);
     const int rows = grad_chunk_rows(n), chunks = (n + rows - 1) / rows;
     const float* dz = tr->dOut;  // d loss / d (layer l's output before its activation)
     float* bufs[2] = {tr->dA, tr->dB};
@@ -322,7 +350,8 @@ void backward(gcv_mlp_trainer* tr, const float* X, const int* depth, const float
             dz = next;
         }
     }
-    k_sum_partials<<<(MLP_NPARAM + 127) / 128, 128, 0, tr->st>>>(tr->part, chunks, MLP_NPARAM, tr->g);
+    k_sum_partials<<<(MLP_NPARAM + SUM_THREADS - 1) / SUM_THREADS + 1, SUM_THREADS, 0, tr->st>>>(
+        tr->part, chunks, MLP_NPARAM, tr->g, tr->loss_part, loss_blocks(n), tr->loss3);
 }
 
 }  // namespace
@@ -354,6 +383,7 @@ gcv_status gcv_mlp_trainer_create(gcv_mlp_trainer** out, int max_batch, unsigned
     if (e == cudaSuccess) e = cudaMalloc(&tr->dA, A);
     if (e == cudaSuccess) e = cudaMalloc(&tr->dB, A);
     if (e == cudaSuccess) e = cudaMalloc(&tr->loss3, 3 * sizeof(float));
+    if (e == cudaSuccess) e = cudaMalloc(&tr->loss_part, (size_t)loss_blocks(max_batch) * 3 * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&tr->part, GRAD_CHUNKS * P);
     if (e != cudaSuccess) {
         gcv_mlp_trainer_destroy(tr);
@@ -383,7 +413,7 @@ gcv_status gcv_mlp_trainer_destroy(gcv_mlp_trainer* tr)
 {
     if (!tr) return GCV_OK;
     float* bufs[] = {tr->w, tr->g, tr->m, tr->v, tr->Z[0], tr->Z[1], tr->Z[2], tr->H[0], tr->H[1], tr->H[2],
-                     tr->out, tr->dOut, tr->dA, tr->dB, tr->loss3, tr->part};
+                     tr->out, tr->dOut, tr->dA, tr->dB, tr->loss3, tr->part, tr->loss_part};
     for (float* b : bufs)
         if (b) cudaFree(b);
     delete tr;
