@@ -58,13 +58,20 @@ __device__ __forceinline__ unsigned long long wk_key(unsigned long long k, int d
 }
 __device__ __forceinline__ int wk_depth(unsigned long long key) { return (int)(key >> 56) & 0x3F; }
 
+// a slot's counts: panels to evaluate (low 16 bits), nodes of the list (8), evaluated
+// panels that were split (8)
+constexpr unsigned WK_ONE_NODE = 0x10001u, WK_ONE_SPLIT = 0x1000000u;
+__device__ __forceinline__ int wk_nodes(unsigned count) { return (int)(count >> 16 & 0xFFu); }
+__device__ __forceinline__ int wk_splits(unsigned count) { return (int)(count >> 24); }
+static_assert(WK_LEAVES + 32 <= 256, "a limit and a round's splits beyond it fit eight bits");
+
 struct WalkWarp {
     unsigned long long key[WK_NODES];
     double val[WK_NODES];   // the panel's K15 (float-float pair, then FP64), finally the running sum
     double whole[WK_SLOTS];  // float-float pair: K15 of the whole interval, or its chord (learned start)
     float tolf[WK_SLOTS];    // rtol times that
     int item[WK_SLOTS], sexp[WK_SLOTS];
-    int count[WK_SLOTS];    // panels to evaluate (low 16 bits), nodes of the list (high 16)
+    unsigned count[WK_SLOTS];  // see wk_nodes
     uint32_t dq[WK_SLOTS];  // learned quarter start depths (0: from the whole interval)
     unsigned char next[WK_NODES], slot[WK_NODES], stack[WK_NODES], freel[WK_NODES], order[WK_NODES];
     unsigned char head[WK_SLOTS], fslot[WK_SLOTS], done[WK_SLOTS], dead[WK_SLOTS], fits[WK_SLOTS], later[WK_SLOTS];
@@ -181,7 +188,7 @@ __global__ void __launch_bounds__(WK_THREADS, PREC == 3 ? 6 : walk_blocks(CODE))
     // slot sl (again) at its root, which goes to stack position `at`
     auto start = [&](int sl, int nd, uint32_t dq, int at) {
         W.head[sl] = (unsigned char)nd;
-        W.count[sl] = 0x10001;
+        W.count[sl] = WK_ONE_NODE;
         W.dead[sl] = WK_LIVE;
         W.dq[sl] = dq;
         W.key[nd] = wk_key(0ull, 0, dq != 0u);
@@ -249,23 +256,24 @@ __global__ void __launch_bounds__(WK_THREADS, PREC == 3 ? 6 : walk_blocks(CODE))
         // replaces the lanes' panels (where `split`) by their halves: the lane
         // keeps the left one in place, the right one is a new node behind it
         auto split_nodes = [&](bool split, bool right_flag, bool left_to_stack) {
+            const unsigned one = left_to_stack ? WK_ONE_NODE + WK_ONE_SPLIT : WK_ONE_NODE;
             if (split) {
                 // the split's two nodes for the one are counted first: of the splits that
                 // an interval wants at once, those beyond its limit see it, so it
                 // is given up if and only if its tree has more leaves than
                 // the limit, whichever rounds its splits fall in
                 const bool learned = CODE > 0 && W.dq[sl] != 0u;
-                if (atomicAdd(&W.count[sl], 0x10001) >> 16 >= (learned ? LCAP : WK_LEAVES)) {
+                if (wk_nodes(atomicAdd(&W.count[sl], one)) >= (learned ? LCAP : WK_LEAVES)) {
                     W.dead[sl] = learned ? WK_PLAIN : WK_DEEP;
                     dead = true;
                     split = false;
-                    atomicSub(&W.count[sl], 0x10001);
+                    atomicSub(&W.count[sl], one);
                 }
             }
             __syncwarp(FULL);
             const int rank = __popc(__ballot_sync(FULL, split) & lt_mask);
             const bool none_left = split && rank >= nfree;
-            if (none_left) atomicSub(&W.count[sl], 0x10001);
+            if (none_left) atomicSub(&W.count[sl], one);
             split = split && !none_left;
             const int cnt = __popc(__ballot_sync(FULL, split));
             if (split) {
@@ -343,7 +351,6 @@ __global__ void __launch_bounds__(WK_THREADS, PREC == 3 ? 6 : walk_blocks(CODE))
                     ok = !finite || accept_fp64<CODE>(coef64(sl), k, depth,
                                                       depth == 0 ? P.rtol : scalbn(tolerance(), W.sexp[sl]));
             }
-            ++my_panels;
             if (ok || depth >= P.max_depth || !finite) {
                 my_nonfinite += !finite;
                 W.val[nd] = pack_ff(Kf);
@@ -377,7 +384,7 @@ __global__ void __launch_bounds__(WK_THREADS, PREC == 3 ? 6 : walk_blocks(CODE))
             }
         }
         // ---- intervals whose last panel was accepted (or given up)
-        const bool fin = active && (!reject || dead) && (atomicSub(&W.count[sl], 1) & 0xFFFF) == 1;
+        const bool fin = active && (!reject || dead) && (atomicSub(&W.count[sl], 1u) & 0xFFFFu) == 1u;
         const unsigned fm = __ballot_sync(FULL, fin);
         if (fin) W.done[ndone + __popc(fm & lt_mask)] = (unsigned char)sl;
         ndone += __popc(fm);
@@ -390,8 +397,10 @@ __global__ void __launch_bounds__(WK_THREADS, PREC == 3 ? 6 : walk_blocks(CODE))
             const int fs = mine ? W.done[ndone + lane] : 0;
             const int why = mine ? W.dead[fs] : WK_LIVE;
             const bool gone = why != WK_LIVE;
-            const int nodes = mine ? W.count[fs] >> 16 : 0;
+            const unsigned counts = mine ? W.count[fs] : 0u;
+            const int nodes = wk_nodes(counts);
             const int cnt = gone ? 0 : nodes;
+            if (!gone) my_panels += cnt + wk_splits(counts);
             const int incl = warp_incl_scan(cnt, lane), total = __shfl_sync(FULL, incl, 31);
             unsigned long long base = 0;
             if constexpr (PREC != 3) {

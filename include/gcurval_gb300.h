@@ -119,7 +119,9 @@ typedef struct gcv_stats {
     int64_t n_curves;
     int64_t n_segments;       /* knot intervals */
     int64_t n_leaves;         /* accepted quadrature panels (table entries) */
-    int64_t n_panels;         /* panels evaluated by the length kernel */
+    int64_t n_panels;         /* panels evaluated by the walks that the table is from (with
+                                 collect_stats); GCV_MAP_HALF_WARP and rtol < 1e-12 also
+                                 count the walks that the deep passes do once more */
     int64_t n_deep_segments;  /* intervals that needed the deep (global-memory) path */
     int64_t n_capped;         /* panels accepted at max_depth without meeting rtol */
     int64_t n_samples;

@@ -88,3 +88,18 @@ def test_trees_near_the_limit(precision, gpu_lib):
     pick = np.flatnonzero((leaves >= 94) & (leaves <= 127))
     assert np.sum((leaves > 96) & (leaves <= 127)) >= 30
     same_alone_as_among_others(few_samples(ref), pick, precision=precision, rtol=1e-12, max_depth=44)
+
+
+@pytest.mark.parametrize("network", [None, START])
+@pytest.mark.parametrize("precision", [g.GCV_MIXED, g.GCV_PLAIN_FP64])
+def test_panels_are_counted_once(precision, network, gpu_lib):
+    """The panel count is the tables': of 500 copies in random order 500 times one copy's, each curve by itself."""
+    ref = Cusps(300, 3, seed=23)
+    kw = dict(precision=precision, rtol=1e-6 if network else 1e-12, max_depth=44)
+    weights = None if network is None else depth_network(network)
+    b = few_samples(ref)
+    alone = [table(b.subset(np.array([i])), weights, **kw)[2] for i in range(b.n_curve)]
+    order = np.random.default_rng(8).permutation(np.repeat(np.arange(b.n_curve), 500))
+    st = table(b.subset(order), weights, **kw)[2]
+    for what in ("n_panels", "n_leaves", "n_capped", "n_deep_segments"):
+        assert st[what] == 500 * sum(a[what] for a in alone), what
