@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(256) k_sgemm(GemmArgs g)
 constexpr int SUM_THREADS = 128;
 constexpr int LOSS_THREADS = 64;  // rows per block of k_loss
 constexpr int LOSS_BLOCKS = 152 * 32;
-int loss_blocks(int n) { return std::min((n + LOSS_THREADS - 1) / LOSS_THREADS, LOSS_BLOCKS); }
+int loss_blocks(int n) { return (int)std::min<int64_t>(((int64_t)n + LOSS_THREADS - 1) / LOSS_THREADS, LOSS_BLOCKS); }
 
 // g[i] = the sum of the chunks' partial gradients, in chunk order; the last block adds
 // up the loss of k_loss's blocks, in a fixed order and in FP64 (added by FP32 atomics,
@@ -283,6 +283,9 @@ int grad_chunk_rows(int n)
     return (rows + GK - 1) / GK * GK;
 }
 
+// the most chunks of any batch up to max_batch rows (a larger batch may take fewer, longer ones)
+int grad_chunks_max(int max_batch) { return (int)std::min<int64_t>(GRAD_CHUNKS, ((int64_t)max_batch + 63) / 64); }
+
 unsigned blocks_for(size_t n) { return (unsigned)std::min<size_t>((n + 255) / 256, 152 * 32); }
 
 }  // namespace
@@ -292,7 +295,7 @@ struct gcv_mlp_trainer {
     cudaStream_t st = nullptr;
     float *w = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
     float *Z[3] = {}, *H[3] = {}, *out = nullptr, *dOut = nullptr, *dA = nullptr, *dB = nullptr, *loss3 = nullptr;
-    float* part = nullptr;  // GRAD_CHUNKS partial gradients, each packed like w
+    float* part = nullptr;  // grad_chunks_max(max_batch) partial gradients, each packed like w
     float* loss_part = nullptr;  // the loss parts of k_loss's blocks
     long long step = 0;
 };
@@ -384,7 +387,7 @@ gcv_status gcv_mlp_trainer_create(gcv_mlp_trainer** out, int max_batch, unsigned
     if (e == cudaSuccess) e = cudaMalloc(&tr->dB, A);
     if (e == cudaSuccess) e = cudaMalloc(&tr->loss3, 3 * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc(&tr->loss_part, (size_t)loss_blocks(max_batch) * 3 * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&tr->part, GRAD_CHUNKS * P);
+    if (e == cudaSuccess) e = cudaMalloc(&tr->part, (size_t)grad_chunks_max(max_batch) * P);
     if (e != cudaSuccess) {
         gcv_mlp_trainer_destroy(tr);
         return tfail(GCV_ERR_OUT_OF_MEMORY, std::string("trainer buffers: ") + cudaGetErrorString(e));
