@@ -225,7 +225,9 @@ __device__ __forceinline__ long long ff_leaf_newton(const TAB* __restrict__ seg,
             // 1.3e-7 was seen; with 3.5e-7 the errors at rtol 1e-11 came out a
             // tenth above the FP64 kernel's)
             const float noise = 5e-7f * fabsf(Fh);
-            bool ok = (eps_t < eps_s ? res : res + noise) <= eps_s;
+            // FP64 tables at every tolerance: without it samples at rtol 1e-9 were
+            // up to 1.4e-10 of the length off, where the FP64 kernel kept 1e-10
+            bool ok = (!FROM64 && eps_t < eps_s ? res : res + noise) <= eps_s;
             // only where the speed changes little over the step: past a cusp E can be
             // small by accident
             if (!ok && fabsf(f1 - f0) + fabsf(ds * dn) <= 0.3f * f0) {
