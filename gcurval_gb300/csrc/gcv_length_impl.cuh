@@ -83,8 +83,10 @@ __device__ __forceinline__ float chord_of(const T* r)
 
 // PREC 0: FP64 panels; PREC 1: float-float panels (GCV_MIXED), whose K15 /
 // G7 / end values enter the same FP64 bookkeeping (error test, leaf table).
+// (One block per SM asked for: without it the compiler takes 4 to 20 registers fewer,
+// and the FP64 walk of 100,000 short spatial cubics 2.86 instead of 2.45 ms.)
 template <int MODE, int CODE, int PREC = 0>
-__global__ void __launch_bounds__(LK_THREADS) k_length(LengthParams P)
+__global__ void __launch_bounds__(LK_THREADS, 1) k_length(LengthParams P)
 {
     static_assert(MODE != 0 || PREC == 0, "the main pass of float-float tables is k_walk");
     constexpr int ROWS = MODE == 0 ? LCAP : 1;
