@@ -205,13 +205,19 @@ struct NoallocSource {
             bspline_setup<P, D>(kv, ctrl + ((int64_t)ko[c] - (int64_t)(P + 1) * c) * D, span, cf);
     }
     __device__ __forceinline__ void finish(int64_t s, double len) const { scratch[HEADER_DOUBLES + s] = len; }
-    // an interval with more leaves than a warp keeps: by its lane alone
-    __device__ __noinline__ void deep(int64_t s, const double* cf) const
+    // one lane alone, all FP64
+    __device__ __forceinline__ double walk(const double* cf, unsigned long long* capped) const
     {
         double der[P * D];
         Eval<bs_code(P, D)>::load_speed(cf, der);
+        return interval_length<bs_code(P, D)>(der, rtol, max_depth, capped);
+    }
+    // an interval with more leaves than a warp keeps (not inlined: it would cost the
+    // warp-wide walk its registers)
+    __device__ __noinline__ void deep(int64_t s, const double* cf) const
+    {
         unsigned long long capped = 0;
-        finish(s, interval_length<bs_code(P, D)>(der, rtol, max_depth, &capped));
+        finish(s, walk(cf, &capped));
         if (capped) count_capped(capped);
     }
     __device__ __forceinline__ void count_capped(unsigned long long n) const
@@ -226,12 +232,14 @@ template <int P, int D>
 __global__ void __launch_bounds__(128) k_noalloc_intervals(NoallocSource<P, D> src, int64_t n_seg)
 {
     if (offsets_bad(src.scratch)) return;
+    unsigned long long capped = 0;
     for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < n_seg;
          s += (int64_t)gridDim.x * blockDim.x) {
         double cf[(P + 1) * D];
         src.setup(s, cf);
-        src.deep(s, cf);
+        src.finish(s, src.walk(cf, &capped));
     }
+    if (capped) src.count_capped(capped);
 }
 
 __global__ void k_noalloc_curves(int n_curve, int P, const int* __restrict__ ko, int64_t n_seg,
