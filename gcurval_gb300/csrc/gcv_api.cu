@@ -363,6 +363,7 @@ struct gcv_ctx {
     DBuf<int64_t> seg_off, coef_off;
     DBuf<int> seg_curve;
     std::vector<int64_t> h_seg_off;
+    bool empty_curves = false;  // some curve has no knot interval
     std::vector<uint8_t> h_kind, h_degree;
     std::vector<double> h_start;  // first parameter value of each curve
     // batches that mix curve codes: segments and curves grouped by code, one
@@ -624,6 +625,7 @@ gcv_status finish_create(gcv_ctx* c, const uint8_t* kind, const uint8_t* degree,
     std::vector<int64_t> seg_off, coef_off;
     CHECK(derive_layout(c, kind, degree, dim, knot_off, ctrl_off, seg_off, coef_off));
     c->h_seg_off = seg_off;
+    for (size_t i = 1; i < seg_off.size() && !c->empty_curves; ++i) c->empty_curves = seg_off[i] == seg_off[i - 1];
     c->h_kind.assign(kind, kind + c->n_curve);
     c->h_degree.assign(degree, degree + c->n_curve);
     (void)knots_host_or_null;
@@ -852,6 +854,8 @@ gcv_status ensure_table_buffers(gcv_ctx* c)
 gcv_status launch_scan(gcv_ctx* c, const Batch& b)
 {
     const int64_t tiles = scan_tiles(c->n_seg);
+    // k_scan writes the lengths of the curves that have intervals
+    if (c->empty_curves) CU(cudaMemsetAsync(c->curve_len.p, 0, (size_t)c->n_curve * sizeof(double), c->stream));
     if (tiles > 0) {
         CU(cudaMemsetAsync(c->scan_status.p, 0, (size_t)(tiles + 1) * sizeof(int), c->stream));
         if (scan_items(c->n_seg) == 4)
@@ -859,8 +863,6 @@ gcv_status launch_scan(gcv_ctx* c, const Batch& b)
         else
             k_scan<32><<<(unsigned)tiles, SCAN_THREADS, 0, c->stream>>>(b, table_view(c), tiles);
         CU(cudaGetLastError());
-    } else if (c->n_curve > 0) {
-        CU(cudaMemsetAsync(c->curve_len.p, 0, (size_t)c->n_curve * sizeof(double), c->stream));
     }
     return GCV_OK;
 }

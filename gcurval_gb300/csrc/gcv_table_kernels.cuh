@@ -167,7 +167,9 @@ __device__ __forceinline__ SegVal shfl_up_sv(const SegVal& x, int d)
     return y;
 }
 
-// Also writes every curve's length (0 for curves without intervals).
+// Also writes the length of every curve that has intervals.  (The thread of a curve's
+// last interval once wrote the zeros of the curves without intervals that follow:
+// a run of 300,000 of them 0.72 ms, one memset 0.01.)
 // scan_status: n_tiles states, then the tile ticket; all 0 at the launch.
 template <int SCAN_ITEMS>
 static __global__ void __launch_bounds__(SCAN_THREADS) k_scan(Batch b, Table t, int64_t n_tiles)
@@ -303,13 +305,7 @@ static __global__ void __launch_bounds__(SCAN_THREADS) k_scan(Batch b, Table t, 
         t.seg_cum[s] = cum;
         const bool end = s + 1 == b.n_seg;
         const bool last = end || (k + 1 < SCAN_ITEMS ? heads >> (k + 1) & 1u : b.seg_curve[s + 1] != b.seg_curve[s]);
-        if (last) {
-            const int c = b.seg_curve[s], next = end ? (int)b.n_curve : b.seg_curve[s + 1];
-            t.curve_len[c] = cum;
-            for (int q = c + 1; q < next; ++q) t.curve_len[q] = 0.0;
-        }
-        if (s == 0)
-            for (int q = 0; q < b.seg_curve[0]; ++q) t.curve_len[q] = 0.0;
+        if (last) t.curve_len[b.seg_curve[s]] = cum;
     }
 }
 
