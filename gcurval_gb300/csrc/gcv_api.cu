@@ -1626,19 +1626,21 @@ gcv_status stage_counts(gcv_ctx* c, const int* n_ptrs, int in_where, int64_t* to
     const int64_t n = c->n_curve;
     std::vector<int> cnt;
     CHECK(to_host(n_ptrs, (size_t)n, in_where, cnt));
+    std::vector<int64_t>& off = c->h_sample_off;
+    off.resize((size_t)n + 1);
+    off[0] = 0;
+    bool negative = false;
+    for (int64_t i = 0; i < n; ++i) {
+        negative |= cnt[(size_t)i] < 0;
+        off[(size_t)i + 1] = off[(size_t)i] + cnt[(size_t)i];
+    }
     if (sizes) {
-        int64_t sum = 0;
-        for (const int x : cnt) sum += x;
+        const int64_t sum = off[(size_t)n];
         *sizes->total = sum;
         if (sum != sizes->positions) return fail(GCV_ERR_INVALID, "sample counts do not add up to the positions given");
         if (sizes->outputs < sum * sizes->width) return fail(GCV_ERR_INVALID, "output too small");
     }
-    std::vector<int64_t>& off = c->h_sample_off;
-    off.assign((size_t)n + 1, 0);
-    for (int64_t i = 0; i < n; ++i) {
-        if (cnt[(size_t)i] < 0) return fail(GCV_ERR_INVALID, "negative sample count");
-        off[(size_t)i + 1] = off[(size_t)i] + cnt[(size_t)i];
-    }
+    if (negative) return fail(GCV_ERR_INVALID, "negative sample count");
     *total = off[(size_t)n];
     CHECK(upload(c->sample_off, off.data(), off.size(), c->stream));
     return GCV_OK;
