@@ -51,7 +51,8 @@ __device__ __forceinline__ ff ff_from_double(double x)
 // x 2^-s -> float-float from the bit pattern, for data of any double range:
 // the caller's s brings the values it works with near 1, and what falls below
 // 2^-70 there is 0 (far under any float-float rounding of them), what rises
-// above 2^126 is infinite.  NaN and infinities pass through.  Selects, no
+// above 2^126 is infinite.  NaN and infinities pass through (s above -1150: a
+// zero's exponent counts as 2^-1023).  Selects, no
 // branches: the samplers convert up to 15 coefficients per Newton step.
 __device__ __forceinline__ ff ff_from_double_scaled(double x, int s)
 {
@@ -64,6 +65,15 @@ __device__ __forceinline__ ff ff_from_double_scaled(double x, int s)
     const float hi = __uint_as_float(sign | (huge ? special : tiny ? 0u : ((unsigned)(e + 127) << 23) | m));
     const float lo = __uint2float_rn(low & 0x1FFFFFFFu) * __uint_as_float(((unsigned)(e - 52 + 127) << 23) | sign);
     return tiny || huge ? ff{hi, 0.0f} : fast_two_sum(hi, lo);
+}
+
+// x 2^-s as (x, s) with x out of the denormals
+__device__ __forceinline__ void lift_denormal(double& x, int& s)
+{
+    if ((__double2hiint(x) & 0x7FF00000) == 0) {
+        x *= 18446744073709551616.0;  // 2^64
+        s += 64;
+    }
 }
 
 // binary exponent of a double's magnitude (0 for 0, infinities and NaN)

@@ -160,6 +160,10 @@ __device__ __forceinline__ void ff_sincospi_small(ff d, ff& s, ff& c)
 }
 
 // ------------------------------------------------------------- evaluators
+// Ellipses whose speeds have an exponent below this may have denormal squares
+// (semi-axes below 2^-511).
+constexpr int ELLIPSE_TINY = -480;
+
 template <int CODE>
 struct EvalFF {
     static constexpr int P = code_degree(CODE);
@@ -186,8 +190,17 @@ struct EvalFF {
     __device__ __forceinline__ static void load(const double* __restrict__ seg, ff* r, int s)
     {
         if constexpr (CODE == 0) {
-            r[0] = ff_from_double_scaled(seg[0], 2 * s);
-            r[1] = ff_from_double_scaled(seg[1], 2 * s);
+            if (s >= ELLIPSE_TINY) {
+                r[0] = ff_from_double_scaled(seg[0], 2 * s);
+                r[1] = ff_from_double_scaled(seg[1], 2 * s);
+            } else {
+                double A = seg[0], B = seg[1];
+                int sA = 2 * s, sB = 2 * s;
+                lift_denormal(A, sA);
+                lift_denormal(B, sB);
+                r[0] = A != 0.0 ? ff_from_double_scaled(A, sA) : ff{0.0f, 0.0f};
+                r[1] = B != 0.0 ? ff_from_double_scaled(B, sB) : ff{0.0f, 0.0f};
+            }
             r[2] = ff{__double2float_rn(seg[2]), 0.0f};
         } else {
 #pragma unroll

@@ -104,8 +104,12 @@ __device__ __forceinline__ double leaf_k15(const double* __restrict__ seg, int s
     int low = 0x7FFFFFFF;
     again = false;
     if constexpr (CODE == 0) {
-        const double B = scale_exp(seg[1], 2 * sexp);
-        double A = scale_exp(seg[0], 2 * sexp), sm, cm;
+        double A = seg[0], B = seg[1], sm, cm;
+        int sA = 2 * sexp, sB = 2 * sexp;
+        lift_denormal(A, sA);
+        lift_denormal(B, sB);
+        A = scale_exp(A, sA);
+        B = scale_exp(B, sB);
         sincospi(fma(mid, ELLIPSE_PIECE_SCALE, seg[2]), &sm, &cm);
         // the pair's rounding enters all 15 nodes alike: its length error is
         // taken back through A (its angle error shifts the panel's nodes

@@ -29,3 +29,23 @@ def test_signs_of_the_axes_do_not_matter(precision, rtol, gpu_lib):
     np.testing.assert_allclose(out[1][0], want, rtol=rtol)
     np.testing.assert_array_equal(out[0][0], out[1][0])
     np.testing.assert_array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("rtol", [1e-10, 1e-12])
+def test_axes_whose_squares_vanish(rtol, gpu_lib):
+    """Semi-axes of 1e-165 and below: length 0, as the FP64 kernels (below rtol 1e-12) have it, and never NaN."""
+    a = 10.0 ** -np.r_[165.0, 172, 173, 174, 180, 250, 300]
+    e = ds.ellipses_from_axes(np.r_[a, -a, a], np.r_[a, a, 0.3 * a])
+    for r in (rtol, 0.5e-12):
+        calc = g.ArclengthCalculateGpu.from_batch(e, precision=g.GCV_PLAIN_FP64, rtol=r)
+        calc.createArclengthTable()
+        assert not calc.getAllCurveArclengths().any()
+
+
+def test_axes_with_denormal_squares(gpu_lib):
+    """Semi-axes of 1e-153 to 1e-157: the squares keep 2^-53 to 2^-28 of themselves."""
+    a = 10.0 ** -np.r_[153.0, 154, 155, 156, 157]
+    e = ds.ellipses_from_axes(np.r_[a, -a], np.r_[a, a])
+    calc = g.ArclengthCalculateGpu.from_batch(e, precision=g.GCV_PLAIN_FP64, rtol=1e-10, max_depth=10)
+    calc.createArclengthTable()
+    np.testing.assert_allclose(calc.getAllCurveArclengths(), 2.0 * np.pi * np.r_[a, a], rtol=1e-8)
