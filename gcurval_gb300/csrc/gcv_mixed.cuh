@@ -341,7 +341,7 @@ __global__ void __maxnreg__(SAMPLE_FF_REGS) k_sample_ff(SampleParams P, const TA
             if (tb <= 0 || (FROM64 && tb > 0x7FF0000000000000ll)) {
                 s = s0;
                 v = -FIX_ONE;
-            } else if (tb >= lb) {
+            } else if (tb >= lb && (!FROM64 || lb >= 0)) {  // (a NaN length with its sign bit set is no end)
                 s = s1 - 1;
                 v = FIX_ONE;
             } else {
@@ -405,7 +405,8 @@ __global__ void __maxnreg__(SAMPLE_FF_REGS) k_sample_ff(SampleParams P, const TA
                     dvg = fminf(fmaxf(dvg, 0.0f), dv);
                 }
                 const TAB* seg = coef + b.coef_off[c] + (int64_t)(s - s0) * code_stride(CODE);
-                const float eps_s = P.eps_frac * (FROM64 ? ff_from_double_scaled(L, sexp).hi : f32_of_f64_trunc(L));
+                const float Ls = FROM64 ? ff_from_double_scaled(L, sexp).hi : f32_of_f64_trunc(L);
+                const float eps_s = P.eps_frac * (Ls == Ls ? Ls : dS.hi);
                 const long long w = ff_leaf_newton<CODE>(seg, sexp, vaf, dv, rl, dS, dvg, eps_s, tight * eps_s, newton);
                 v = vfix + (w < 0 ? 0 : w > dfix ? dfix : w);
             }

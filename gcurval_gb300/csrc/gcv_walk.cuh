@@ -103,6 +103,20 @@ __device__ __forceinline__ int interval_exponent(const double* __restrict__ seg)
     }
 }
 
+// K15 of a panel in FP64 whose float-float panel is infinite or NaN: with infinite
+// control points FP64 has an infinite length where float-float has NaN, and
+// samples are placed by it
+template <int CODE>
+__device__ __noinline__ double nonfinite_k15(const double* __restrict__ seg, unsigned long long k, int depth)
+{
+    double r[MAX_COEF];
+    Eval<CODE>::load_speed(seg, r);
+    const double hw = pow2_neg(depth);
+    double K, G, fe, qe;
+    panel_k15<CODE>(r, fma(__ull2double_rn(k), 2.0 * hw, -1.0), hw, K, G, fe, qe);
+    return K;
+}
+
 // the FP64 error test of one panel of an FP64 table (panels whose float-float
 // error estimate lands within 1 % or the float-float noise of the tolerance)
 template <int CODE>
@@ -425,10 +439,13 @@ __global__ void __launch_bounds__(WK_THREADS, PREC == 3 ? 6 : walk_blocks(CODE))
                     bool again = false;
                     if (g < total) {
                         const int qs = W.slot[q];
-                        const ff kf = unpack_ff(W.val[q]);
-                        double K = ff_to_double(kf);
-                        if (W.fits[qs] && isfinite(kf.hi))
-                            K = leaf_k15<CODE>(coef64(qs), W.sexp[qs], W.key[q] & WK_K_MASK, wk_depth(W.key[q]), again);
+                        double K = 0.0;
+                        if (W.fits[qs]) {
+                            const unsigned long long k = W.key[q] & WK_K_MASK;
+                            const int depth = wk_depth(W.key[q]);
+                            K = isfinite(unpack_ff(W.val[q]).hi) ? leaf_k15<CODE>(coef64(qs), W.sexp[qs], k, depth, again)
+                                                                 : nonfinite_k15<CODE>(coef64(qs), k, depth);
+                        }
                         if (!again) W.val[q] = K;
                     }
                     if constexpr (CODE > 0) {
