@@ -260,27 +260,17 @@ int sm_count()
 
 }  // namespace
 
-// the curve codes' slots in per-code tables: ellipse 0, then degree 1-5 in
-// 2D (1-5) and in 3D (6-10)
-constexpr int N_CODE_SLOTS = GCV_N_CODE_SLOTS;
-inline int code_slot(int code) { return code == CODE_ELLIPSE ? 0 : 1 + (code_dim(code) - 2) * 5 + (code_degree(code) - 1); }
-
 // Launch shapes picked by the autotuner: persistent length workers per SM
-// (cap on the occupancy) for each curve code's main pass and for the deep
+// (cap on the occupancy) for the main passes of every curve code and the deep
 // passes, and the sampling kernels' block size and blocks per SM.
 struct Knobs {
-    int length_cap[N_CODE_SLOTS];
-    int deep_cap = 32;
+    int length_cap = 32;
     int sample_threads = 256;
     int sample_blocks_per_sm = 64;
-    Knobs()
-    {
-        for (int& x : length_cap) x = 32;
-    }
     bool operator==(const Knobs& o) const
     {
-        return std::memcmp(length_cap, o.length_cap, sizeof(length_cap)) == 0 && deep_cap == o.deep_cap &&
-               sample_threads == o.sample_threads && sample_blocks_per_sm == o.sample_blocks_per_sm;
+        return length_cap == o.length_cap && sample_threads == o.sample_threads &&
+               sample_blocks_per_sm == o.sample_blocks_per_sm;
     }
 };
 // The first TUNE_TRIALS table builds (and samplings) of a batch shape not seen
@@ -293,8 +283,7 @@ inline int trial_length_cap(int i) { return i == 1 ? 4 : (i == 2 ? 6 : 32); }
 inline Knobs trial_knobs(int i)
 {
     Knobs k;
-    for (int& x : k.length_cap) x = trial_length_cap(i);
-    k.deep_cap = trial_length_cap(i);
+    k.length_cap = trial_length_cap(i);
     if (i == 1) {
         k.sample_threads = 128;
         k.sample_blocks_per_sm = 128;
@@ -833,8 +822,9 @@ gcv_status ensure_table_buffers(gcv_ctx* c)
     CHECK(c->leaf_cnt.reserve(ns));
     CHECK(c->curve_len.reserve((size_t)std::max<int64_t>(c->n_curve, 1)));
     if (c->leaf_cap == 0) {
-        // about three leaves per interval at the default tolerances; a pool
-        // that turns out short sends the rest to the deep passes, which grow it
+        // about three leaves per interval at the default tolerances; with a pool
+        // that turns out short k_walk's pass is run again with a larger one (the
+        // FP64 and half-warp walks send the rest to the deep passes, which grow it)
         c->leaf_cap = 3 * (int64_t)ns + 4096;
         CHECK(c->leaf_v.reserve((size_t)c->leaf_cap));
         CHECK(c->leaf_cum.reserve((size_t)c->leaf_cap));
@@ -908,7 +898,7 @@ gcv_status launch_length_code(gcv_ctx* c, int code, const LengthParams& P, cudaS
     const int sms = sm_count();
     cudaError_t e = cudaErrorInvalidValue;
     if constexpr (MODE == 0) {
-        const int cap = c->knobs.length_cap[code_slot(code)];
+        const int cap = c->knobs.length_cap;
         // FP64 tables: k_walk wherever its float-float partition resolves the
         // tolerance and the depth, the FP64 walk beyond
         const bool half_warp = c->opt.mapping == GCV_MAP_HALF_WARP;
@@ -926,7 +916,7 @@ gcv_status launch_length_code(gcv_ctx* c, int code, const LengthParams& P, cudaS
         default: return fail(GCV_ERR_INVALID, "no length kernel for curve code " + std::to_string(code));
         }
     } else {
-        const int cap = c->knobs.deep_cap;
+        const int cap = c->knobs.length_cap;
         switch (code) {
         case CODE_ELLIPSE: e = length_launch<MODE, CODE_ELLIPSE, PREC>(P, st, sms, cap); break;
         case bs_code(3, 2): e = length_launch<MODE, bs_code(3, 2), PREC>(P, st, sms, cap); break;
@@ -1004,9 +994,7 @@ void select_knobs(gcv_ctx* c)
         }
     }
     if (c->len_trial >= 0 && c->len_trial < TUNE_TRIALS) {
-        const Knobs k = trial_knobs(c->len_trial);
-        std::memcpy(c->knobs.length_cap, k.length_cap, sizeof(k.length_cap));
-        c->knobs.deep_cap = k.deep_cap;
+        c->knobs.length_cap = trial_length_cap(c->len_trial);
     }
     if (c->smp_trial >= 0 && c->smp_trial < TUNE_TRIALS) {
         const Knobs k = trial_knobs(c->smp_trial);
@@ -1026,9 +1014,7 @@ int argmin3(const double* v)
 // the length shapes of finished trials: the one with the fastest length phase
 void choose_length_knobs(gcv_ctx* c, Knobs& k)
 {
-    const int best = trial_length_cap(argmin3(c->len_ms));
-    for (int& x : k.length_cap) x = best;
-    k.deep_cap = best;
+    k.length_cap = trial_length_cap(argmin3(c->len_ms));
 }
 
 void tune_finish_if_done(gcv_ctx* c)
@@ -2280,8 +2266,8 @@ gcv_status gcv_get_stats(gcv_ctx* ctx, gcv_stats* out)
         }
     }
     cudaGetLastError();
-    ctx->stats.length_blocks_per_sm = ctx->code >= 0 ? ctx->knobs.length_cap[code_slot(ctx->code)] : ctx->knobs.deep_cap;
-    for (int sl = 0; sl < N_CODE_SLOTS; ++sl) ctx->stats.length_blocks_per_sm_code[sl] = ctx->knobs.length_cap[sl];
+    ctx->stats.length_blocks_per_sm = ctx->knobs.length_cap;
+    for (int& x : ctx->stats.length_blocks_per_sm_code) x = ctx->knobs.length_cap;
     ctx->stats.sample_threads = ctx->knobs.sample_threads;
     ctx->stats.sample_blocks_per_sm = ctx->knobs.sample_blocks_per_sm;
     ctx->stats.tuned = ctx->len_trial < 0 ? 1 : 0;

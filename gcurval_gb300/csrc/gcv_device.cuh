@@ -240,28 +240,6 @@ __device__ __forceinline__ void load_speed_dyn(int code, const double* __restric
     }
 }
 
-__device__ __forceinline__ double speed_dyn(int code, const double* r, double v)
-{
-    switch (code) {
-#define GCV_CASE(C)                                                                                \
-    case C: return Eval<C>::speed(r, v);
-        GCV_FOR_EACH_CODE(GCV_CASE)
-#undef GCV_CASE
-    default: return 0.0;
-    }
-}
-
-__device__ __forceinline__ double speed_slope_dyn(int code, const double* r, double v, double& q)
-{
-    switch (code) {
-#define GCV_CASE(C)                                                                                \
-    case C: return Eval<C>::speed_slope(r, v, q);
-        GCV_FOR_EACH_CODE(GCV_CASE)
-#undef GCV_CASE
-    default: q = 0.0; return 0.0;
-    }
-}
-
 __device__ __forceinline__ void point_dyn(int code, const double* __restrict__ seg, double v, double* out)
 {
     switch (code) {

@@ -19,42 +19,6 @@ __host__ __device__ constexpr ffc split_const(double x)
 }
 __device__ __forceinline__ ff to_ff(ffc c) { return ff{c.hi, c.lo}; }
 
-// ------------------------------------------------- sin^2(pi x), |x| <= 1
-// sin^2(pi x) has period 1 and is even: fold x to y in [0, 1/2]; then
-// sin^2(pi y) = S(y) for y <= 1/4 and 1 - S(1/2 - y) above, with S the
-// even series S(u) = sin^2(pi u) = sum_{k >= 1} c_k u^(2k),
-// c_k = (-1)^(k+1) 2^(2k-1) pi^(2k) / (2k)!, for |u| <= 1/4.  Eleven terms:
-// the twelfth is below 1e-19 there, far under float-float rounding.
-constexpr int SIN2_TERMS = 11;
-__host__ __device__ constexpr double sin2pi_coef(int k)
-{
-    double c = 0.5;  // (2 pi)^(2k) / (2k)! / 2
-    for (int i = 1; i <= 2 * k; ++i) c *= 2.0 * PI / i;
-    return (k % 2 == 1) ? c : -c;
-}
-
-// x in [-1, 1] -> u in [0, 1/4] and whether the result is 1 - S(u)
-__device__ __forceinline__ ff sinpi_sq_fold(ff x, bool& upper)
-{
-    ff y = x.hi < 0.0f ? ff_neg(x) : x;
-    if (y.hi > 0.5f) y = ff_add_f(ff_neg(y), 1.0f);  // 1 - |x|
-    upper = y.hi > 0.25f;
-    return upper ? ff_add_f(ff_neg(y), 0.5f) : y;
-}
-
-// sin^2(pi x) for x in [-1, 1]
-__device__ __forceinline__ ff ff_sinpi_sq(ff x)
-{
-    bool up;
-    const ff u = sinpi_sq_fold(x, up);
-    const ff U = ff_mul(u, u);
-    ff p = to_ff(split_const(sin2pi_coef(SIN2_TERMS)));
-#pragma unroll
-    for (int k = SIN2_TERMS - 1; k >= 1; --k) p = ff_fma(p, U, to_ff(split_const(sin2pi_coef(k))));
-    const ff S = ff_mul(p, U);
-    return up ? ff_add_f(ff_neg(S), 1.0f) : S;
-}
-
 // sin(pi x) and cos(pi x) for small x by their Taylor series, at compile time
 __host__ __device__ constexpr double series_sinpi(double x)
 {
@@ -213,27 +177,8 @@ struct EvalFF {
                 }
         }
     }
-    __device__ __forceinline__ static ff speed(const ff* r, ff v)
-    {
-        if constexpr (CODE == 0) {
-            // sqrt(B + A sin^2(pi w)), w = w0 + v / ELLIPSE_PIECES in [-1, 1]
-            const ff w = ff_add_f(ff_scale(v, (float)ELLIPSE_PIECE_SCALE), r[2].hi);
-            const ff s2 = ff_sinpi_sq(w);
-            return ff_sqrt(ff_fma(r[0], s2, r[1]));
-        } else {
-            ff s{0.0f, 0.0f};
-#pragma unroll
-            for (int d = 0; d < D; ++d) {
-                ff acc = r[(P - 1) * D + d];
-#pragma unroll
-                for (int k = P - 2; k >= 0; --k) acc = ff_fma(acc, v, r[k * D + d]);
-                s = d == 0 ? ff_mul(acc, acc) : ff_fma(acc, acc, s);
-            }
-            return ff_sqrt(s);
-        }
-    }
-    // the speeds at two points at once (packed lanes): the arithmetic of
-    // speed() lane by lane, each coefficient splat into both lanes
+    // the speeds of a B-spline piece at two points at once, in packed lanes, each
+    // coefficient splat into both
     __device__ __forceinline__ static ff2 speed2(const ff* r, ff2 v)
     {
         static_assert(CODE != 0, "ellipse sums go by angle addition");
@@ -479,9 +424,9 @@ __device__ __forceinline__ void panel_k15_ff_pairs(ff* b, unsigned long long k, 
     G = ff_scale(gg, hw);
 }
 
-// the float-float panel of a curve code: node pairs for B-splines, node by
-// node for the ellipse's sin(pi x) integrand; r (the interval's speed
-// coefficients) is scratch: the B-spline panel shifts it in place
+// the float-float panel of a curve code, by node pairs: B-splines from the
+// polynomials shifted to the midpoint, ellipses by angle addition; r (the interval's
+// speed coefficients) is scratch: the B-spline panel shifts it in place
 template <int CODE>
 __device__ __forceinline__ void panel_ff(ff* r, unsigned long long k, int depth, ff& K, ff& G)
 {

@@ -172,27 +172,8 @@ constexpr int SAMPLE_RUNS_PER_SM = 96;
 // sample's total error within 1.1 rtol * L.
 constexpr double SAMPLE_EPS_FRAC = 0.1;
 
-constexpr int SAMPLE_THREADS = 256;      // default block size
 constexpr int SAMPLE_THREADS_MAX = 512;  // largest block size the autotuner tries
 constexpr int NEWTON_MAXIT = 16;
-
-template <int CODE>
-__device__ __forceinline__ double speed_of(int code, const double* r, double v)
-{
-    if constexpr (CODE >= 0)
-        return Eval<CODE>::speed(r, v);
-    else
-        return speed_dyn(code, r, v);
-}
-
-template <int CODE>
-__device__ __forceinline__ double speed_slope_of(int code, const double* r, double v, double& q)
-{
-    if constexpr (CODE >= 0)
-        return Eval<CODE>::speed_slope(r, v, q);
-    else
-        return speed_slope_dyn(code, r, v, q);
-}
 
 // Newton on one leaf [va, vb] (cumulative lengths base, cb) for the target rr,
 // from the guess vg: F(v) = S(v) - rr with S(v) = S(va) + GL8(va, v) or

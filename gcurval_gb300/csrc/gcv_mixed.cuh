@@ -280,7 +280,7 @@ __device__ __forceinline__ long long ff_leaf_newton(const TAB* __restrict__ seg,
 // were worth 0.47 ms of it.
 constexpr int SAMPLE_FF_REGS = 64;
 static_assert(SAMPLE_FF_REGS * SAMPLE_THREADS_MAX <= 65536, "a block of SAMPLE_THREADS_MAX must fit one SM");
-// residual, of the curve's length, that counts as an iterate's (at least eps_frac)
+// residual, of the curve's length, that counts as an iterate's (at most eps_frac)
 constexpr float SAMPLE_TIGHT = 4e-11f;
 //
 // TAB = double runs the same kernel on an FP64 table (GCV_PLAIN_FP64 at

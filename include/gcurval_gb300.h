@@ -59,9 +59,10 @@ typedef enum gcv_enum {
 } gcv_enum;
 
 typedef enum gcv_precision {
-    GCV_PLAIN_FP64 = 0,    /* FP64 lengths, sums, targets and parameters; at rtol >= 1e-12
-                              the Newton steps inside one table entry run in float-float
-                              (48 bits), below it in FP64 */
+    GCV_PLAIN_FP64 = 0,    /* FP64 lengths, sums, targets and parameters.  At rtol >= 1e-12
+                              the decision to split a panel is made in float-float (48
+                              bits; in FP64 near the tolerance), and so are the Newton
+                              steps inside one table entry; below it all in FP64 */
     GCV_MIXED = 1          /* FP32 integrand and panels; FP64 prefix sum,
                               error test near tolerance and final Newton step */
 } gcv_precision;
@@ -134,7 +135,8 @@ typedef struct gcv_stats {
        candidate, later ones use the fastest (tuned = 1) */
     int length_blocks_per_sm, sample_threads, sample_blocks_per_sm, tuned;
     /* persistent length workers per SM of each curve code's main pass, by
-       slot: ellipse 0, degree 1..5 in 2D at 1..5, in 3D at 6..10 */
+       slot: ellipse 0, degree 1..5 in 2D at 1..5, in 3D at 6..10 (one shape
+       for all: length_blocks_per_sm) */
     int length_blocks_per_sm_code[GCV_N_CODE_SLOTS];
 } gcv_stats;
 
