@@ -467,7 +467,11 @@ def roofline_of(batch, r, plain_r, is_plain: bool, workload: str, precision: str
     the batch (plain_r's panels x 16 and Newton iterations x 10) x the
     reference's FLOPs per evaluation, over the phase's time; the library's
     own count (its own evaluations x its cheaper per-evaluation FLOPs) is
-    given beside it."""
+    given beside it.  At rtol >= 1e-12 every form runs k_walk and k_sample_ff,
+    whose panels and Newton steps are on the FP32 pipes (the plain form's leaf
+    sums in FP64 beside them), so the FP32 peak is the bound; below, the plain
+    form runs k_length and k_sample on the FP64 pipe."""
+    fp64_only = is_plain and batch.rtol < 1e-12
     n_samples = batch.total_samples
     fpe = flops_per_eval(batch)
     ms_inf = r["ms_learned"]
@@ -483,14 +487,14 @@ def roofline_of(batch, r, plain_r, is_plain: bool, workload: str, precision: str
     sv_len = float(np.mean(src["n_panels"])) * 16.0 * f_len
     sv_samp = float(np.mean(src["n_newton"])) * 10.0 * f_smp
     if ms_s >= ms_l:
-        dom, flops, own, ms = "k_sample", sv_samp, own_samp, ms_s
+        dom, flops, own, ms = "k_sample" if fp64_only else "k_sample_ff", sv_samp, own_samp, ms_s
         bytes_alg = n_samples * (8 + 8 + 8) + batch.n_curve * 8
         units = n_samples
     else:
-        dom, flops, own, ms = "k_length", sv_len, own_len, ms_l
+        dom, flops, own, ms = "k_length" if fp64_only else "k_walk", sv_len, own_len, ms_l
         bytes_alg = batch.knots.nbytes + batch.ctrl.nbytes + int(batch.n_segments.sum()) * 8
         units = float(batch.n_segments.sum())
-    peak = fp64_peak if is_plain else fp32_peak
+    peak = fp64_peak if fp64_only else fp32_peak
     achieved = flops / (ms * 1e-3) / 1e12
     traffic = None
     prof = os.path.join(ROOT, "profiles", "traffic_per_unit.json")
@@ -502,12 +506,12 @@ def roofline_of(batch, r, plain_r, is_plain: bool, workload: str, precision: str
         except (ValueError, OSError):
             traffic = None
     return {
-        "kernel": dom, "bound": "fp64" if is_plain else "fp32",
+        "kernel": dom, "bound": "fp64" if fp64_only else "fp32",
         "achieved": round(achieved, 4), "peak": round(peak, 4), "unit": "TFLOP/s", "frac": round(achieved / peak, 4),
         "peak_source": "measured in-run by gcv_measure_fma_peak (FMA probe kernel)",
         "work": ("evaluations of the plain FP64 method (panels x 16 + Newton iterations x 10) x FLOPs per "
                  "evaluation of the reference's de Boor / ellipse derivative"),
-        "flops_per_eval_reference": round(f_smp if dom == "k_sample" else f_len, 3),
+        "flops_per_eval_reference": round(f_smp if dom.startswith("k_sample") else f_len, 3),
         "traffic": traffic, "ms_per_launch": round(ms, 4), "algorithmic_flops_per_launch": flops,
         "own_count": {"flops_per_eval": round(fpe, 3), "flops": own, "achieved": round(own / (ms * 1e-3) / 1e12, 4),
                       "frac": round(own / (ms * 1e-3) / 1e12 / peak, 4),
