@@ -10,6 +10,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <shared_mutex>
 #include <tuple>
 #include <cmath>
 #include <cstdio>
@@ -57,6 +58,22 @@ gcv_status cuda_fail(cudaError_t e, const char* what)
         gcv_status s_ = (st);                                                                      \
         if (s_ != GCV_OK) return s_;                                                               \
     } while (0)
+
+// Waiting for the whole device while any stream is being captured makes that
+// capture invalid, whichever thread waits.  A capture (gcv_step_graph) holds this
+// gate shared; what waits for the device (cudaFree does) passes it alone.
+std::shared_mutex g_capture_gate;
+
+void wait_for_device()
+{
+    std::unique_lock<std::shared_mutex> g(g_capture_gate);
+    cudaDeviceSynchronize();
+}
+void device_free(void* p)
+{
+    std::unique_lock<std::shared_mutex> g(g_capture_gate);
+    cudaFree(p);
+}
 
 // ---------------------------------------------------- device memory cache
 // A destroyed context hands its device buffers to a process-wide cache, and
@@ -116,7 +133,7 @@ size_t release_cache(int dev)
     const int cur = current_device();
     for (auto& d : drop) {
         if (d.second != cur) cudaSetDevice(d.second);
-        cudaFree(d.first);
+        device_free(d.first);
         if (d.second != cur) cudaSetDevice(cur);
     }
     return bytes;
@@ -141,7 +158,7 @@ size_t release_oldest(int dev, size_t want)
             g_cache.erase(oldest);
         }
     }
-    for (void* q : drop) cudaFree(q);
+    for (void* q : drop) device_free(q);
     return bytes;
 }
 
@@ -175,7 +192,7 @@ void dev_recycle(void* p, size_t bytes)
 {
     if (!p) return;
     if (!cache_enabled()) {
-        cudaFree(p);
+        device_free(p);
         return;
     }
     std::lock_guard<std::mutex> g(g_cache_m);
@@ -221,7 +238,7 @@ struct DBuf {
     // while the context's work may still be in flight
     void release()
     {
-        if (p && owned) cudaFree(p);
+        if (p && owned) device_free(p);
         p = nullptr;
         n = 0;
         bytes = 0;
@@ -486,7 +503,7 @@ void destroy_ctx(gcv_ctx* c)
     if (!c) return;
     // the context's buffers go to the memory cache idle, as cudaFree would
     // have left them
-    if (cache_enabled()) cudaDeviceSynchronize();
+    if (cache_enabled()) wait_for_device();
     c->kind.recycle();
     c->degree.recycle();
     c->dim.recycle();
@@ -501,7 +518,7 @@ void destroy_ctx(gcv_ctx* c)
     c->curve_list.recycle();
     c->starts.recycle();
     c->feat16.recycle();
-    if (c->mlp_w) cudaFree(c->mlp_w);
+    if (c->mlp_w) device_free(c->mlp_w);
     c->list_sample_off.recycle();
     c->coef.recycle();
     c->seg_t0.recycle();
@@ -768,7 +785,9 @@ public:
             used_[h] = false;
             cudaError_t e = cudaEventRecord(c_->kit->join[h], c_->kit->helper[h]);
             if (e == cudaSuccess) e = cudaStreamWaitEvent(c_->stream, c_->kit->join[h], 0);
-            if (e != cudaSuccess && st == GCV_OK) st = cuda_fail(e, "joining a helper stream");
+            if (e == cudaSuccess) continue;
+            cudaGetLastError();  // not left for the next launch's check
+            if (st == GCV_OK) st = cuda_fail(e, "joining a helper stream");
         }
         return st;
     }
@@ -1659,6 +1678,9 @@ std::vector<double> widen_host(const float* p, size_t n)
 
 // ===================================================================== ABI
 
+// for the library's other parts
+extern "C" void gcv_internal_device_free(void* p) { device_free(p); }
+
 extern "C" {
 
 const char* gcv_status_string(gcv_status s)
@@ -1860,7 +1882,7 @@ gcv_status gcv_destroy(gcv_ctx* ctx)
 {
     if (!ctx) return fail(GCV_ERR_INVALID, "ctx is NULL");
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    else cudaDeviceSynchronize();
+    else wait_for_device();
     destroy_ctx(ctx);
     return GCV_OK;
 }
@@ -2020,7 +2042,7 @@ gcv_status gcv_free_result(gcv_result* r)
     if (!r) return fail(GCV_ERR_INVALID, "result is NULL");
     if (r->data) {
         if (r->store_where == GCV_DEVICE)
-            cudaFree(r->data);
+            device_free(r->data);
         else
             std::free(r->data);
     }
@@ -2229,7 +2251,7 @@ gcv_status gcv_free_result_f32(gcv_result_f32* r)
     if (!r) return fail(GCV_ERR_INVALID, "result is NULL");
     if (r->data) {
         if (r->store_where == GCV_DEVICE)
-            cudaFree(r->data);
+            device_free(r->data);
         else
             std::free(r->data);
     }
@@ -2334,7 +2356,7 @@ gcv_status gcv_measure_fma_peak(int which, double* tflops)
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    cudaFree(out);
+    device_free(out);
     const double flops = 2.0 * 8.0 * iters * (double)threads * blocks;
     *tflops = flops / (best * 1e-3) / 1e12;
     return GCV_OK;
@@ -2381,18 +2403,25 @@ gcv_status gcv_step_graph(gcv_ctx* ctx, const int* d_counts, const double* d_pos
         cudaStream_t cap = c->stream ? c->stream : c->gstream;
         CU(cudaStreamSynchronize(user));
         c->stream = cap;
-        cudaError_t e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
-        gcv_status st = e == cudaSuccess ? GCV_OK : cuda_fail(e, "cudaStreamBeginCapture");
-        if (st == GCV_OK) st = enqueue_table_graph(c);
-        if (st == GCV_OK) st = enqueue_sampling_graph(c, d_counts, d_pos, is_relative, what, d_out);
         cudaGraph_t g = nullptr;
-        e = cudaStreamEndCapture(cap, &g);
+        cudaError_t e;
+        gcv_status st;
+        {
+            std::shared_lock<std::shared_mutex> gate(g_capture_gate);
+            e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
+            st = e == cudaSuccess ? GCV_OK : cuda_fail(e, "cudaStreamBeginCapture");
+            if (st == GCV_OK) st = enqueue_table_graph(c);
+            if (st == GCV_OK) st = enqueue_sampling_graph(c, d_counts, d_pos, is_relative, what, d_out);
+            e = cudaStreamEndCapture(cap, &g);
+        }
         c->stream = user;
-        if (st != GCV_OK) {
+        if (st != GCV_OK || e != cudaSuccess) {
+            if (st == GCV_OK) st = cuda_fail(e, "cudaStreamEndCapture");
+            cudaGetLastError();  // the ended capture's error is not left for the next launch's check
             if (g) cudaGraphDestroy(g);
+            c->kit.reset();  // its streams were part of the capture
             return st;
         }
-        if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
         c->graph = g;
         e = cudaGraphInstantiate(&c->gexec, g, 0);
         if (e != cudaSuccess) {
@@ -2497,7 +2526,7 @@ gcv_status gcv_set_learned_model(gcv_ctx* ctx, const float* host_weights)
     CU(cudaStreamSynchronize(ctx->stream));
     drop_graph(ctx);  // a captured step holds the old weights
     if (ctx->mlp_w) {
-        cudaFree(ctx->mlp_w);
+        device_free(ctx->mlp_w);
         ctx->mlp_w = nullptr;
     }
     if (!host_weights) return GCV_OK;
@@ -2506,7 +2535,7 @@ gcv_status gcv_set_learned_model(gcv_ctx* ctx, const float* host_weights)
     void* w = nullptr;
     cudaError_t e = mlp_upload_bf16(host_weights, &w);
     if (e != cudaSuccess) {
-        if (w) cudaFree(w);
+        if (w) device_free(w);
         return cuda_fail(e, "network upload");
     }
     ctx->mlp_w = w;

@@ -35,6 +35,7 @@
 #include "gcv_decimal.cuh"
 
 extern "C" gcv_status gcv_internal_fail(gcv_status s, const char* msg);
+extern "C" void gcv_internal_device_free(void* p);
 
 struct gcv_bundle {
     cudaStream_t stream = nullptr;
@@ -409,7 +410,7 @@ struct DMem {
     DMem& operator=(const DMem&) = delete;
     ~DMem()
     {
-        if (p) cudaFree(p);
+        if (p) gcv_internal_device_free(p);
     }
     template <typename T>
     T* as() const
@@ -423,12 +424,12 @@ void free_bundle(gcv_bundle* b)
 {
     if (!b) return;
     if (b->stream || b->vals) cudaStreamSynchronize(b->stream);
-    cudaFree(b->vals);
-    cudaFree(b->rec_tok);
-    cudaFree(b->rec_p);
-    cudaFree(b->rec_nc);
-    cudaFree(b->knot_off);
-    cudaFree(b->ctrl_off);
+    gcv_internal_device_free(b->vals);
+    gcv_internal_device_free(b->rec_tok);
+    gcv_internal_device_free(b->rec_p);
+    gcv_internal_device_free(b->rec_nc);
+    gcv_internal_device_free(b->knot_off);
+    gcv_internal_device_free(b->ctrl_off);
     delete b;
 }
 

@@ -18,6 +18,8 @@
 
 using namespace gcv;
 
+extern "C" void gcv_internal_device_free(void* p);
+
 namespace {
 
 thread_local std::string g_err_train;
@@ -418,7 +420,7 @@ gcv_status gcv_mlp_trainer_destroy(gcv_mlp_trainer* tr)
     float* bufs[] = {tr->w, tr->g, tr->m, tr->v, tr->Z[0], tr->Z[1], tr->Z[2], tr->H[0], tr->H[1], tr->H[2],
                      tr->out, tr->dOut, tr->dA, tr->dB, tr->loss3, tr->part, tr->loss_part};
     for (float* b : bufs)
-        if (b) cudaFree(b);
+        if (b) gcv_internal_device_free(b);
     delete tr;
     return GCV_OK;
 }

@@ -1,7 +1,7 @@
 """Curves without a knot interval (a single span's knots short) have length 0 wherever
 they stand, in a table built over recycled memory too, and a long run of them takes no
-longer than its memory: a table of two curves among 400,000 empty ones is built in less
-than twice the time of the two alone and ten clears of the lengths."""
+longer than its memory: the prefix sums of two curves among 400,000 empty ones take less
+than a tenth of a millisecond more than those of the two alone."""
 import numpy as np
 import pytest
 
@@ -57,4 +57,4 @@ def test_a_long_run_costs_a_clear(gpu_lib):
     b, two, _ = batch(0, 400_000, 0)
     _, alone = build(two, g.GCV_MIXED, times=15)
     _, among = build(b, g.GCV_MIXED, times=15)
-    assert among <= 2.0 * alone + 10 * 1e3 * 400_000 * 8 / 2e12
+    assert among <= alone + 0.1
